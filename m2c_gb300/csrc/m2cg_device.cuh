@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <cfloat>
 #include "../../include/m2cg.h"
+#include "m2cg_intfp.cuh"
 
 #define M2CG_DEV __device__ __forceinline__
 
@@ -42,6 +43,50 @@ M2CG_DEV bool lt_zero_bits(double x) { long long b = bits(x); return b < 0 && b 
 M2CG_DEV bool abs_lt_bits(double x, double c) { return (bits(x) & 0x7fffffffffffffffll) < bits(c); }
 M2CG_DEV bool is_pos_inf(double x) { return bits(x) == 0x7ff0000000000000ll; }
 M2CG_DEV bool is_neg_inf(double x) { return bits(x) == (long long)0xfff0000000000000ull; }
+// Comparisons, minima and maxima of any two doubles on the integer pipe: the
+// results of the FP64 instructions for every operand (an FP64 comparison costs
+// a full slot of the FP64 pipe, and 115 cycles of latency on a dependent chain).
+M2CG_DEV bool is_nan_bits(double x) { return (bits(x) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll; }
+M2CG_DEV bool i_le0(double x) {   // x <= 0: +0, or -0 down to -infinity
+  const unsigned long long u = (unsigned long long)bits(x);
+  return u == 0ull || u - 0x8000000000000000ull <= 0x7ff0000000000000ull;
+}
+M2CG_DEV bool i_lt0(double x) {   // x < 0
+  return (unsigned long long)bits(x) - 0x8000000000000001ull <= 0x7fefffffffffffffull;
+}
+M2CG_DEV bool i_eq0(double x) { return ((unsigned long long)bits(x) << 1) == 0ull; }
+// order-preserving integer of a double that is not NaN (-0 just below +0)
+M2CG_DEV long long i_key(double x) {
+  const int m = __double2hiint(x) >> 31;
+  return ((long long)(__double2hiint(x) ^ (m & 0x7fffffff)) << 32) | (unsigned)(__double2loint(x) ^ m);
+}
+M2CG_DEV bool i_special(double a, double b) {   // an infinity or NaN among the two
+  return (__double2hiint(a) & 0x7ff00000) == 0x7ff00000 || (__double2hiint(b) & 0x7ff00000) == 0x7ff00000;
+}
+static __device__ __noinline__ bool lt_fp64(double a, double b) { return a < b; }
+static __device__ __noinline__ double min_fp64(double a, double b) { return fmin(a, b); }
+M2CG_DEV bool i_lt(double a, double b) {
+  if (i_special(a, b)) return lt_fp64(a, b);
+  return i_key(a) < i_key(b) && ((bits(a) | bits(b)) << 1) != 0;
+}
+M2CG_DEV bool i_le(double a, double b) {
+  if (i_special(a, b)) return lt_fp64(a, b) || a == b;
+  return i_key(a) <= i_key(b) || ((bits(a) | bits(b)) << 1) == 0;
+}
+M2CG_DEV double i_min(double a, double b) {
+  if (i_special(a, b)) return min_fp64(a, b);
+  return i_key(a) <= i_key(b) ? a : b;
+}
+M2CG_DEV double i_max(double a, double b) {
+  if (i_special(a, b)) return -min_fp64(-a, -b);
+  return i_key(a) >= i_key(b) ? a : b;
+}
+// a b < 0: opposite signs, unless the product underflows to zero or an operand is zero or NaN
+M2CG_DEV bool i_prod_lt0(double a, double b) {
+  const unsigned ea = (unsigned)(bits(a) >> 52) & 0x7ffu, eb = (unsigned)(bits(b) >> 52) & 0x7ffu;
+  if (ea + eb < 1100u || ea - 1u > 2045u || eb - 1u > 2045u) return i_lt0(__dmul_rn(a, b));
+  return (bits(a) ^ bits(b)) < 0;
+}
 
 // Reciprocal and reciprocal square root: the hardware approximations of the
 // PTX ISA (rcp.approx.ftz.f64, rsqrt.approx.ftz.f64; about 2^-20 relative
@@ -64,115 +109,85 @@ M2CG_DEV double rsqrt_fast(double x) {
   return fma(y * e, fma(e, 0.375, 0.5), y);
 }
 
-// Correctly rounded quotients a / b for several numerators over one divisor,
-// after P. Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", IBM J. Res. Dev. 34(1), 1990 (theorems restated in
-// Muller et al., Handbook of Floating-Point Arithmetic, ch. on division with
-// an FMA).  In round-to-nearest binary64 without underflow or overflow:
-//   (1) if y1 is within one ulp of 1/b and the significand of b is not all
-//       ones, y = y1 + y1 (1 - b y1) (two FMAs) is RN(1/b);
-//   (2) if y = RN(1/b) and q is within one ulp of a/b, the remainder
-//       a - b q is exact in one FMA and q + (a - b q) y rounds to RN(a/b).
-// q0 = RN(a y) can be 1.5 ulp off, so one remainder step brings it within
-// half an ulp first: five FP64 operations per quotient against the ~9 of a
-// full division, which pays from the second quotient of a divisor on
-// (measured on GB300, one dependent chain: 590 cycles for a / b, 321 for the
-// five operations, 372 for y).  Operands outside the range where the theorems
-// hold -- zero, subnormal, infinite or NaN operands, quotients near the
-// exponent limits, divisors with an all-ones significand -- take the IEEE
-// division instead, so every result equals a / b bit for bit
-// (m2cg_selftest_quotient checks that on random and edge-case operands).
+// Quotients of several numerators over one divisor: the divisor's fixed-point
+// reciprocal (m2cg_intfp.cuh) is formed once, each quotient takes the
+// remaining 40 integer instructions of ddiv.  Correctly rounded, equal to a / b
+// bit for bit (m2cg_selftest_quotient checks that on random and edge-case
+// operands); operands or results outside the normal range take the IEEE
+// division out of line.
 struct Quot {
-  double b, y;
-  bool fast;
+  double b;
+  uint64_t D, R;
 };
 M2CG_DEV int exp_field(double x) { return (int)((bits(x) >> 52) & 0x7ff); }
 M2CG_DEV Quot quot_of(double b) {
   Quot q;
   q.b = b;
-  const int eb = exp_field(b);
-  q.fast = (unsigned)(eb - 128) <= 1792u && (bits(b) & 0xfffffffffffffll) != 0xfffffffffffffll;
-  q.y = 0.0;
-  if (q.fast) {
-    const double y1 = rcp_fast(b);
-    q.y = fma(fma(-b, y1, 1.0), y1, y1);
-  }
+  q.D = if_sig(if_hi(b), if_lo(b));
+  q.R = if_recip(q.D);
   return q;
 }
-// the IEEE division out of line: one copy of its code however many quotients
-// fall back, which keeps the solver's hot loops small in the instruction cache
-static __device__ __noinline__ double ieee_div(double a, double b) { return a / b; }
-M2CG_DEV double qdiv(double a, const Quot& d) {
-  const int ea = exp_field(a), eq = ea - exp_field(d.b) + 1023;
-  if (!d.fast || (unsigned)(ea - 128) > 1792u || (unsigned)(eq - 128) > 1792u) return ieee_div(a, d.b);
-  double q = __dmul_rn(a, d.y);
-  q = fma(fma(-d.b, q, a), d.y, q);
-  return fma(fma(-d.b, q, a), d.y, q);
+M2CG_DEV bool qfast(double a, const Quot& d) { return if_div_range(a, d.b); }
+static __device__ __noinline__ double qdiv_call(double a, double b, uint64_t D, uint64_t R) {
+  return if_div_range(a, b) ? if_div_core(a, b, D, R) : a / b;
 }
-// 1 / b from the same divisor: y itself is RN(1/b)
-M2CG_DEV double qrcp(const Quot& d) { return d.fast ? d.y : ieee_div(1.0, d.b); }
-// The same calls with Shared = false are plain IEEE divisions.  The shared
-// reciprocal shortens a dependent chain (a lone solve on an otherwise idle
-// FP64 pipe) but issues a few more FP64-pipe slots per divisor than the
-// divisions it replaces, so code whose pipe is full (a warp of independent
-// solves per lane) keeps the divisions.  Both give the same bits.
-template <bool Shared> M2CG_DEV Quot quot_of_t(double b) {
-  if constexpr (Shared) return quot_of(b);
-  Quot q;
-  q.b = b;
-  q.y = 0.0;
-  q.fast = false;
-  return q;
-}
-template <bool Shared> M2CG_DEV double qdiv_t(double a, const Quot& d) {
-  if constexpr (Shared) return qdiv(a, d);
-  return a / d.b;
-}
-template <bool Shared> M2CG_DEV double qrcp_t(const Quot& d) {
-  if constexpr (Shared) return qrcp(d);
-  return 1.0 / d.b;
-}
+M2CG_DEV double qdiv(double a, const Quot& d) { return qdiv_call(a, d.b, d.D, d.R); }
 
 // ---- equation of state ----------------------------------------------------
 M2CG_DEV double eos_p(const DevMat& M, double rho, double e) {
   if (M.type == M2CG_EOS_SG) return M.gam1 * rho * e - M.gamPs;   // gamPs = RN(gamma * pc), the same product
-  if (M.type == M2CG_EOS_NASG) return M.gam1 * (e - M.q) / (1.0 / rho - M.b) - M.gamPs;
-  double eta = 1.0 - M.rho0 / rho;
-  return M.rho0_c0_c0 * eta * (1.0 - M.G0_half * eta) / ((1.0 - M.s * eta) * (1.0 - M.s * eta)) + M.G0_rho0 * (e - M.e0);
+  if (M.type == M2CG_EOS_NASG) return ddiv(M.gam1 * (e - M.q), ddiv(1.0, rho) - M.b) - M.gamPs;
+  double eta = 1.0 - ddiv(M.rho0, rho);
+  return ddiv(M.rho0_c0_c0 * eta * (1.0 - M.G0_half * eta), (1.0 - M.s * eta) * (1.0 - M.s * eta)) + M.G0_rho0 * (e - M.e0);
 }
 M2CG_DEV double eos_e(const DevMat& M, double rho, double p) {
-  if (M.type == M2CG_EOS_SG) return (p + M.gamPs) / (M.gam1 * rho);
-  if (M.type == M2CG_EOS_NASG) return M.invgam1 * (p + M.gamPs) * (1.0 / rho - M.b) + M.q;
-  double eta = 1.0 - M.rho0 / rho;
-  return (p - M.rho0_c0_c0 * eta * (1.0 - M.G0_half * eta) / ((1.0 - M.s * eta) * (1.0 - M.s * eta))) / M.G0_rho0 + M.e0;
+  if (M.type == M2CG_EOS_SG) return ddiv(p + M.gamPs, M.gam1 * rho);
+  if (M.type == M2CG_EOS_NASG) return M.invgam1 * (p + M.gamPs) * (ddiv(1.0, rho) - M.b) + M.q;
+  double eta = 1.0 - ddiv(M.rho0, rho);
+  return ddiv(p - ddiv(M.rho0_c0_c0 * eta * (1.0 - M.G0_half * eta), (1.0 - M.s * eta) * (1.0 - M.s * eta)), M.G0_rho0) + M.e0;
 }
 M2CG_DEV double eos_dpdrho(const DevMat& M, double rho, double e) {
   if (M.type == M2CG_EOS_SG) return M.gam1 * e;
-  if (M.type == M2CG_EOS_NASG) { double V = 1.0 / rho; return M.gam1 * V * V * (e - M.q) / ((V - M.b) * (V - M.b)); }
-  double eta = 1.0 - M.rho0 / rho;
+  if (M.type == M2CG_EOS_NASG) { double V = ddiv(1.0, rho); return ddiv(M.gam1 * V * V * (e - M.q), (V - M.b) * (V - M.b)); }
+  double eta = 1.0 - ddiv(M.rho0, rho);
   double S = 1.0 - M.s * eta;
-  return M.rho0_c0_c0 * (1.0 + (M.s - 2.0 * M.G0_half) * eta) / (S * S * S) * M.rho0 / (rho * rho);
+  return ddiv(ddiv(M.rho0_c0_c0 * (1.0 + (M.s - 2.0 * M.G0_half) * eta), S * S * S) * M.rho0, rho * rho);
 }
 M2CG_DEV double eos_Gamma(const DevMat& M, double rho) {
   if (M.type == M2CG_EOS_SG) return M.gam1;
-  if (M.type == M2CG_EOS_NASG) return M.gam1 / (1.0 - M.b * rho);
-  return M.G0_rho0 / rho;
+  if (M.type == M2CG_EOS_NASG) return ddiv(M.gam1, 1.0 - M.b * rho);
+  return ddiv(M.G0_rho0, rho);
 }
-// VarFcnBase.h:219-223
+// VarFcnBase.h:219-223.  The quotients that share a divisor or an operand are
+// formed once (NASG's 1/rho enters p, dp/drho and, through p / rho, c^2).
 M2CG_DEV double eos_c2(const DevMat& M, double rho, double e) {
-  return eos_dpdrho(M, rho, e) + eos_p(M, rho, e) / rho * eos_Gamma(M, rho);
+  if (M.type == M2CG_EOS_NASG) {
+    const double eq = M.gam1 * (e - M.q);
+    const Quot R = quot_of(rho);
+    const double V = qdiv(1.0, R);
+    const double p = ddiv(eq, V - M.b) - M.gamPs;
+    const double dpdrho = ddiv(M.gam1 * V * V * (e - M.q), (V - M.b) * (V - M.b));
+    return dpdrho + qdiv(p, R) * ddiv(M.gam1, 1.0 - M.b * rho);
+  }
+  return eos_dpdrho(M, rho, e) + ddiv(eos_p(M, rho, e), rho) * eos_Gamma(M, rho);
 }
-// eos_c2 with its division by rho through a reciprocal the caller shares (same bits)
-template <bool Shared> M2CG_DEV double eos_c2_q(const DevMat& M, double rho, const Quot& R, double e) {
-  return eos_dpdrho(M, rho, e) + qdiv_t<Shared>(eos_p(M, rho, e), R) * eos_Gamma(M, rho);
+// eos_c2 with its divisions by rho through a reciprocal the caller shares (same bits)
+M2CG_DEV double eos_c2_q(const DevMat& M, double rho, const Quot& R, double e) {
+  if (M.type == M2CG_EOS_NASG) {
+    const double V = qdiv(1.0, R);
+    const double p = ddiv(M.gam1 * (e - M.q), V - M.b) - M.gamPs;
+    const double dpdrho = ddiv(M.gam1 * V * V * (e - M.q), (V - M.b) * (V - M.b));
+    return dpdrho + qdiv(p, R) * ddiv(M.gam1, 1.0 - M.b * rho);
+  }
+  return eos_dpdrho(M, rho, e) + qdiv(eos_p(M, rho, e), R) * eos_Gamma(M, rho);
 }
 // CheckState: true = nonphysical (VarFcnSG.h:96-108, VarFcnNASG.h:73-85, VarFcnBase.h:120-140)
 M2CG_DEV bool eos_bad(const DevMat& M, double rho, double p) {
-  if (!isfinite(rho) || !isfinite(p)) return true;
-  if (M.type == M2CG_EOS_SG || M.type == M2CG_EOS_NASG) return (rho <= 0.0 || p + M.Pstiff <= 0.0);
-  if (rho <= 0.0) return true;
+  if (!is_finite_bits(rho) || !is_finite_bits(p)) return true;
+  if (M.type == M2CG_EOS_SG || M.type == M2CG_EOS_NASG) return i_le0(rho) || i_le0(p + M.Pstiff);
+  if (i_le0(rho)) return true;
   double e = eos_e(M, rho, p);
-  return eos_dpdrho(M, rho, e) + p / rho * eos_Gamma(M, rho) <= 0.0;
+  return eos_dpdrho(M, rho, e) + ddiv(p, rho) * eos_Gamma(M, rho) <= 0.0;
 }
 M2CG_DEV bool eos_bad5(const DevMat& M, const double* V) {
   if (!isfinite(V[1]) || !isfinite(V[2]) || !isfinite(V[3])) return true;
@@ -233,14 +248,14 @@ M2CG_DEV void cons_to_prim_fast(const DevMat& M, const double* U, double* V) {
 // VarFcnBase.h:173-186
 M2CG_DEV void cons_to_prim(const DevMat& M, const double* U, double* V) {
   V[0] = U[0];
-  double invRho = 1.0 / U[0];
+  double invRho = ddiv(1.0, U[0]);
   V[1] = U[1] * invRho; V[2] = U[2] * invRho; V[3] = U[3] * invRho;
   double e = (U[4] - 0.5 * V[0] * (V[1] * V[1] + V[2] * V[2] + V[3] * V[3])) * invRho;
   V[4] = eos_p(M, V[0], e);
 }
 M2CG_DEV double total_enthalpy(const DevMat& M, const double* V) {
   double e = eos_e(M, V[0], V[4]);
-  return e + 0.5 * (V[1] * V[1] + V[2] * V[2] + V[3] * V[3]) + V[4] / V[0];
+  return e + 0.5 * (V[1] * V[1] + V[2] * V[2] + V[3] * V[3]) + ddiv(V[4], V[0]);
 }
 
 // ---- physical flux (FluxFcnBase.h:82-123) ------------------------------------
@@ -254,7 +269,7 @@ M2CG_DEV void phys_flux(const DevMat& M, int dir, const double* V, double* F) {
   F[4] = rhou * H;
 }
 
-M2CG_DEV double avg(double w1, double f1, double w2, double f2) { return (w1 * f1 + w2 * f2) / (w1 + w2); }
+M2CG_DEV double avg(double w1, double f1, double w2, double f2) { return ddiv(w1 * f1 + w2 * f2, w1 + w2); }
 
 // Generalized Roe-averaged state of Hu et al. (FluxFcnHLLC.h:57-126)
 struct RoeHat {
@@ -262,43 +277,43 @@ struct RoeHat {
 };
 M2CG_DEV void roe_hat(const DevMat& M, int dir, const double* Vm, const double* Vp, RoeHat& r) {
   const double eps = 1e-10;
-  r.rho_hat = sqrt(Vm[0] * Vp[0]);
-  r.srm = sqrt(Vm[0]);
-  r.srp = sqrt(Vp[0]);
+  r.rho_hat = dsqrt(Vm[0] * Vp[0]);
+  r.srm = dsqrt(Vm[0]);
+  r.srp = dsqrt(Vp[0]);
   double drho = Vp[0] - Vm[0];
   double dp = Vp[4] - Vm[4];
-  double diff = (Vp[1 + dir] - Vm[1 + dir]) / (r.srm + r.srp);
-  r.p_over_rho_hat = avg(r.srm, Vm[4] / Vm[0], r.srp, Vp[4] / Vp[0]) + 0.5 * diff * diff;
+  double diff = ddiv(Vp[1 + dir] - Vm[1 + dir], r.srm + r.srp);
+  r.p_over_rho_hat = avg(r.srm, ddiv(Vm[4], Vm[0]), r.srp, ddiv(Vp[4], Vp[0])) + 0.5 * diff * diff;
   r.em = eos_e(M, Vm[0], Vm[4]);
   r.ep = eos_e(M, Vp[0], Vp[4]);
   double de = r.ep - r.em;
   r.e_hat = avg(r.srm, r.em, r.srp, r.ep);
-  double w_rho = drho * drho / (r.rho_hat * r.rho_hat);
-  double w_e = de * de / (r.e_hat * r.e_hat);
+  double w_rho = ddiv(drho * drho, r.rho_hat * r.rho_hat);
+  double w_e = ddiv(de * de, r.e_hat * r.e_hat);
   double denom = w_rho + w_e + eps;
   double dpdrho_avg = avg(r.srm, eos_dpdrho(M, Vm[0], r.em), r.srp, eos_dpdrho(M, Vp[0], r.ep));
   double Gamma_avg = avg(r.srm, eos_Gamma(M, Vm[0]), r.srp, eos_Gamma(M, Vp[0]));
   double t1 = (w_e + eps) * dpdrho_avg;
-  double t2 = (dp - Gamma_avg * r.rho_hat * de) * drho / (r.rho_hat * r.rho_hat);
-  r.dpdrho_hat = (t1 + t2) / denom;
+  double t2 = ddiv((dp - Gamma_avg * r.rho_hat * de) * drho, r.rho_hat * r.rho_hat);
+  r.dpdrho_hat = ddiv(t1 + t2, denom);
   double g1 = (w_rho + eps) * Gamma_avg;
-  double g2 = (dp - dpdrho_avg * drho) * de / (r.rho_hat * r.e_hat * r.e_hat);
-  r.Gamma_hat = (g1 + g2) / denom;
+  double g2 = ddiv((dp - dpdrho_avg * drho) * de, r.rho_hat * r.e_hat * r.e_hat);
+  r.Gamma_hat = ddiv(g1 + g2, denom);
   r.c2_hat = r.dpdrho_hat + r.Gamma_hat * r.p_over_rho_hat;
   if (r.c2_hat <= 0) { r.c_hat = eps; r.c2_hat = eps * eps; }
-  else r.c_hat = sqrt(r.c2_hat);
+  else r.c_hat = dsqrt(r.c2_hat);
 }
 
 // FluxFcnHLLC.h:158-192
 M2CG_DEV void hllc_fstar(const DevMat& M, int dir, const double* V, double S, double Sstar, double* F) {
   double velo = V[1 + dir];
-  double rhostar = V[0] * (S - velo) / (S - Sstar);
+  double rhostar = ddiv(V[0] * (S - velo), S - Sstar);
   double U[5];
   prim_to_cons(M, V, U);
   double Us[5];
   Us[0] = 1.0; Us[1] = V[1]; Us[2] = V[2]; Us[3] = V[3];
   Us[1 + dir] = Sstar;
-  Us[4] = U[4] / V[0] + (Sstar - velo) * (Sstar + V[4] / (V[0] * (S - velo)));
+  Us[4] = ddiv(U[4], V[0]) + (Sstar - velo) * (Sstar + ddiv(V[4], V[0] * (S - velo)));
   phys_flux(M, dir, V, F);
 #pragma unroll
   for (int i = 0; i < 5; i++) F[i] += S * (Us[i] * rhostar - U[i]);
@@ -311,8 +326,8 @@ M2CG_DEV bool flux_hllc(const DevMat& M, int dir, const double* Vm, const double
   double cm = eos_c2(M, Vm[0], r.em);
   double cp = eos_c2(M, Vp[0], r.ep);
   bool ok = !(cm < 0.0) && !(cp < 0.0);
-  cm = sqrt(fmax(cm, 0.0));
-  cp = sqrt(fmax(cp, 0.0));
+  cm = dsqrt(fmax(cm, 0.0));
+  cp = dsqrt(fmax(cp, 0.0));
   double vm = Vm[1 + dir], vp = Vp[1 + dir];
   double vh = avg(r.srm, vm, r.srp, vp);
   double Sm = fmin(vm - cm, vh - r.c_hat);
@@ -320,8 +335,8 @@ M2CG_DEV bool flux_hllc(const DevMat& M, int dir, const double* Vm, const double
   if (0.0 <= Sm) phys_flux(M, dir, Vm, F);
   else if (0.0 >= Sp) phys_flux(M, dir, Vp, F);
   else {
-    double Sstar = (Vp[4] - Vm[4] + Vm[0] * vm * (Sm - vm) - Vp[0] * vp * (Sp - vp)) /
-                   (Vm[0] * (Sm - vm) - Vp[0] * (Sp - vp));
+    double Sstar = ddiv(Vp[4] - Vm[4] + Vm[0] * vm * (Sm - vm) - Vp[0] * vp * (Sp - vp),
+                        Vm[0] * (Sm - vm) - Vp[0] * (Sp - vp));
     if (Sstar >= 0.0) hllc_fstar(M, dir, Vm, Sm, Sstar, F);
     else hllc_fstar(M, dir, Vp, Sp, Sstar, F);
   }
@@ -471,8 +486,8 @@ M2CG_DEV bool flux_llf2(const DevMat& Mm, const DevMat& Mp, int dir, const doubl
   double cm = eos_c2(Mm, Vm[0], em);
   double cp = eos_c2(Mp, Vp[0], ep);
   bool ok = !(cm < 0.0) && !(cp < 0.0);
-  cm = sqrt(fmax(cm, 0.0));
-  cp = sqrt(fmax(cp, 0.0));
+  cm = dsqrt(fmax(cm, 0.0));
+  cp = dsqrt(fmax(cp, 0.0));
   double a = fmax(fabs(Vm[1 + dir]) + cm, fabs(Vp[1 + dir]) + cp);
   double fm[5], fp[5], Um[5], Up[5];
   phys_flux(Mm, dir, Vm, fm);
@@ -487,8 +502,8 @@ M2CG_DEV bool flux_llf2(const DevMat& Mm, const DevMat& Mp, int dir, const doubl
 // FluxFcnGenRoe.h:63-221 with the eigenvectors of FluxFcnBase.h:154-176 (F),
 // 203-225 (G), 252-274 (H).
 M2CG_DEV bool flux_genroe(const DevMat& M, int dir, const double* Vm, const double* Vp, double del, double* F) {
-  double srm = sqrt(Vm[0]), srp = sqrt(Vp[0]);
-  double rho_hat = sqrt(Vm[0] * Vp[0]);
+  double srm = dsqrt(Vm[0]), srp = dsqrt(Vp[0]);
+  double rho_hat = dsqrt(Vm[0] * Vp[0]);
   double vel[3];
 #pragma unroll
   for (int m = 0; m < 3; m++) vel[m] = avg(srm, Vm[1 + m], srp, Vp[1 + m]);
@@ -500,19 +515,19 @@ M2CG_DEV bool flux_genroe(const DevMat& M, int dir, const double* Vm, const doub
   double c = r.c_hat, c2 = r.c2_hat;
   double vn = vel[dir];
   double vel2 = vel[0] * vel[0] + vel[1] * vel[1] + vel[2] * vel[2];
-  double e_term = r.e_hat + 0.5 * vel2 - r.dpdrho_hat / r.Gamma_hat;
+  double e_term = r.e_hat + 0.5 * vel2 - ddiv(r.dpdrho_hat, r.Gamma_hat);
   double lam[5] = {vn - c, vn, vn, vn, vn + c};
   double a[5];
-  a[0] = (dp - rho_hat * c * dvel[dir]) / (2 * c2);
-  a[4] = (dp + rho_hat * c * dvel[dir]) / (2 * c2);
+  a[0] = ddiv(dp - rho_hat * c * dvel[dir], 2 * c2);
+  a[4] = ddiv(dp + rho_hat * c * dvel[dir], 2 * c2);
 #pragma unroll
-  for (int p = 1; p <= 3; p++) a[p] = (p - 1 == dir) ? (-dp / c2 + drho) : rho_hat * dvel[p - 1];
+  for (int p = 1; p <= 3; p++) a[p] = (p - 1 == dir) ? (ddiv(-dp, c2) + drho) : rho_hat * dvel[p - 1];
   double tol = lam[0];
 #pragma unroll
   for (int i = 1; i < 5; i++) if (fabs(lam[i]) > tol) tol = fabs(lam[i]);
   tol *= del;
 #pragma unroll
-  for (int i = 0; i < 5; i++) if (fabs(lam[i]) < tol) lam[i] = (lam[i] * lam[i] + tol * tol) / (2 * tol);
+  for (int i = 0; i < 5; i++) if (fabs(lam[i]) < tol) lam[i] = ddiv(lam[i] * lam[i] + tol * tol, 2 * tol);
   double fm[5], fp[5];
   phys_flux(M, dir, Vm, fm);
   phys_flux(M, dir, Vp, fp);

@@ -1,7 +1,7 @@
 // Measurement and self-check helpers: the FP64 pipe peak of this GPU (eight
 // independent binary64 FMA chains per thread, enough warps per SM to hide the
 // pipe's latency; the denominator of the FP64 roofline of the stage kernels)
-// and the bit-exactness check of the shared-reciprocal quotients.
+// and the bit-exactness check of the integer-pipe quotients and roots.
 #include <algorithm>
 #include <cuda_runtime.h>
 #include "m2cg.h"
@@ -98,7 +98,7 @@ __global__ void k_selftest_quotient(int64_t n, uint64_t seed, unsigned long long
         if ((r3 >> 40) & 1) { a = x; b = y; } else { a = y; b = x; }
         break;
       }
-      case 5: {   // exponents at and around the limits of the shared-reciprocal path
+      case 5: {   // exponents at and around 128 and 1920
         const int ea = ((r3 & 1) ? 128 : 1920) + (int)((r3 >> 1) % 9) - 4;
         const int eb = ((r3 >> 8) & 1) ? 1023 + (int)((r3 >> 9) % 1000) - 500 : ((r3 >> 20) & 1 ? 128 : 1920) + (int)((r3 >> 21) % 9) - 4;
         a = with_exp(r1, ea); b = with_exp(r2, eb);
@@ -119,9 +119,16 @@ __global__ void k_selftest_quotient(int64_t n, uint64_t seed, unsigned long long
     const double q = m2cg::qdiv(a, d), ref = a / b;
     const bool both_nan = isnan(q) && isnan(ref);
     if (!both_nan && __double_as_longlong(q) != __double_as_longlong(ref)) bad++;
-    if (d.fast && __double_as_longlong(d.y) != __double_as_longlong(1.0 / b)) bad++;
-    const int ea = m2cg::exp_field(a), eq = ea - m2cg::exp_field(b) + 1023;
-    fast += (d.fast && ea >= 128 && ea <= 1920 && eq >= 128 && eq <= 1920) ? 1 : 0;
+    if (m2cg::qfast(1.0, d) && __double_as_longlong(m2cg::qdiv(1.0, d)) != __double_as_longlong(1.0 / b)) bad++;
+    const double w = fabs(a), root = m2cg::dsqrt(w);
+    if (!isnan(w) && __double_as_longlong(root) != __double_as_longlong(sqrt(w))) bad++;
+    const double dq = m2cg::ddiv(a, b);
+    if (!both_nan && __double_as_longlong(dq) != __double_as_longlong(ref)) bad++;
+    double q2, w2;   // the paired form, also with the other quotient out of range
+    m2cg::ddiv2(a, b, 1.0, w, q2, w2);
+    if (!both_nan && __double_as_longlong(q2) != __double_as_longlong(ref)) bad++;
+    if (!isnan(w) && __double_as_longlong(w2) != __double_as_longlong(1.0 / w)) bad++;
+    fast += m2cg::qfast(a, d) ? 1 : 0;
   }
   if (bad) atomicAdd(&out[0], bad);
   if (fast) atomicAdd(&out[1], fast);

@@ -51,22 +51,21 @@ struct PathCache {
   // below the last one, so the pressures strictly decrease and a binary search
   // finds the same index.
   M2CG_DEV int last_above(double ps) const {
-    if (!(get(0, 0) > ps)) return 0;
+    if (!i_lt(ps, get(0, 0))) return 0;
     int lo = 0, hi = n - 1;  // get(lo, 0) > ps
     while (lo < hi) {
       int mid = (lo + hi + 1) >> 1;
-      if (get(mid, 0) > ps) lo = mid;
+      if (i_lt(ps, get(mid, 0))) lo = mid;
       else hi = mid - 1;
     }
     return lo;
   }
 };
 
-// SharedDiv: the Cash-Karp and RK4 steps form each repeated divisor's
-// reciprocal once (qdiv), for the latency-bound solves of the finite-volume
-// step; false keeps the IEEE divisions (batched independent problems).
-template <bool SharedDiv>
-struct ExactRiemannDevT {
+// Divisions and square roots run on the integer pipe (m2cg_intfp.cuh), bit for
+// bit the IEEE results: a solve is one chain of dependent operations, and an
+// FP64 division holds its SM sub-partition's FP64 unit for 560 cycles.
+struct ExactRiemannDev {
   const Mats* mats;
   RiemannPrm P;
   PathCache path1, path3;
@@ -95,10 +94,9 @@ struct ExactRiemannDevT {
   }
 
   M2CG_DEV const DevMat& mat(int id) const { return mats->m[id]; }
-  // the division policy (shared reciprocals or IEEE divisions, same bits)
-  M2CG_DEV static Quot qof(double b) { return quot_of_t<SharedDiv>(b); }
-  M2CG_DEV static double qd(double a, const Quot& d) { return qdiv_t<SharedDiv>(a, d); }
-  M2CG_DEV static double qr(const Quot& d) { return qrcp_t<SharedDiv>(d); }
+  M2CG_DEV static Quot qof(double b) { return quot_of(b); }
+  M2CG_DEV static double qd(double a, const Quot& d) { return qdiv(a, d); }
+  M2CG_DEV static double qr(const Quot& d) { return qdiv(1.0, d); }
 
   // The sound speed of the state a Runge-Kutta step starts from.  The next
   // step of an integration starts where the last one ended (an accepted step)
@@ -147,7 +145,7 @@ struct ExactRiemannDevT {
   }
   // only after the caller has checked c^2 >= 0
   M2CG_DEV static double side_c(SideMemo& m) {
-    if (!(m.have & 4u)) { m.c = sqrt(side_c2(m)); m.have |= 4u; }
+    if (!(m.have & 4u)) { m.c = dsqrt(side_c2(m)); m.have |= 4u; }
     return m.c;
   }
   M2CG_DEV static double side_dpdrho(SideMemo& m) {
@@ -155,7 +153,7 @@ struct ExactRiemannDevT {
     return m.dpdrho;
   }
   M2CG_DEV static double side_oor(SideMemo& m) {
-    if (!(m.have & 16u)) { m.oor = 1.0 / m.rho; m.have |= 16u; }
+    if (!(m.have & 16u)) { m.oor = ddiv(1.0, m.rho); m.have |= 16u; }
     return m.oor;
   }
   M2CG_DEV static bool memo_hit(const EosMemo& m, const DevMat& M, double rho, double p) {
@@ -180,9 +178,9 @@ struct ExactRiemannDevT {
     double c_0_square, c_0;
     if (!memo_get(M, rho_0, p_0, c_0_square, c_0)) {
       double e_0 = eos_e(M, rho_0, p_0);
-      c_0_square = eos_c2_q<SharedDiv>(M, rho_0, R0, e_0);
-      if (rho_0 <= 0 || c_0_square < 0) return false;
-      c_0 = sqrt(c_0_square);
+      c_0_square = eos_c2_q(M, rho_0, R0, e_0);
+      if (i_le0(rho_0) || i_lt0(c_0_square)) return false;
+      c_0 = dsqrt(c_0_square);
       memo_start = EosMemo{&M, rho_0, p_0, c_0_square, c_0};
     }
     const Quot C0 = qof(c_0_square);
@@ -190,41 +188,41 @@ struct ExactRiemannDevT {
     double p_1 = p_0 + 0.2 * dp;
     double e_1 = eos_e(M, rho_1, p_1);
     double c_1_square = eos_c2(M, rho_1, e_1);
-    if (rho_1 <= 0 || c_1_square < 0) return false;
+    if (i_le0(rho_1) || i_lt0(c_1_square)) return false;
     const Quot C1 = qof(c_1_square);
     double rho_2 = rho_0 + qd(3. / 40. * dp, C0) + qd(9. / 40. * dp, C1);
     double p_2 = p_1 + 3. / 10. * dp;
     double e_2 = eos_e(M, rho_2, p_2);
     const Quot R2 = qof(rho_2);
-    double c_2_square = eos_c2_q<SharedDiv>(M, rho_2, R2, e_2);
-    if (rho_2 <= 0 || c_2_square < 0) return false;
-    double c_2 = sqrt(c_2_square);
+    double c_2_square = eos_c2_q(M, rho_2, R2, e_2);
+    if (i_le0(rho_2) || i_lt0(c_2_square)) return false;
+    double c_2 = dsqrt(c_2_square);
     const Quot C2 = qof(c_2_square);
     double rho_3 = rho_0 + qd(3. / 10. * dp, C0) - qd(9. / 10. * dp, C1) + qd(6. / 5. * dp, C2);
     double p_3 = p_0 + 3. / 5. * dp;
     double e_3 = eos_e(M, rho_3, p_3);
     const Quot R3 = qof(rho_3);
-    double c_3_square = eos_c2_q<SharedDiv>(M, rho_3, R3, e_3);
-    if (rho_3 <= 0 || c_3_square < 0) return false;
-    double c_3 = sqrt(c_3_square);
+    double c_3_square = eos_c2_q(M, rho_3, R3, e_3);
+    if (i_le0(rho_3) || i_lt0(c_3_square)) return false;
+    double c_3 = dsqrt(c_3_square);
     const Quot C3 = qof(c_3_square);
     double rho_4 = rho_0 - qd(11. / 54. * dp, C0) + qd(2.5 * dp, C1) - qd(70. / 27. * dp, C2) +
                    qd(35. / 27. * dp, C3);
     double p_4 = p_0 + dp;
     double e_4 = eos_e(M, rho_4, p_4);
     const Quot R4 = qof(rho_4);
-    double c_4_square = eos_c2_q<SharedDiv>(M, rho_4, R4, e_4);
-    if (rho_4 <= 0 || c_4_square < 0) return false;
-    double c_4 = sqrt(c_4_square);
+    double c_4_square = eos_c2_q(M, rho_4, R4, e_4);
+    if (i_le0(rho_4) || i_lt0(c_4_square)) return false;
+    double c_4 = dsqrt(c_4_square);
     const Quot C4 = qof(c_4_square);
     double rho_5 = rho_0 + qd(1631. / 55296. * dp, C0) + qd(175. / 512. * dp, C1) +
                    qd(575. / 13824. * dp, C2) + qd(44275. / 110592. * dp, C3) + qd(253. / 4096. * dp, C4);
     double p_5 = p_0 + 7. / 8. * dp;
     double e_5 = eos_e(M, rho_5, p_5);
     const Quot R5 = qof(rho_5);
-    double c_5_square = eos_c2_q<SharedDiv>(M, rho_5, R5, e_5);
-    if (rho_5 <= 0 || c_5_square < 0) return false;
-    double c_5 = sqrt(c_5_square);
+    double c_5_square = eos_c2_q(M, rho_5, R5, e_5);
+    if (i_le0(rho_5) || i_lt0(c_5_square)) return false;
+    double c_5 = dsqrt(c_5_square);
     const Quot C5 = qof(c_5_square);
     double drho = (qd(37. / 378., C0) + qd(250. / 621., C2) + qd(125. / 594., C3) + qd(512. / 1771., C5)) * dp;
     double drho_err = (qd(2825. / 27648., C0) + qd(18575. / 48384., C2) + qd(13525. / 55296., C3) +
@@ -233,8 +231,8 @@ struct ExactRiemannDevT {
     double du = (qd(qd(37. / 378., S0), R0) + qd(qd(250. / 621., S2), R2) + qd(qd(125. / 594., S3), R3) +
                  qd(qd(512. / 1771., S5), R5)) * dp;
     double du_err = (qd(qd(2825. / 27648., S0), R0) + qd(qd(18575. / 48384., S2), R2) +
-                     qd(qd(13525. / 55296., S3), R3) + qd(277. / 14336. / c_4, R4) + qd(qd(0.25, S5), R5)) * dp;
-    if (isnan(du) || isnan(du_err)) return false;
+                     qd(qd(13525. / 55296., S3), R3) + qd(ddiv(277. / 14336., c_4), R4) + qd(qd(0.25, S5), R5)) * dp;
+    if (is_nan_bits(du) || is_nan_bits(du_err)) return false;
     rhoErr = fabs(drho_err - drho);
     uErr = fabs(du_err - du);
     rho = rho_0 + drho;
@@ -242,9 +240,9 @@ struct ExactRiemannDevT {
     u = (wave == 1) ? u_0 - du : u_0 + du;
     double e = eos_e(M, rho, p);
     double c = eos_c2(M, rho, e);
-    if (rho <= 0 || c < 0) return false;
+    if (i_le0(rho) || i_lt0(c)) return false;
     const double c2 = c;
-    c = sqrt(c);
+    c = dsqrt(c);
     memo_end = EosMemo{&M, rho, p, c2, c};
     xi = (wave == 1) ? u - c : u + c;
     return true;
@@ -259,9 +257,9 @@ struct ExactRiemannDevT {
     double c_0_square, c_0;
     if (!memo_get(M, rho_0, p_0, c_0_square, c_0)) {
       double e_0 = eos_e(M, rho_0, p_0);
-      c_0_square = eos_c2_q<SharedDiv>(M, rho_0, R0, e_0);
-      if (rho_0 <= 0 || c_0_square < 0) return false;
-      c_0 = sqrt(c_0_square);
+      c_0_square = eos_c2_q(M, rho_0, R0, e_0);
+      if (i_le0(rho_0) || i_lt0(c_0_square)) return false;
+      c_0 = dsqrt(c_0_square);
       memo_start = EosMemo{&M, rho_0, p_0, c_0_square, c_0};
     }
     const Quot C0 = qof(c_0_square);
@@ -269,37 +267,37 @@ struct ExactRiemannDevT {
     double p_1 = p_0 + 0.5 * dp;
     double e_1 = eos_e(M, rho_1, p_1);
     const Quot R1 = qof(rho_1);
-    double c_1_square = eos_c2_q<SharedDiv>(M, rho_1, R1, e_1);
-    if (rho_1 <= 0 || c_1_square < 0) return false;
-    double c_1 = sqrt(c_1_square);
+    double c_1_square = eos_c2_q(M, rho_1, R1, e_1);
+    if (i_le0(rho_1) || i_lt0(c_1_square)) return false;
+    double c_1 = dsqrt(c_1_square);
     const Quot C1 = qof(c_1_square);
     double rho_2 = rho_0 + qd(0.5 * dp, C1);
     double p_2 = p_1;
     double e_2 = eos_e(M, rho_2, p_2);
     const Quot R2 = qof(rho_2);
-    double c_2_square = eos_c2_q<SharedDiv>(M, rho_2, R2, e_2);
-    if (rho_2 <= 0 || c_2_square < 0) return false;
-    double c_2 = sqrt(c_2_square);
+    double c_2_square = eos_c2_q(M, rho_2, R2, e_2);
+    if (i_le0(rho_2) || i_lt0(c_2_square)) return false;
+    double c_2 = dsqrt(c_2_square);
     const Quot C2 = qof(c_2_square);
     double rho_3 = rho_0 + qd(dp, C2);
     double p_3 = p_0 + dp;
     double e_3 = eos_e(M, rho_3, p_3);
     const Quot R3 = qof(rho_3);
-    double c_3_square = eos_c2_q<SharedDiv>(M, rho_3, R3, e_3);
-    if (rho_3 <= 0 || c_3_square < 0) return false;
-    double c_3 = sqrt(c_3_square);
-    double drho = 1.0 / 6.0 * dp * (qr(C0) + 2.0 * (qr(C1) + qr(C2)) + 1. / c_3_square);
+    double c_3_square = eos_c2_q(M, rho_3, R3, e_3);
+    if (i_le0(rho_3) || i_lt0(c_3_square)) return false;
+    double c_3 = dsqrt(c_3_square);
+    double drho = 1.0 / 6.0 * dp * (qr(C0) + 2.0 * (qr(C1) + qr(C2)) + ddiv(1., c_3_square));
     double du = 1.0 / 6.0 * dp *
-                (qd(1. / c_0, R0) + 2.0 * (qd(1. / c_1, R1) + qd(1. / c_2, R2)) + qd(1. / c_3, R3));
-    if (isnan(du)) return false;
+                (qd(ddiv(1., c_0), R0) + 2.0 * (qd(ddiv(1., c_1), R1) + qd(ddiv(1., c_2), R2)) + qd(ddiv(1., c_3), R3));
+    if (is_nan_bits(du)) return false;
     rho = rho_0 + drho;
     p = p_0 + dp;
     u = (wave == 1) ? u_0 - du : u_0 + du;
     double e = eos_e(M, rho, p);
     double c = eos_c2(M, rho, e);
-    if (rho <= 0 || c < 0) return false;
+    if (i_le0(rho) || i_lt0(c)) return false;
     const double c2 = c;
-    c = sqrt(c);
+    c = dsqrt(c);
     memo_end = EosMemo{&M, rho, p, c2, c};
     xi = (wave == 1) ? u - c : u + c;
     return true;
@@ -311,27 +309,27 @@ struct ExactRiemannDevT {
                                                  double* Vrare) {
     double rhos_0 = rho, us_0 = u, ps_0 = p, xi_0;
     double rhos_1 = rho, us_1 = u, ps_1 = p, xi_1 = 0;
-    double dp_target = (p - ps) / P.numSteps;
+    double dp_target = ddiv(p - ps, P.numSteps);
     SideMemo& sm = side(wave, M, rho, p);
     double dpdrho = side_dpdrho(sm);
-    double drho_op1 = (p - ps) / dpdrho / P.numSteps;
-    double drho_op2 = rho / (2.5 * P.numSteps);
-    double drho_target = fmin(drho_op1, drho_op2);
-    double dp = fmin(dp_target, drho_target * dpdrho);
-    double tol_end = P.tol_rare * fmax(1.0, fabs(p));
+    double drho_op1 = ddiv(ddiv(p - ps, dpdrho), P.numSteps);
+    double drho_op2 = ddiv(rho, 2.5 * P.numSteps);
+    double drho_target = i_min(drho_op1, drho_op2);
+    double dp = i_min(dp_target, drho_target * dpdrho);
+    double tol_end = P.tol_rare * i_max(1.0, fabs(p));
     double c = side_c2(sm);
-    if (rho <= 0 || c < 0) return false;
+    if (i_le0(rho) || i_lt0(c)) return false;
     c = side_c(sm);
     if (path.n > 1) {
       int index0 = path.last_above(ps);
       ps_0 = path.get(index0, 0);
       rhos_0 = path.get(index0, 1);
       us_0 = path.get(index0, 2);
-      dp = fmin((p - ps) / P.numSteps, ps_0 - ps);
+      dp = i_min(ddiv(p - ps, P.numSteps), ps_0 - ps);
     }
     xi_0 = (wave == 1) ? u - c : u + c;
     for (int i = 0; i < P.numSteps * 5; i++) {
-      if (fabs(ps_1 - ps) <= tol_end) {
+      if (i_le(fabs(ps_1 - ps), tol_end)) {
         rhos = rhos_1;
         us = us_1;
         return !eos_bad(M, rhos, ps);
@@ -342,28 +340,35 @@ struct ExactRiemannDevT {
         if (dp == 0.0) break;
         continue;
       }
-      if (ps_1 - ps < -tol_end) { dp = ps_0 - ps; continue; }
-      if (ps_1 < path.get(path.n - 1, 0)) path.push(ps_1, rhos_1, us_1);
-      if (trans_rare && Vrare && xi_0 * xi_1 <= 0) {
+      if (i_lt(ps_1 - ps, -tol_end)) { dp = ps_0 - ps; continue; }
+      if (i_lt(ps_1, path.get(path.n - 1, 0))) path.push(ps_1, rhos_1, us_1);
+      if (trans_rare && Vrare && i_le0(xi_0 * xi_1)) {
         *trans_rare = true;
         double w0 = fabs(xi_1), w1 = fabs(xi_0);
         double ww = w0 + w1;
-        w0 /= ww;
-        w1 /= ww;
+        w0 = ddiv(w0, ww);
+        w1 = ddiv(w1, ww);
         Vrare[0] = w0 * rhos_0 + w1 * rhos_1;
         Vrare[1] = w0 * us_0 + w1 * us_1;
         Vrare[2] = w0 * ps_0 + w1 * ps_1;
       }
-      dp = fmin(fmin(dp_target, ps_1 - ps), 4.0 * dp);
+      dp = i_min(i_min(dp_target, ps_1 - ps), 4.0 * dp);
       rhos_0 = rhos_1; us_0 = us_1; ps_0 = ps_1; xi_0 = xi_1;
     }
     return false;
   }
 
-  // Hugoniot residual, ExactRiemannSolverBase.h:66-83
-  M2CG_DEV double hugo(const DevMat& M, double e, double pavg, double one_over_rho, double ps, double rhos) const {
-    double es = eos_e(M, rhos, ps);
-    return es - e + pavg * (1.0 / rhos - one_over_rho);
+  // Hugoniot residual, ExactRiemannSolverBase.h:66-83.  A stiffened gas's two
+  // divisions are independent: their integer chains run interleaved.
+  __device__ __noinline__ static double hugo(const DevMat& M, double e, double pavg, double one_over_rho, double ps,
+                                             double rhos) {
+    double es, oors;
+    if (M.type == M2CG_EOS_SG) ddiv2(ps + M.gamPs, M.gam1 * rhos, 1.0, rhos, es, oors);
+    else if (M.type == M2CG_EOS_NASG) {   // 1 / rho serves both terms
+      oors = ddiv(1.0, rhos);
+      es = M.invgam1 * (ps + M.gamPs) * (oors - M.b) + M.q;
+    } else { es = eos_e(M, rhos, ps); oors = ddiv(1.0, rhos); }
+    return es - e + pavg * (oors - one_over_rho);
   }
 
   // ExactRiemannSolverBase.cpp:1212-1624
@@ -372,16 +377,16 @@ struct ExactRiemannDevT {
     const DevMat& M = mat(id);
     rhos = rho;
     us = u;
-    if (p > ps && nonadaptive) return rarefaction_fixed(wave, path, M, rho, u, p, ps, rhos, us, trans_rare, Vrare);
-    if (p > ps) {
+    if (i_lt(ps, p) && nonadaptive) return rarefaction_fixed(wave, path, M, rho, u, p, ps, rhos, us, trans_rare, Vrare);
+    if (i_lt(ps, p)) {
       double rhos_0 = rho, us_0 = u, ps_0 = p, xi_0;
       double rhos_1 = rho, us_1 = u, ps_1 = p, xi_1 = 0;
-      double dp = (p - ps) / P.numSteps;
-      double dp_min = dp / 2.5;
-      double tol_end = P.tol_rare * fmax(1.0, fabs(p));
+      double dp = ddiv(p - ps, P.numSteps);
+      double dp_min = ddiv(dp, 2.5);
+      double tol_end = P.tol_rare * i_max(1.0, fabs(p));
       SideMemo& sm = side(wave, M, rho, p);
       double c = side_c2(sm);
-      if (rho <= 0 || c < 0) return false;
+      if (i_le0(rho) || i_lt0(c)) return false;
       c = side_c(sm);
       int index0 = 0;
       if (path.n > 1) {
@@ -389,9 +394,9 @@ struct ExactRiemannDevT {
         ps_0 = path.get(index0, 0);
         rhos_0 = path.get(index0, 1);
         us_0 = path.get(index0, 2);
-        dp_min = (ps_0 - ps) / P.numSteps / 2.5;
+        dp_min = ddiv(ddiv(ps_0 - ps, P.numSteps), 2.5);
         if (index0 != path.n - 1) dp = ps_0 - ps;
-        else dp = fmin(path.get(index0 - 1, 0) - path.get(index0, 0), ps_0 - ps);
+        else dp = i_min(path.get(index0 - 1, 0) - path.get(index0, 0), ps_0 - ps);
       }
       double xi = (wave == 1) ? u - c : u + c;
       xi_0 = xi;
@@ -399,7 +404,7 @@ struct ExactRiemannDevT {
       double uErr = 0., rhoErr = 0.;
       const double errBar = fmax(1.0e-8, fmin(1.0e-5, 100.0 * P.tol_rare));
       for (int i = 0; i < P.numSteps * 3; i++) {
-        if (fabs(ps_1 - ps) <= tol_end) {
+        if (i_le(fabs(ps_1 - ps), tol_end)) {
           rhos = rhos_1;
           us = us_1;
           if (eos_bad(M, rhos, ps)) return false;
@@ -408,29 +413,29 @@ struct ExactRiemannDevT {
         }
         bool ok = rk45(wave, M, rhos_0, us_0, ps_0, dp, rhos_1, us_1, ps_1, xi_1, uErr, rhoErr);
         if (!ok) { dp = dp / 2.0; continue; }
-        if (ps_1 - ps < -tol_end) { dp = ps_0 - ps; continue; }
-        double uS = uErr / c + 1.e-30;
-        double rS = rhoErr / rho + 1.e-30;
-        if (isnan(rS) || isnan(uS)) return false;
-        if (rS >= errBar && dp > dp_min) {
-          double t = 0.9 * dp * pow(fabs(errBar / rS), 0.25);
-          t = fmax(fmax(t, 0.2 * dp), dp_min);
-          dp = fmin(t, ps_0 - ps);
+        if (i_lt(ps_1 - ps, -tol_end)) { dp = ps_0 - ps; continue; }
+        double uS = ddiv(uErr, c) + 1.e-30;
+        double rS = ddiv(rhoErr, rho) + 1.e-30;
+        if (is_nan_bits(rS) || is_nan_bits(uS)) return false;
+        if (i_le(errBar, rS) && i_lt(dp_min, dp)) {
+          double t = 0.9 * dp * pow(fabs(ddiv(errBar, rS)), 0.25);
+          t = i_max(i_max(t, 0.2 * dp), dp_min);
+          dp = i_min(t, ps_0 - ps);
           continue;
         }
-        if (uS >= errBar && dp > dp_min) {
-          double t = 0.9 * dp * pow(fabs(errBar / uS), 0.25);
-          t = fmax(fmax(t, 0.2 * dp), dp_min);
-          dp = fmin(t, ps_0 - ps);
+        if (i_le(errBar, uS) && i_lt(dp_min, dp)) {
+          double t = 0.9 * dp * pow(fabs(ddiv(errBar, uS)), 0.25);
+          t = i_max(i_max(t, 0.2 * dp), dp_min);
+          dp = i_min(t, ps_0 - ps);
           continue;
         }
-        if (ps_1 < path.get(path.n - 1, 0)) path.push(ps_1, rhos_1, us_1);
-        if (trans_rare && Vrare && xi_0 * xi_1 <= 0) {
+        if (i_lt(ps_1, path.get(path.n - 1, 0))) path.push(ps_1, rhos_1, us_1);
+        if (trans_rare && Vrare && i_le0(xi_0 * xi_1)) {
           *trans_rare = true;
           double w0 = fabs(xi_1), w1 = fabs(xi_0);
           double ww = w0 + w1;
-          w0 /= ww;
-          w1 /= ww;
+          w0 = ddiv(w0, ww);
+          w1 = ddiv(w1, ww);
           Vrare[0] = w0 * rhos_0 + w1 * rhos_1;
           Vrare[1] = w0 * us_0 + w1 * us_1;
           Vrare[2] = w0 * ps_0 + w1 * ps_1;
@@ -438,13 +443,13 @@ struct ExactRiemannDevT {
         // the next step size; skipped when the next pass ends the loop and
         // never reads it (the common case of a solve that restarts from the
         // path cache: one step to the end point)
-        if (!(fabs(ps_1 - ps) <= tol_end) && i + 1 < P.numSteps * 3) {
-          double tr = 0.9 * dp * pow(fabs(errBar / rS), 0.2);
-          double tu = 0.9 * dp * pow(fabs(errBar / uS), 0.2);
-          double t = fmin(tr, tu);
-          t = fmin(t, 10 * dp);
-          t = fmax(t, dp_min);
-          dp = fmin(t, ps_1 - ps);
+        if (!i_le(fabs(ps_1 - ps), tol_end) && i + 1 < P.numSteps * 3) {
+          double tr = 0.9 * dp * pow(fabs(ddiv(errBar, rS)), 0.2);
+          double tu = 0.9 * dp * pow(fabs(ddiv(errBar, uS)), 0.2);
+          double t = i_min(tr, tu);
+          t = i_min(t, 10 * dp);
+          t = i_max(t, dp_min);
+          dp = i_min(t, ps_1 - ps);
         }
         rhos_0 = rhos_1; us_0 = us_1; ps_0 = ps_1; xi_0 = xi_1;
       }
@@ -455,18 +460,18 @@ struct ExactRiemannDevT {
       double pavg = 0.5 * (p + ps);
       double oor = side_oor(sm);
       double f0, f1;
-      double drho = fmax(fabs(rhos0 - rhos1), 0.001 * rhos0);
+      double drho = i_max(fabs(rhos0 - rhos1), 0.001 * rhos0);
       bool found0 = false, found1 = false;
-      if (fmin(rhos0, rhos1) >= rho) {
+      if (i_le(rho, i_min(rhos0, rhos1))) {
         f0 = hugo(M, e, pavg, oor, ps, rhos0);
         f1 = hugo(M, e, pavg, oor, ps, rhos1);
-        if (f0 * f1 <= 0) {
-          if (rhos0 > rhos1) { double t = rhos0; rhos0 = rhos1; rhos1 = t; t = f0; f0 = f1; f1 = t; }
+        if (i_le0(f0 * f1)) {
+          if (i_lt(rhos1, rhos0)) { double t = rhos0; rhos0 = rhos1; rhos1 = t; t = f0; f0 = f1; f1 = t; }
           found0 = found1 = true;
         } else { rhos0 = rhos1; f0 = f1; }
       } else {
-        if (rhos1 > rhos0) { rhos0 = rhos1; f0 = hugo(M, e, pavg, oor, ps, rhos0); }
-        if (rhos0 < rho) { rhos0 = rho; f0 = hugo(M, e, pavg, oor, ps, rhos0); found0 = true; }
+        if (i_lt(rhos0, rhos1)) { rhos0 = rhos1; f0 = hugo(M, e, pavg, oor, ps, rhos0); }
+        if (i_lt(rhos0, rho)) { rhos0 = rho; f0 = hugo(M, e, pavg, oor, ps, rhos0); found0 = true; }
         else f0 = hugo(M, e, pavg, oor, ps, rhos0);
       }
       if (!found0 || !found1) {
@@ -480,16 +485,16 @@ struct ExactRiemannDevT {
           tmp = rhos1; ftmp = f1;
           rhos1 = rhos0; f1 = f0;
           rhos0 = rhos1 - factor * drho;
-          if (rhos0 <= rho) { rhos0 = rho; found0 = true; }
+          if (i_le(rhos0, rho)) { rhos0 = rho; found0 = true; }
           f0 = hugo(M, e, pavg, oor, ps, rhos0);
-          if (f0 * f1 <= 0) found0 = found1 = true;
+          if (i_le0(f0 * f1)) found0 = found1 = true;
           else {
             rhos1 = tmp; f1 = ftmp;
             tmp = rhos0; ftmp = f0;
             rhos0 = rhos1; f0 = f1;
             rhos1 = rhos0 + factor * drho;
             f1 = hugo(M, e, pavg, oor, ps, rhos1);
-            if (f0 * f1 <= 0) found0 = found1 = true;
+            if (i_le0(f0 * f1)) found0 = found1 = true;
             else { rhos0 = tmp; f0 = ftmp; drho = rhos1 - rhos0; }
           }
         }
@@ -500,35 +505,36 @@ struct ExactRiemannDevT {
             rhos0 = rhos1; f0 = f1;
             rhos1 = rhos0 + 2.5 * drho;
             f1 = hugo(M, e, pavg, oor, ps, rhos1);
-            if (f0 * f1 <= 0) found1 = true;
+            if (i_le0(f0 * f1)) found1 = true;
             else drho = rhos1 - rhos0;
           }
         }
       }
-      double loc_tol = P.tol_shock * fmin(rhos0, rhos1);
+      double loc_tol = P.tol_shock * i_min(rhos0, rhos1);
       double s_first = 0, s_second = 0;
-      if (f0 == 0.0) s_first = s_second = rhos0;
-      else if (f1 == 0.0) s_first = s_second = rhos1;
+      if (i_eq0(f0)) s_first = s_second = rhos0;
+      else if (i_eq0(f1)) s_first = s_second = rhos1;
       else {
         double rhos2 = rhos1, f2 = f1;
+        drho = rhos1 - rhos0;
         int it;
         for (it = 0; it < P.maxIts_shock; it++) {
-          drho = rhos1 - rhos0;
-          rhos2 = rhos2 - f2 * (rhos1 - rhos0) / (f1 - f0);
-          if (rhos2 >= rhos1 || rhos2 <= rhos0) rhos2 = rhos0 + 0.5 * (rhos1 - rhos0);
+          rhos2 = rhos2 - ddiv(f2 * drho, f1 - f0);
+          if (i_le(rhos1, rhos2) || i_le(rhos2, rhos0)) rhos2 = rhos0 + 0.5 * drho;
           f2 = hugo(M, e, pavg, oor, ps, rhos2);
-          if (f2 == 0.0) { s_first = s_second = rhos2; break; }
-          if (f2 * f0 < 0) { rhos1 = rhos2; f1 = f2; }
+          if (i_eq0(f2)) { s_first = s_second = rhos2; break; }
+          if (i_prod_lt0(f2, f0)) { rhos1 = rhos2; f1 = f2; }
           else { rhos0 = rhos2; f0 = f2; }
-          if (rhos1 - rhos0 < loc_tol) { s_first = rhos0; s_second = rhos1; break; }
+          drho = rhos1 - rhos0;
+          if (i_lt(drho, loc_tol)) { s_first = rhos0; s_second = rhos1; break; }
         }
         if (it == P.maxIts_shock) return false;
       }
       rhos = 0.5 * (s_first + s_second);
-      double du = -(ps - p) * (1.0 / rhos - 1.0 / rho);
-      if (du < 0) return false;
+      double du = -(ps - p) * (ddiv(1.0, rhos) - side_oor(sm));
+      if (i_lt0(du)) return false;
       if (eos_bad(M, rhos, ps)) return false;
-      us = (wave == 1) ? u - sqrt(du) : u + sqrt(du);
+      us = (wave == 1) ? u - dsqrt(du) : u + dsqrt(du);
     }
     return true;
   }
@@ -546,12 +552,12 @@ struct ExactRiemannDevT {
                         double cr, int idr, double& p0, double& rhol0, double& rhor0, double& ul0, double& ur0,
                         double& p1, double& rhol1, double& rhor1, double& ul1, double& ur1) {
     double Cl = rhol * cl, Cr = rhor * cr;
-    p0 = (Cr * pl + Cl * pr + Cl * Cr * (ul - ur)) / (Cl + Cr);
+    p0 = ddiv(Cr * pl + Cl * pr + Cl * Cr * (ul - ur), Cl + Cr);
     // the prediction replaces the acoustic estimate only where the acoustic
     // pressure jump exceeds warm_gate times the impedance-weighted pressure:
     // the linearization's error grows like the square of that ratio, and
     // below it acoustic theory is closer than the network
-    const double pbar = (Cr * pl + Cl * pr) / (Cl + Cr);
+    const double pbar = ddiv(Cr * pl + Cl * pr, Cl + Cr);
     warm_used = warm_p > 0.0 && fabs(p0 - pbar) > P.warm_gate * fabs(pbar);
     if (warm_used) {
       // learned warm start: the two starting points bracket the prediction,
@@ -570,11 +576,11 @@ struct ExactRiemannDevT {
     evals++;
     if (!rho_u_star(1, path1, rhol, ul, pl, p0, idl, rhol, (p0 > pl) ? rhol * 1.1 : rhol * 0.9, rhol0, ul0, nullptr, nullptr)) return 0;
     if (!rho_u_star(3, path3, rhor, ur, pr, p0, idr, rhor, (p0 > pr) ? rhor * 1.1 : rhor * 0.9, rhor0, ur0, nullptr, nullptr)) return 0;
-    double Clbar = (ul0 == ul) ? Cl : fabs(p0 - pl) / fabs(ul0 - ul);
-    double Crbar = (ur0 == ur) ? Cr : fabs(p0 - pr) / fabs(ur0 - ur);
-    p1 = (Crbar * pl + Clbar * pr + Clbar * Crbar * (ul - ur)) / (Clbar + Crbar);
+    double Clbar = (ul0 == ul) ? Cl : ddiv(fabs(p0 - pl), fabs(ul0 - ul));
+    double Crbar = (ur0 == ur) ? Cr : ddiv(fabs(p0 - pr), fabs(ur0 - ur));
+    p1 = ddiv(Crbar * pl + Clbar * pr + Clbar * Crbar * (ul - ur), Clbar + Crbar);
     double tmp = fmax(fabs(p0), fabs(p1));
-    if (fabs(p1 - p0) / tmp < 1.0e-8) p1 = p0 + 1.0e-8 * tmp;
+    if (ddiv(fabs(p1 - p0), tmp) < 1.0e-8) p1 = p0 + 1.0e-8 * tmp;
     evals++;
     if (!rho_u_star(1, path1, rhol, ul, pl, p1, idl, rhol, rhol0, rhol1, ul1, nullptr, nullptr)) return 1;
     if (!rho_u_star(3, path3, rhor, ur, pr, p1, idr, rhor, rhor0, rhor1, ur1, nullptr, nullptr)) return 1;
@@ -654,7 +660,7 @@ struct ExactRiemannDevT {
       if (f0 * f1 <= 0.0) return true;
       if (warm_used && i >= P.warm_tries) { warm_miss = true; return false; }
       if (fabs(f0 - f1) > 1e-9) {
-        p2 = p1 - f1 * (p1 - p0) / (f1 - f0);
+        p2 = p1 - ddiv(f1 * (p1 - p0), f1 - f0);
         if (p2 < p0) p2 -= 0.1 * (p1 - p0);
         else p2 += 0.1 * (p1 - p0);
       } else p2 = 1.1 * p1;
@@ -703,18 +709,18 @@ struct ExactRiemannDevT {
       bool star = false;
       if (pl >= p2) {
         const DevMat& M = mat(idl);
-        double cl2 = sqrt(fmax(eos_c2(M, rhol2, eos_e(M, rhol2, p2)), 0.0));
+        double cl2 = dsqrt(fmax(eos_c2(M, rhol2, eos_e(M, rhol2, p2)), 0.0));
         if (u2 - cl2 <= 0) star = true;
-      } else if ((rhol2 * u2 - rhol * ul) / (rhol2 - rhol) <= 0) star = true;
+      } else if (ddiv(rhol2 * u2 - rhol * ul, rhol2 - rhol) <= 0) star = true;
       if (star) { Vs[0] = rhol2; Vs[1] = u2 * dir[0]; Vs[2] = u2 * dir[1]; Vs[3] = u2 * dir[2]; Vs[4] = p2; }
       else { Vs[0] = rhol; Vs[1] = ul * dir[0]; Vs[2] = ul * dir[1]; Vs[3] = ul * dir[2]; Vs[4] = pl; }
     } else {
       bool star = false;
       if (pr >= p2) {
         const DevMat& M = mat(idr);
-        double cr2 = sqrt(fmax(eos_c2(M, rhor2, eos_e(M, rhor2, p2)), 0.0));
+        double cr2 = dsqrt(fmax(eos_c2(M, rhor2, eos_e(M, rhor2, p2)), 0.0));
         if (u2 - cr2 >= 0) star = true;
-      } else if ((rhor2 * u2 - rhor * ur) / (rhor2 - rhor) >= 0) star = true;
+      } else if (ddiv(rhor2 * u2 - rhor * ur, rhor2 - rhor) >= 0) star = true;
       if (star) { Vs[0] = rhor2; Vs[1] = u2 * dir[0]; Vs[2] = u2 * dir[1]; Vs[3] = u2 * dir[2]; Vs[4] = p2; }
       else { Vs[0] = rhor; Vs[1] = ur * dir[0]; Vs[2] = ur * dir[1]; Vs[3] = ur * dir[2]; Vs[4] = pr; }
     }
@@ -780,8 +786,8 @@ struct ExactRiemannDevT {
       id = idl;
       return -1;
     }
-    cl = sqrt(cl);
-    cr = sqrt(cr);
+    cl = dsqrt(cl);
+    cr = dsqrt(cr);
     double p0 = DBL_MIN, ul0 = 0, ur0 = 0, rhol0 = DBL_MIN, rhor0 = DBL_MIN;
     double p1 = DBL_MIN, ul1 = 0, ur1 = 0, rhol1 = DBL_MIN, rhor1 = DBL_MIN;
     double p2 = DBL_MIN, ul2 = 0, ur2 = 0, rhol2 = DBL_MIN, rhor2 = DBL_MIN;
@@ -816,13 +822,14 @@ struct ExactRiemannDevT {
     // the stopping rule's two denominators do not change during the loop
     const Quot Qp = qof(fmax(fabs(pl + 0.5 * rhol * ul * ul), fabs(pr + 0.5 * rhor * ur * ur)));
     const Quot Qc = qof(fmax(cl, cr));
+    const double tol_either = P.tol_main * 1e-3;
     int iter;
     for (iter = 0; iter < P.maxIts_main; iter++) {
       double denom = f1 - f0;
-      if (denom == 0) p2 = p0 + 0.5 * (p1 - p0);
+      if (i_eq0(denom)) p2 = p0 + 0.5 * (p1 - p0);
       else {
-        p2 = p2 - f2 * (p1 - p0) / denom;
-        if (p2 <= p0 || p2 >= p1) p2 = p0 + 0.5 * (p1 - p0);
+        p2 = p2 - ddiv(f2 * (p1 - p0), denom);
+        if (i_le(p2, p0) || i_le(p1, p2)) p2 = p0 + 0.5 * (p1 - p0);
       }
       // the reference's "try_again" loop (ExactRiemannSolverBase.cpp:239-278)
       bool pass = false;
@@ -846,11 +853,11 @@ struct ExactRiemannDevT {
       }
       if (!pass) break;
       f2 = ul2 - ur2;
-      if (f0 * f2 < 0.0) { p1 = p2; f1 = f2; rhol1 = rhol2; rhor1 = rhor2; }
+      if (i_prod_lt0(f0, f2)) { p1 = p2; f1 = f2; rhol1 = rhol2; rhor1 = rhor2; }
       else { p0 = p2; f0 = f2; rhol0 = rhol2; rhor0 = rhor2; }
       double err_p = qd(fabs(p1 - p0), Qp);
       double err_u = qd(fabs(f2), Qc);
-      if ((err_p < P.tol_main && err_u < P.tol_main) || (err_p < P.tol_main * 1e-3) || (err_u < P.tol_main * 1e-3)) break;
+      if ((i_lt(err_p, P.tol_main) && i_lt(err_u, P.tol_main)) || i_lt(err_p, tol_either) || i_lt(err_u, tol_either)) break;
       trans_rare = false;
     }
     finalize(dir, Vm, Vp, rhol, ul, pl, idl, rhor, ur, pr, idr, rhol2, rhor2, 0.5 * (ul2 + ur2), p2, trans_rare, Vrare,
@@ -858,7 +865,5 @@ struct ExactRiemannDevT {
     return (iter == P.maxIts_main) ? 1 : 0;
   }
 };
-using ExactRiemannDev = ExactRiemannDevT<false>;
-using ExactRiemannChainDev = ExactRiemannDevT<true>;
 
 }  // namespace m2cg
