@@ -166,6 +166,21 @@ M2CG_INT_SLOW double ddiv(double a, double b) {
   const uint64_t D = if_sig(if_hi(b), if_lo(b));
   return if_div_core(a, b, D, if_recip(D));
 }
+// ddiv for a chain that waits for each result (few active lanes): where the
+// estimate's error bound cannot reach the next 54-bit quotient, the remainder
+// is skipped (97 % of the quotients).
+M2CG_INT_SLOW double ddiv_lat(double a, double b) {
+  if (!if_div_range(a, b)) return a / b;
+  const uint32_t ah = if_hi(a), al = if_lo(a), bh = if_hi(b);
+  const uint64_t D = if_sig(bh, if_lo(b));
+  const uint64_t T = if_mulhi64(if_sig(ah, al), if_recip(D));
+  const uint32_t s = ((uint32_t)(T >> 62) ^ 1u) & 1u;
+  uint64_t Q = T >> (9u - s);
+  if ((((uint32_t)T + 8u) & (0x1ffu >> s)) < 8u)   // the floor of T + 8 may be one more
+    Q += ((uint64_t)(al << (21u + s)) << 32) - Q * (D >> 11) >= (D >> 11) ? 1u : 0u;
+  return if_pack(((ah ^ bh) & 0x80000000u) + ((((ah >> 20) & 0x7ffu) - ((bh >> 20) & 0x7ffu) + 1022u - s) << 20),
+                 (Q + 1u) >> 1);
+}
 M2CG_INT void ddiv2(double a, double b, double c, double d, double& q, double& r) {
   const bool ok = if_div_range(a, b) && if_div_range(c, d);
   const uint64_t D = if_sig(if_hi(b), if_lo(b)), E = if_sig(if_hi(d), if_lo(d));

@@ -62,10 +62,36 @@ struct PathCache {
   }
 };
 
+// Cash-Karp coefficients by lane for rk45_coop (0: the lane takes no part).
+// rk45_a[k]: quotients by c_k^2 -- lanes 0..4 stage densities (times dp), 5 the
+// density increment, 6 its error estimate; rk45_p: stage pressures; rk45_u and
+// rk45_stage: the velocity terms' coefficients and stages.
+static __device__ const double rk45_a[6][8] = {
+    {0.2, 3. / 40., 3. / 10., -(11. / 54.), 1631. / 55296., 37. / 378., 2825. / 27648., 0.},
+    {0., 9. / 40., -(9. / 10.), 2.5, 175. / 512., 0., 0., 0.},
+    {0., 0., 6. / 5., -(70. / 27.), 575. / 13824., 250. / 621., 18575. / 48384., 0.},
+    {0., 0., 0., 35. / 27., 44275. / 110592., 125. / 594., 13525. / 55296., 0.},
+    {0., 0., 0., 0., 253. / 4096., 0., 277. / 14336., 0.},
+    {0., 0., 0., 0., 0., 512. / 1771., 0.25, 0.}};
+static __device__ const double rk45_p[8] = {0.2, 3. / 10., 3. / 5., 1., 7. / 8., 1., 1., 1.};
+static __device__ const double rk45_u[9] = {37. / 378.,      250. / 621.,     125. / 594.,     512. / 1771., 2825. / 27648.,
+                                            18575. / 48384., 13525. / 55296., 277. / 14336., 0.25};
+static __device__ const int rk45_stage[9] = {0, 2, 3, 5, 0, 2, 3, 4, 5};
+
 // Divisions and square roots run on the integer pipe (m2cg_intfp.cuh), bit for
 // bit the IEEE results: a solve is one chain of dependent operations, and an
 // FP64 division holds its SM sub-partition's FP64 unit for 560 cycles.
-struct ExactRiemannDev {
+//
+// Coop: the 32 lanes of a warp solve one problem together.  They all follow
+// the same path on the same values (an FP64 instruction holds the pipe for 64
+// cycles whatever the number of active lanes, so the redundancy is free), and
+// where the reference's formulas have several independent quotients, roots,
+// powers or sums, each lane forms one of them and a shuffle hands it on.  The
+// operations and their order per value are the same: the same bits.  A solve's
+// latency falls to a half to a third; a warp of 32 independent problems
+// (Coop = false) has the higher throughput.
+template <bool Coop>
+struct ExactRiemannDevT {
   const Mats* mats;
   RiemannPrm P;
   PathCache path1, path3;
@@ -94,6 +120,8 @@ struct ExactRiemannDev {
   }
 
   M2CG_DEV const DevMat& mat(int id) const { return mats->m[id]; }
+  M2CG_DEV static int lane() { return (int)(threadIdx.x & 31u); }
+  M2CG_DEV static double bc(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
   M2CG_DEV static Quot qof(double b) { return quot_of(b); }
   M2CG_DEV static double qd(double a, const Quot& d) { return qdiv(a, d); }
   M2CG_DEV static double qr(const Quot& d) { return qdiv(1.0, d); }
@@ -167,12 +195,130 @@ struct ExactRiemannDev {
     return false;
   }
 
+  // c^2 at (rho, p): eos_e then eos_c2, a Noble-Abel gas's independent
+  // quotients in separate lanes.
+  __device__ __noinline__ static double c2_coop(const DevMat& M, double rho, double p) {
+    if (M.type == M2CG_EOS_SG) {
+      const double g = M.gam1 * rho;
+      const double e = ddiv_lat(p + M.gamPs, g);
+      return M.gam1 * e + ddiv_lat(g * e - M.gamPs, rho) * M.gam1;
+    }
+    if (M.type == M2CG_EOS_NASG) {
+      const double V = ddiv_lat(1.0, rho), vb = V - M.b;
+      const double e1 = (M.invgam1 * (p + M.gamPs) * vb + M.q) - M.q;
+      const int l = lane();
+      const double n1 = M.gam1 * V * V * e1, d1 = vb * vb, d2 = 1.0 - M.b * rho, n0 = M.gam1 * e1;
+      const double q = ddiv_lat(l == 0 ? n0 : l == 1 ? n1 : M.gam1, l == 0 ? vb : l == 1 ? d1 : d2);
+      return bc(q, 1) + ddiv_lat(bc(q, 0) - M.gamPs, rho) * bc(q, 2);
+    }
+    return eos_c2(M, rho, eos_e(M, rho, p));
+  }
+
+  // rk45 by a warp.  Lane j < 5 accumulates stage j + 1's density, lanes 5 and 6
+  // the density increment and its error estimate, one quotient per lane and
+  // stage; then nine lanes hold the terms of the velocity increment and of its
+  // error estimate.
+  __device__ __noinline__ bool rk45_coop(int wave, const DevMat& M, double rho_0, double u_0, double p_0, double dp,
+                                         double& rho, double& u, double& p, double& xi, double& uErr,
+                                         double& rhoErr) const {
+    const int l = lane(), j = l < 8 ? l : 7, j9 = l < 9 ? l : 8;
+    dp = -dp;
+    const double md = rk45_p[j] * dp;
+    double pk = p_0 + md;
+    const double p2 = bc(pk, 0) + md;   // p_2 = p_1 + 3/10 dp
+    if (j == 1) pk = p2;
+    double c2, c0;
+    if (!memo_get(M, rho_0, p_0, c2, c0)) {
+      c2 = c2_coop(M, rho_0, p_0);
+      if (i_le0(rho_0) || i_lt0(c2)) return false;
+      memo_start = EosMemo{&M, rho_0, p_0, c2, dsqrt(c2)};
+    }
+    double S = j < 5 ? rho_0 : 0.0, cq = c2, rq = rho_0;
+    for (int k = 0; k < 6; k++) {
+      const double a = rk45_a[k][j], ad = a * dp;
+      const bool on = a != 0.0;
+      const double q = ddiv_lat(on ? (j < 5 ? ad : a) : 1.0, c2);
+      const double S1 = S + q;
+      if (on) S = S1;
+      if (k == 5) break;
+      const double rk = bc(S, k);
+      c2 = c2_coop(M, rk, bc(pk, k));
+      if (i_le0(rk) || i_lt0(c2)) return false;
+      if (rk45_stage[j9] == k + 1) { cq = c2; rq = rk; }
+    }
+    const double D = S * dp;
+    const double w = ddiv_lat(ddiv_lat(rk45_u[j9], dsqrt(cq)), rq);
+    const int b = l == 0 ? 0 : 4;
+    double T = bc(w, b) + bc(w, b + 1) + bc(w, b + 2) + bc(w, b + 3);
+    const double T1 = T + bc(w, 8);
+    if (l) T = T1;
+    const double U = T * dp;
+    const double drho = bc(D, 5), drho_err = bc(D, 6), du = bc(U, 0), du_err = bc(U, 1);
+    if (is_nan_bits(du) || is_nan_bits(du_err)) return false;
+    rhoErr = fabs(drho_err - drho);
+    uErr = fabs(du_err - du);
+    rho = rho_0 + drho;
+    p = p_0 + dp;
+    u = (wave == 1) ? u_0 - du : u_0 + du;
+    const double ce = c2_coop(M, rho, p);
+    if (i_le0(rho) || i_lt0(ce)) return false;
+    const double c = dsqrt(ce);
+    memo_end = EosMemo{&M, rho, p, ce, c};
+    xi = (wave == 1) ? u - c : u + c;
+    return true;
+  }
+
+  // rk4 by a warp: the quotients by c_k^2 in two lanes, then 1 / c_k / rho_k of
+  // the four stages in four, the two weighted sums in two.
+  __device__ __noinline__ bool rk4_coop(int wave, const DevMat& M, double rho_0, double u_0, double p_0, double dp,
+                                        double& rho, double& u, double& p, double& xi) const {
+    const int l = lane();
+    dp = -dp;
+    const double hdp = 0.5 * dp;
+    double c2, c0;
+    if (!memo_get(M, rho_0, p_0, c2, c0)) {
+      c2 = c2_coop(M, rho_0, p_0);
+      if (i_le0(rho_0) || i_lt0(c2)) return false;
+      memo_start = EosMemo{&M, rho_0, p_0, c2, dsqrt(c2)};
+    }
+    const double pm = p_0 + hdp, pe = p_0 + dp;
+    double cq = c2, rq = rho_0, rr = 0.0;
+    for (int k = 0; k < 4; k++) {
+      const double q = ddiv_lat((l == 0 && k < 3) ? (k < 2 ? hdp : dp) : 1.0, c2);
+      const double r1 = bc(q, 1);
+      if (l == k) rr = r1;
+      if (k == 3) break;
+      const double rk = rho_0 + bc(q, 0);
+      c2 = c2_coop(M, rk, k < 2 ? pm : pe);
+      if (i_le0(rk) || i_lt0(c2)) return false;
+      if (l == k + 1) { cq = c2; rq = rk; }
+    }
+    const double w = ddiv_lat(ddiv_lat(1.0, dsqrt(cq)), rq);
+    // every lane takes part in every shuffle; lane 0 sums the density's terms, lane 1 the velocity's
+    const double r0 = bc(rr, 0), r1 = bc(rr, 1), r2 = bc(rr, 2), r3 = bc(rr, 3);
+    const double w0 = bc(w, 0), w1 = bc(w, 1), w2 = bc(w, 2), w3 = bc(w, 3);
+    const double v0 = l == 0 ? r0 : w0, v1 = l == 0 ? r1 : w1, v2 = l == 0 ? r2 : w2, v3 = l == 0 ? r3 : w3;
+    const double D = 1.0 / 6.0 * dp * (v0 + 2.0 * (v1 + v2) + v3);
+    const double drho = bc(D, 0), du = bc(D, 1);
+    if (is_nan_bits(du)) return false;
+    rho = rho_0 + drho;
+    p = p_0 + dp;
+    u = (wave == 1) ? u_0 - du : u_0 + du;
+    const double ce = c2_coop(M, rho, p);
+    if (i_le0(rho) || i_lt0(ce)) return false;
+    const double c = dsqrt(ce);
+    memo_end = EosMemo{&M, rho, p, ce, c};
+    xi = (wave == 1) ? u - c : u + c;
+    return true;
+  }
+
   // Cash-Karp step, ExactRiemannSolverBase.cpp:1771-1896.  The same
   // operations in the same order; a divisor that serves several quotients
   // (c_k^2, c_k, rho_k) takes its correctly rounded reciprocal once and each
   // quotient comes out of qdiv bit-identical to the division.
   __device__ __noinline__ bool rk45(int wave, const DevMat& M, double rho_0, double u_0, double p_0, double dp,
                      double& rho, double& u, double& p, double& xi, double& uErr, double& rhoErr) const {
+    if constexpr (Coop) return rk45_coop(wave, M, rho_0, u_0, p_0, dp, rho, u, p, xi, uErr, rhoErr);
     dp = -dp;
     const Quot R0 = qof(rho_0);
     double c_0_square, c_0;
@@ -252,6 +398,7 @@ struct ExactRiemannDev {
   // (shared reciprocals as in rk45)
   __device__ __noinline__ bool rk4(int wave, const DevMat& M, double rho_0, double u_0, double p_0, double dp,
                                    double& rho, double& u, double& p, double& xi) const {
+    if constexpr (Coop) return rk4_coop(wave, M, rho_0, u_0, p_0, dp, rho, u, p, xi);
     dp = -dp;
     const Quot R0 = qof(rho_0);
     double c_0_square, c_0;
@@ -363,7 +510,12 @@ struct ExactRiemannDev {
   __device__ __noinline__ static double hugo(const DevMat& M, double e, double pavg, double one_over_rho, double ps,
                                              double rhos) {
     double es, oors;
-    if (M.type == M2CG_EOS_SG) ddiv2(ps + M.gamPs, M.gam1 * rhos, 1.0, rhos, es, oors);
+    if (Coop && M.type == M2CG_EOS_SG) {
+      const bool o = lane() & 1;
+      const double q = ddiv_lat(o ? 1.0 : ps + M.gamPs, o ? rhos : M.gam1 * rhos);
+      es = bc(q, 0);
+      oors = bc(q, 1);
+    } else if (M.type == M2CG_EOS_SG) ddiv2(ps + M.gamPs, M.gam1 * rhos, 1.0, rhos, es, oors);
     else if (M.type == M2CG_EOS_NASG) {   // 1 / rho serves both terms
       oors = ddiv(1.0, rhos);
       es = M.invgam1 * (ps + M.gamPs) * (oors - M.b) + M.q;
@@ -414,8 +566,15 @@ struct ExactRiemannDev {
         bool ok = rk45(wave, M, rhos_0, us_0, ps_0, dp, rhos_1, us_1, ps_1, xi_1, uErr, rhoErr);
         if (!ok) { dp = dp / 2.0; continue; }
         if (i_lt(ps_1 - ps, -tol_end)) { dp = ps_0 - ps; continue; }
-        double uS = ddiv(uErr, c) + 1.e-30;
-        double rS = ddiv(rhoErr, rho) + 1.e-30;
+        double uS, rS;
+        if constexpr (Coop) {
+          const double q = ddiv_lat(lane() ? uErr : rhoErr, lane() ? c : rho) + 1.e-30;
+          rS = bc(q, 0);
+          uS = bc(q, 1);
+        } else {
+          uS = ddiv(uErr, c) + 1.e-30;
+          rS = ddiv(rhoErr, rho) + 1.e-30;
+        }
         if (is_nan_bits(rS) || is_nan_bits(uS)) return false;
         if (i_le(errBar, rS) && i_lt(dp_min, dp)) {
           double t = 0.9 * dp * pow(fabs(ddiv(errBar, rS)), 0.25);
@@ -444,8 +603,15 @@ struct ExactRiemannDev {
         // never reads it (the common case of a solve that restarts from the
         // path cache: one step to the end point)
         if (!i_le(fabs(ps_1 - ps), tol_end) && i + 1 < P.numSteps * 3) {
-          double tr = 0.9 * dp * pow(fabs(ddiv(errBar, rS)), 0.2);
-          double tu = 0.9 * dp * pow(fabs(ddiv(errBar, uS)), 0.2);
+          double tr, tu;
+          if constexpr (Coop) {
+            const double q = 0.9 * dp * pow(fabs(ddiv(errBar, lane() ? uS : rS)), 0.2);
+            tr = bc(q, 0);
+            tu = bc(q, 1);
+          } else {
+            tr = 0.9 * dp * pow(fabs(ddiv(errBar, rS)), 0.2);
+            tu = 0.9 * dp * pow(fabs(ddiv(errBar, uS)), 0.2);
+          }
           double t = i_min(tr, tu);
           t = i_min(t, 10 * dp);
           t = i_max(t, dp_min);
@@ -519,7 +685,7 @@ struct ExactRiemannDev {
         drho = rhos1 - rhos0;
         int it;
         for (it = 0; it < P.maxIts_shock; it++) {
-          rhos2 = rhos2 - ddiv(f2 * drho, f1 - f0);
+          rhos2 = rhos2 - (Coop ? ddiv_lat(f2 * drho, f1 - f0) : ddiv(f2 * drho, f1 - f0));
           if (i_le(rhos1, rhos2) || i_le(rhos2, rhos0)) rhos2 = rhos0 + 0.5 * drho;
           f2 = hugo(M, e, pavg, oor, ps, rhos2);
           if (i_eq0(f2)) { s_first = s_second = rhos2; break; }
@@ -855,8 +1021,15 @@ struct ExactRiemannDev {
       f2 = ul2 - ur2;
       if (i_prod_lt0(f0, f2)) { p1 = p2; f1 = f2; rhol1 = rhol2; rhor1 = rhor2; }
       else { p0 = p2; f0 = f2; rhol0 = rhol2; rhor0 = rhor2; }
-      double err_p = qd(fabs(p1 - p0), Qp);
-      double err_u = qd(fabs(f2), Qc);
+      double err_p, err_u;
+      if constexpr (Coop) {
+        const double q = ddiv_lat(lane() ? fabs(f2) : fabs(p1 - p0), lane() ? Qc.b : Qp.b);
+        err_p = bc(q, 0);
+        err_u = bc(q, 1);
+      } else {
+        err_p = qd(fabs(p1 - p0), Qp);
+        err_u = qd(fabs(f2), Qc);
+      }
       if ((i_lt(err_p, P.tol_main) && i_lt(err_u, P.tol_main)) || i_lt(err_p, tol_either) || i_lt(err_u, tol_either)) break;
       trans_rare = false;
     }
@@ -865,5 +1038,7 @@ struct ExactRiemannDev {
     return (iter == P.maxIts_main) ? 1 : 0;
   }
 };
+using ExactRiemannDev = ExactRiemannDevT<false>;
+using ExactRiemannCoop = ExactRiemannDevT<true>;
 
 }  // namespace m2cg
