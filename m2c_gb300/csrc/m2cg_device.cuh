@@ -88,26 +88,43 @@ M2CG_DEV bool i_prod_lt0(double a, double b) {
   return (bits(a) ^ bits(b)) < 0;
 }
 
-// Reciprocal and reciprocal square root: the hardware approximations of the
-// PTX ISA (rcp.approx.ftz.f64, rsqrt.approx.ftz.f64; about 2^-20 relative
-// error) refined by one third-order Householder step,
-//   r' = r (1 + e + e^2),            e = 1 - x r
-//   y' = y (1 + e/2 + 3 e^2 / 8),    e = 1 - x y^2,
-// which leaves at most about one ulp of error (checked on the device against
-// correctly rounded 1/x over 1e-20..1e20: max 2.2e-16).  Call sites pass
-// finite, positive, normal arguments.
-M2CG_DEV double rcp_fast(double x) {
+M2CG_DEV bool i_ge0(double x) {   // x >= 0
+  const unsigned long long u = (unsigned long long)bits(x);
+  return u <= 0x7ff0000000000000ull || u == 0x8000000000000000ull;
+}
+M2CG_DEV bool i_gt0(double x) { return (unsigned long long)bits(x) - 1ull <= 0x7fefffffffffffffull; }
+
+// Reciprocal and reciprocal square root to 0.51 ulp on the integer pipe
+// (m2cg_intfp.cuh: 68 and 99 cycles per warp against 204 and 369 for the
+// refined FP64 estimates, and none of them on the FP64 pipe that bounds the
+// stage kernels).  Operands outside the normal range -- zero, subnormal,
+// infinite, NaN, a negative argument of the root -- take the FP64 form: the
+// hardware estimate of the PTX ISA refined by one third-order Householder step.
+static __device__ __noinline__ double rcp_fp64(double x) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
   double e = fma(-x, r, 1.0);
   return fma(r, fma(e, e, e), r);
 }
-M2CG_DEV double rsqrt_fast(double x) {
+static __device__ __noinline__ double rsqrt_fp64(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   double e = fma(-x, y * y, 1.0);
   return fma(y * e, fma(e, 0.375, 0.5), y);
 }
+M2CG_DEV double rcp_fast(double x) {
+  if (!if_rcp_range(if_hi(x))) return rcp_fp64(x);
+  return if_rcp_core(if_hi(x), if_lo(x));
+}
+M2CG_DEV double rsqrt_fast(double x) {
+  if (!if_rsqrt_range(if_hi(x))) return rsqrt_fp64(x);
+  return if_rsqrt_core(if_hi(x), if_lo(x));
+}
+
+// The same as calls, for kernels whose straight-line code would not fit the
+// instruction cache with dozens of copies.
+static __device__ __noinline__ double rcp_call(double x) { return rcp_fast(x); }
+static __device__ __noinline__ double rsqrt_call(double x) { return rsqrt_fast(x); }
 
 // Quotients of several numerators over one divisor: the divisor's fixed-point
 // reciprocal (m2cg_intfp.cuh) is formed once, each quotient takes the
@@ -208,7 +225,7 @@ M2CG_DEV bool eos_bad5_fast(const DevMat& M, const double* V) {
   if (!is_finite_bits(V[0]) || !is_finite_bits(V[1]) || !is_finite_bits(V[2]) || !is_finite_bits(V[3]) ||
       !is_finite_bits(V[4]))
     return true;
-  if (M.type == M2CG_EOS_SG || M.type == M2CG_EOS_NASG) return le_zero_bits(V[0]) || le_zero_bits(V[4] + M.Pstiff);
+  if (M.type == M2CG_EOS_SG || M.type == M2CG_EOS_NASG) return le_zero_bits(V[0]) || i_le(V[4], -M.Pstiff);   // p + Pstiff <= 0 without the addition
   return eos_bad(M, V[0], V[4]);
 }
 M2CG_DEV bool eos_clip_fast(const DevMat& M, double* V) {
@@ -343,13 +360,13 @@ M2CG_DEV bool flux_hllc(const DevMat& M, int dir, const double* Vm, const double
   return ok;
 }
 
-// ---- HLLC with shared reciprocals ------------------------------------------
-// The same flux as flux_hllc (FluxFcnHLLC.h:57-245) with every division of the
-// reference rewritten as a product with a reciprocal that is computed once:
-// 1/rho and sqrt(rho) come from one rsqrt per side, the Roe-average weight
-// 1/(sqrt(rho_m)+sqrt(rho_p)) is shared by all five averages, and the star-state
-// algebra uses three more reciprocals.  Results agree with the reference order
-// to a few ulps.
+// ---- HLLC for the FP64 pipe ---------------------------------------------------
+// The same flux as flux_hllc (FluxFcnHLLC.h:57-245) in the fewest FP64
+// instructions (57 for a stiffened gas; the FP64 pipe bounds the stage
+// kernels): reciprocals and roots on the integer pipe, 1/rho and sqrt(rho) from
+// one reciprocal root per side, the Roe weight shared by all averages,
+// comparisons and selections on the integer pipe.  Results agree with the
+// reference's order to a few ulps.
 struct Side {
   double rho, vn, p, inv_rho, sr, e, dpdrho, Gamma, c2, c;
 };
@@ -357,125 +374,102 @@ M2CG_DEV void side_eos(const DevMat& M, const double* V, int dir, Side& S) {
   S.rho = V[0];
   S.vn = V[1 + dir];
   S.p = V[4];
-  double y = rsqrt_fast(S.rho);
+  double y = rsqrt_call(S.rho);
   S.sr = S.rho * y;
   S.inv_rho = y * y;
   if (M.type == M2CG_EOS_SG) {
     // c^2 = dp/drho + p/rho Gamma = gamma (p + p_inf) / rho (VarFcnSG.h:64-68,
     // VarFcnBase.h:219-223), the same value to rounding without the
-    // cancellation of the two terms near p = -p_inf
-    S.e = (S.p + M.gamPs) * M.invgam1 * S.inv_rho;
-    S.dpdrho = M.gam1 * S.e;
-    S.Gamma = M.gam1;
+    // cancellation of the two terms near p = -p_inf.  e follows where it is used.
+    S.e = 0.0;
     S.c2 = M.gam * (S.p + M.Pstiff) * S.inv_rho;
-    S.c = (S.c2 > 0.0) ? S.c2 * rsqrt_fast(S.c2) : 0.0;
+    S.c = i_gt0(S.c2) ? S.c2 * rsqrt_call(S.c2) : 0.0;
     return;
   } else if (M.type == M2CG_EOS_NASG) {
     double vb = S.inv_rho - M.b;
     S.e = M.invgam1 * (S.p + M.gamPs) * vb + M.q;
-    double r = S.inv_rho * rcp_fast(vb);
+    double r = S.inv_rho * rcp_call(vb);
     S.dpdrho = M.gam1 * (S.e - M.q) * r * r;
-    S.Gamma = M.gam1 * rcp_fast(1.0 - M.b * S.rho);
+    S.Gamma = M.gam1 * rcp_call(1.0 - M.b * S.rho);
   } else {
     S.e = eos_e(M, S.rho, S.p);
     S.dpdrho = eos_dpdrho(M, S.rho, S.e);
     S.Gamma = eos_Gamma(M, S.rho);
   }
   S.c2 = S.dpdrho + S.p * S.inv_rho * S.Gamma;
-  S.c = (S.c2 > 0.0) ? S.c2 * rsqrt_fast(S.c2) : 0.0;
-}
-M2CG_DEV void phys_flux_side(int dir, const double* V, const Side& S, double* F) {
-  double k2 = V[1] * V[1] + V[2] * V[2] + V[3] * V[3];
-  double H = S.e + 0.5 * k2 + S.p * S.inv_rho;
-  double m = S.rho * S.vn;
-  F[0] = m;
-  F[1] = m * V[1]; F[2] = m * V[2]; F[3] = m * V[3];
-  F[1 + dir] = fma(m, S.vn, S.p);
-  F[4] = m * H;
-}
-M2CG_DEV void hllc_fstar_side(int dir, const double* V, const Side& S, double Sw, double Sstar, double* F) {
-  double t = Sw - S.vn;
-  double rhostar = S.rho * t * rcp_fast(Sw - Sstar);
-  double k2 = V[1] * V[1] + V[2] * V[2] + V[3] * V[3];
-  double Eo = S.e + 0.5 * k2;   // U[4] / rho
-  double U[5] = {S.rho, S.rho * V[1], S.rho * V[2], S.rho * V[3], S.rho * Eo};
-  double Us[5] = {1.0, V[1], V[2], V[3], Eo + (Sstar - S.vn) * (Sstar + S.p * S.inv_rho * rcp_fast(t))};
-  Us[1 + dir] = Sstar;
-  phys_flux_side(dir, V, S, F);
-#pragma unroll
-  for (int i = 0; i < 5; i++) F[i] = fma(Sw, fma(Us[i], rhostar, -U[i]), F[i]);
+  S.c = i_gt0(S.c2) ? S.c2 * rsqrt_call(S.c2) : 0.0;
 }
 M2CG_DEV bool flux_hllc_fast(const DevMat& M, int dir, const double* Vm, const double* Vp, double* F) {
   const double eps = 1e-10;
   Side A, B;
   side_eos(M, Vm, dir, A);
   side_eos(M, Vp, dir, B);
-  double inv_s = rcp_fast(A.sr + B.sr);
-  double rho_hat = A.sr * B.sr;
-  double irr = A.inv_rho * B.inv_rho;          // 1 / rho_hat^2
-  double drho = B.rho - A.rho;
-  double dp = B.p - A.p;
-  double diff = (B.vn - A.vn) * inv_s;
-  double p_over_rho_hat = (A.sr * (A.p * A.inv_rho) + B.sr * (B.p * B.inv_rho)) * inv_s + 0.5 * diff * diff;
-  double e_hat = (A.sr * A.e + B.sr * B.e) * inv_s;
+  const double inv_s = rcp_call(A.sr + B.sr);
+  const double dp = B.p - A.p;
+  const double diff = (B.vn - A.vn) * inv_s;
   double c2_hat;
   if (M.type == M2CG_EOS_SG) {
     // Stiffened gas: p is linear in rho e with the constant Gamma = gamma - 1,
     // and the Roe-averaged jumps satisfy d(rho e) = rho_hat de + e_hat drho
     // exactly, so the generalized averages of FluxFcnHLLC.h:99-119 reduce to
-    // Gamma_hat = gamma - 1 and dp/drho_hat = (gamma - 1) e_hat: the same value
-    // without the weights w_rho, w_e and two reciprocals (the reference's form
-    // carries its rounding through a cancellation when dp ~ Gamma rho_hat de).
-    c2_hat = M.gam1 * (e_hat + p_over_rho_hat);
+    // Gamma_hat = gamma - 1 and dp/drho_hat = (gamma - 1) e_hat; with
+    // (gamma - 1)(e + p / rho) = c^2, c_hat^2 is the average of the two c^2 plus
+    // (gamma - 1) diff^2 / 2 (the reference's form carries its rounding through
+    // a cancellation when dp ~ Gamma rho_hat de).
+    c2_hat = fma(0.5 * M.gam1 * diff, diff, (A.sr * A.c2 + B.sr * B.c2) * inv_s);
   } else {
+    const double p_over_rho_hat = (A.sr * (A.p * A.inv_rho) + B.sr * (B.p * B.inv_rho)) * inv_s + 0.5 * diff * diff;
+    const double e_hat = (A.sr * A.e + B.sr * B.e) * inv_s;
+    const double rho_hat = A.sr * B.sr;
+    const double irr = A.inv_rho * B.inv_rho;          // 1 / rho_hat^2
+    const double drho = B.rho - A.rho;
     double de = B.e - A.e;
-    double inv_e = rcp_fast(e_hat);
+    double inv_e = rcp_call(e_hat);
     double w_rho = drho * drho * irr;
     double de_e = de * inv_e;
     double w_e = de_e * de_e;
-    double inv_den = rcp_fast(w_rho + w_e + eps);
+    double inv_den = rcp_call(w_rho + w_e + eps);
     double dpdrho_avg = (A.sr * A.dpdrho + B.sr * B.dpdrho) * inv_s;
     double Gamma_avg = (A.sr * A.Gamma + B.sr * B.Gamma) * inv_s;
     double dpdrho_hat = ((w_e + eps) * dpdrho_avg + (dp - Gamma_avg * rho_hat * de) * drho * irr) * inv_den;
     double Gamma_hat = ((w_rho + eps) * Gamma_avg + (dp - dpdrho_avg * drho) * de_e * inv_e * (A.inv_rho * B.sr * B.inv_rho * A.sr)) * inv_den;
     c2_hat = dpdrho_hat + Gamma_hat * p_over_rho_hat;
   }
-  double c_hat = (c2_hat <= 0.0) ? eps : c2_hat * rsqrt_fast(c2_hat);
-  double vh = (A.sr * A.vn + B.sr * B.vn) * inv_s;
-  double Sm = fmin(A.vn - A.c, vh - c_hat);
-  double Sp = fmax(B.vn + B.c, vh + c_hat);
-  bool ok = !(A.c2 < 0.0) && !(B.c2 < 0.0);
-  // FluxFcnHLLC.h:226-241: F_L, F_R, F*_L or F*_R.  The side is selected
-  // first and its flux evaluated once, so lanes of a warp whose faces pick
-  // different sides do not run both branches (the same operations as
-  // phys_flux_side / hllc_fstar_side on the chosen side).
-  const bool sup_l = 0.0 <= Sm, sup_r = 0.0 >= Sp;
+  const double c_hat = i_le0(c2_hat) ? eps : c2_hat * rsqrt_call(c2_hat);
+  const double vh = (A.sr * A.vn + B.sr * B.vn) * inv_s;
+  const double Sm = i_min(A.vn - A.c, vh - c_hat);
+  const double Sp = i_max(B.vn + B.c, vh + c_hat);
+  const bool ok = !i_lt0(A.c2) && !i_lt0(B.c2);
+  // FluxFcnHLLC.h:226-241: F_L, F_R, F*_L or F*_R.  The side K and its state --
+  // (rho, vn, p) or the star state (rho*, S*, p*) -- are selected first and the
+  // flux evaluated once, so lanes of a warp whose faces differ do not run
+  // several branches.  F* = F + S (U* - U) is the physical flux of the star
+  // state with energy E* (the jump conditions across S): no cancellation
+  // between S U* and S U.
+  const bool sup_l = i_ge0(Sm), sup_r = i_le0(Sp);
   const double am = A.rho * (Sm - A.vn), bp = B.rho * (Sp - B.vn);
-  const double Sstar = (dp + am * A.vn - bp * B.vn) * rcp_fast(am - bp);
-  const bool left = sup_l || (!sup_r && Sstar >= 0.0);
+  const double Sstar = (dp + am * A.vn - bp * B.vn) * rcp_call(am - bp);
+  const bool left = sup_l || (!sup_r && i_ge0(Sstar)), sup = sup_l || sup_r;
   // value selects (no pointer to either side, which would put them in memory)
-  Side K;
-  K.rho = left ? A.rho : B.rho;
-  K.vn = left ? A.vn : B.vn;
-  K.p = left ? A.p : B.p;
-  K.inv_rho = left ? A.inv_rho : B.inv_rho;
-  K.e = left ? A.e : B.e;
   double V[5];
 #pragma unroll
   for (int i = 0; i < 5; i++) V[i] = left ? Vm[i] : Vp[i];
-  phys_flux_side(dir, V, K, F);
-  if (!sup_l && !sup_r) {
-    const double Sw = left ? Sm : Sp;
-    double t = Sw - K.vn;
-    double rhostar = K.rho * t * rcp_fast(Sw - Sstar);
-    double k2 = V[1] * V[1] + V[2] * V[2] + V[3] * V[3];
-    double Eo = K.e + 0.5 * k2;   // U[4] / rho
-    double U[5] = {K.rho, K.rho * V[1], K.rho * V[2], K.rho * V[3], K.rho * Eo};
-    double Us[5] = {1.0, V[1], V[2], V[3], Eo + (Sstar - K.vn) * (Sstar + K.p * K.inv_rho * rcp_fast(t))};
-    Us[1 + dir] = Sstar;
-#pragma unroll
-    for (int i = 0; i < 5; i++) F[i] = fma(Sw, fma(Us[i], rhostar, -U[i]), F[i]);
-  }
+  const double inv_rho = left ? A.inv_rho : B.inv_rho;
+  const double vn = V[1 + dir], p = V[4];
+  const double e = M.type == M2CG_EOS_SG ? (p + M.gamPs) * M.invgam1 * inv_rho : (left ? A.e : B.e);
+  const double a = left ? am : bp;                    // rho (S - vn)
+  const double Sw = left ? Sm : Sp;
+  const double rs = a * rcp_call(Sw - Sstar);
+  const double w = sup ? vn : Sstar, rw = sup ? V[0] : rs;
+  const double dv = w - vn;
+  const double ps = fma(a, dv, p), de = dv * fma(p, rcp_call(a), w);
+  const double pw = sup ? p : ps;
+  const double E = fma(0.5, V[1] * V[1] + V[2] * V[2] + V[3] * V[3], e) + (sup ? 0.0 : de);
+  const double m = rw * w;
+  F[0] = m;
+  F[1] = m * V[1]; F[2] = m * V[2]; F[3] = m * V[3];
+  F[1 + dir] = fma(m, w, pw);
+  F[4] = fma(m, E, pw * w);
   return ok;
 }
 
@@ -560,26 +554,20 @@ M2CG_DEV double gen_minmod(double alpha, double dq0, double dq1) {
   if (dq0 > 0.0 && dq1 > 0.0) return fmin(alpha * dq0, fmin(0.5 * (dq0 + dq1), alpha * dq1));
   return 0.0;
 }
-// van Albada with the sign / magnitude tests on the integer pipe and one
-// reciprocal (same value as van_albada to an ulp).  a = dq0^2 and b = dq1^2
-// come in precomputed (a difference shared by two neighbouring cells is squared
-// once); every operation is pinned (no contraction), so the split and fused
-// stage kernels produce the same bits.
-M2CG_DEV double van_albada_sq(double dq0, double dq1, double a, double b) {
+// van Albada on the integer pipe (if_van_albada: 182 cycles per warp with one
+// FP64 multiplication, against 666 for the FP64 form with its ten); products
+// next to the 1e-16 threshold and special operands take the FP64 form.  Every
+// operation is pinned (no contraction), so the split and fused stage kernels
+// produce the same bits.
+static __device__ __noinline__ double van_albada_fp64(double dq0, double dq1) {
   double pr = __dmul_rn(dq0, dq1);
   if (le_zero_bits(pr) || abs_lt_bits(pr, 1e-16)) return 0.0;
+  const double a = __dmul_rn(dq0, dq0), b = __dmul_rn(dq1, dq1);
   return __dmul_rn(fma(dq1, a, __dmul_rn(dq0, b)), rcp_fast(__dadd_rn(a, b)));
 }
-M2CG_DEV double van_albada_fast(double dq0, double dq1) {
-  return van_albada_sq(dq0, dq1, __dmul_rn(dq0, dq0), __dmul_rn(dq1, dq1));
+static __device__ __noinline__ double van_albada_fast(double dq0, double dq1) {
+  double s;
+  if (!if_van_albada(dq0, dq1, s)) s = van_albada_fp64(dq0, dq1);
+  return s;
 }
-// k = 2 on a uniform mesh (Reconstructor.cpp:103-121 with A = B = 1)
-M2CG_DEV double van_albada(double dq0, double dq1) {
-  double pr = dq0 * dq1;
-  if (pr <= 0.0) return 0.0;
-  if (fabs(pr) < 1e-16) return 0.0;
-  double a = dq0 * dq0, b = dq1 * dq1;
-  return (dq1 * a + dq0 * b) / (a + b);
-}
-
 }  // namespace m2cg

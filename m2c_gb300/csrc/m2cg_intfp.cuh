@@ -209,19 +209,23 @@ M2CG_INT_SLOW double dsqrt(double x) {
 // (b a^2 + a b^2) / (a^2 + b^2) for two differences of the same sign, with a
 // the smaller: a h, h = b (a + b) / (a^2 + b^2) in [1, 1.21], h in fixed point
 // from the significands (a's shifted to b's exponent: h depends on a / b to
-// 2^-60) and one binary64 multiplication.
-M2CG_INT bool if_van_albada(double x, double y, double& out) {
+// 2^-60) and one binary64 multiplication; 0 for opposite signs and for a
+// product below 1e-16.  Returns 1 with the slope, or 0 where the product is
+// next to 1e-16 or an operand is special (the caller's FP64 form decides).
+M2CG_INT int if_van_albada(double x, double y, double& out) {
   const uint32_t xh = if_hi(x), yh = if_hi(y);
   const uint32_t ux = xh & 0x7fffffffu, uy = yh & 0x7fffffffu;
   const bool xs = ux < uy || (ux == uy && if_lo(x) < if_lo(y));   // |x| < |y|
-  const double a = xs ? x : y;
-  const uint32_t ah = xs ? xh : yh, al = if_lo(a);
+  const uint32_t ah = xs ? xh : yh, al = xs ? if_lo(x) : if_lo(y);
   const uint32_t bh = xs ? yh : xh, bl = xs ? if_lo(y) : if_lo(x);
   const uint32_t ea = (ah >> 20) & 0x7ffu, eb = (bh >> 20) & 0x7ffu;
-  // decided or out of range: product's exponent near 1e-16 or below, or a
-  // special operand
-  if (ea + eb < 1994u || eb > 2000u || ea == 0u) return false;
-  if ((int32_t)(ah ^ bh) < 0) { out = 0.0; return true; }
+  out = 0.0;
+  if (eb > 2000u) return 0;
+  // the product lies in [2^(ea + eb - 2046), 4 x that); 1e-16 = 2^-53.15
+  if (ea + eb <= 1990u) return 1;
+  if (ea + eb < 1994u) return 0;
+  if ((int32_t)(ah ^ bh) < 0) return 1;
+  if (ea == 0u) return 0;
   const uint32_t sh = eb - ea;
   const uint64_t B = if_sig(bh, bl), A = if_sig(ah, al) >> (sh < 63u ? sh : 63u);
   const uint64_t b2 = if_sqrhi64(B) >> 2;                    // b^2 2^60
@@ -229,8 +233,8 @@ M2CG_INT bool if_van_albada(double x, double y, double& out) {
   const uint64_t num = b2 + (if_mulhi64(A, B) >> 2);
   const int z = if_clz((uint32_t)(den >> 32));               // 0 < z < 4
   const uint64_t h = if_mulhi64(num << (z - 1), if_recip(den << z));   // h 2^61
-  out = if_mul(a, if_pack(1022u << 20, (h + 256u) >> 9));
-  return true;
+  out = if_mul(if_dbl(ah, al), if_pack(1022u << 20, (h + 256u) >> 9));
+  return 1;
 }
 
 }  // namespace m2cg

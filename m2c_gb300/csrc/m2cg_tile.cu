@@ -71,10 +71,10 @@ __device__ __forceinline__ void tma_box(void* dst, const CUtensorMap* map, uint6
 }
 
 // ---- one face state ---------------------------------------------------------
-// Limited slope of one variable from its two one-sided differences (and their
-// squares, for van Albada), as in k_reconstruct.
-__device__ __forceinline__ double slope(const Params& P, double dq0, double dq1, double a, double b) {
-  if (P.limiter == M2CG_LIM_VANALBADA) return van_albada_sq(dq0, dq1, a, b);
+// Limited slope of one variable from its two one-sided differences, as in
+// k_reconstruct.
+__device__ __forceinline__ double slope(const Params& P, double dq0, double dq1) {
+  if (P.limiter == M2CG_LIM_VANALBADA) return van_albada_fast(dq0, dq1);
   if (P.limiter == M2CG_LIM_GENERALIZED_MINMOD) return gen_minmod(P.minmod_coeff, dq0, dq1);
   return 0.5 * (dq0 + dq1);
 }
@@ -111,7 +111,7 @@ struct GlobalCells {
 // Face f (vl, vr, vb, vt, vk, vf) of cell c before any check
 // (Reconstructor.cpp:426-716), with the arithmetic of k_reconstruct.
 template <class A>
-M2CG_DEV void raw_face(const Params& P, const A& a, typename A::C c, int f, int myid, double* out) {
+__device__ __noinline__ void raw_face(const Params& P, const A& a, typename A::C c, int f, int myid, double* out) {
   double q[5];
 #pragma unroll
   for (int p = 0; p < 5; p++) q[p] = a.q(p, c);
@@ -128,7 +128,7 @@ M2CG_DEV void raw_face(const Params& P, const A& a, typename A::C c, int f, int 
   for (int p = 0; p < 5; p++) {
     double dq0 = q[p] - a.q(p, cm);
     double dq1 = a.q(p, cp) - q[p];
-    double s = slope(P, dq0, dq1, __dmul_rn(dq0, dq0), __dmul_rn(dq1, dq1));
+    double s = slope(P, dq0, dq1);
     if (zero) s = 0.0;
     out[p] = fma(h, s, q[p]);
   }
@@ -189,9 +189,11 @@ __device__ __forceinline__ void warp_count(unsigned long long* c, int v) {
 __device__ __forceinline__ void cell_faces_dir(const Params& P, const DevMat& M, const SmemCells& a, SmemCells::C c,
                                                int d, const double* q, int myid, double* vm, double* vp,
                                                bool& done, int& nclip, int& nbad) {
+  bool badm, badp;
   if (P.rec_type == M2CG_REC_CONSTANT) {
 #pragma unroll
     for (int p = 0; p < 5; p++) { vm[p] = q[p]; vp[p] = q[p]; }
+    badm = badp = eos_bad5_fast(M, q);
   } else {
     const SmemCells::C cm = a.nb(c, d, -1), cp = a.nb(c, d, 1);
     const bool zero = P.slope_zero && (a.idv(cm) != myid || a.idv(cp) != myid);
@@ -199,19 +201,23 @@ __device__ __forceinline__ void cell_faces_dir(const Params& P, const DevMat& M,
     for (int p = 0; p < 5; p++) {
       const double dq0 = q[p] - a.q(p, cm);
       const double dq1 = a.q(p, cp) - q[p];
-      double sl = slope(P, dq0, dq1, __dmul_rn(dq0, dq0), __dmul_rn(dq1, dq1));
+      double sl = slope(P, dq0, dq1);
       if (zero) sl = 0.0;
       vm[p] = fma(-0.5, sl, q[p]);
       vp[p] = fma(0.5, sl, q[p]);
     }
-    if (!done && eos_bad5_fast(M, vm)) {
+    badm = eos_bad5_fast(M, vm);
+    badp = eos_bad5_fast(M, vp);
+    if (!done && badm) {
 #pragma unroll
       for (int p = 0; p < 5; p++) vm[p] = q[p];
+      badm = eos_bad5_fast(M, vm);
       done = true;
     }
-    if (!done && eos_bad5_fast(M, vp)) {
+    if (!done && badp) {
 #pragma unroll
       for (int p = 0; p < 5; p++) vp[p] = q[p];
+      badp = eos_bad5_fast(M, vp);
       done = true;
     }
   }
@@ -219,17 +225,18 @@ __device__ __forceinline__ void cell_faces_dir(const Params& P, const DevMat& M,
   if (eos_clip_fast(M, t)) {
 #pragma unroll
     for (int p = 0; p < 5; p++) vm[p] = q[p];
+    badm = eos_bad5_fast(M, vm);
     nclip++;
   }
-  nbad += eos_bad5_fast(M, vm);
 #pragma unroll
   for (int p = 0; p < 5; p++) t[p] = vp[p];
   if (eos_clip_fast(M, t)) {
 #pragma unroll
     for (int p = 0; p < 5; p++) vp[p] = q[p];
+    badp = eos_bad5_fast(M, vp);
     nclip++;
   }
-  nbad += eos_bad5_fast(M, vp);
+  nbad += (int)badm + (int)badp;
 }
 
 // One checked face state of a cell outside the tile's own cells (a halo cell,
