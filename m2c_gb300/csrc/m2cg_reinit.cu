@@ -17,10 +17,10 @@
 // in plain binary64.  The residual is written for GB300's FP64 pipe, which
 // bounds this loop: the one-sided differences are multiplied by 1/h where the
 // reference divides by the difference of two cell-centre coordinates (equal to
-// h up to the rounding of those coordinates), signs flip and maxima are taken
-// on the integer pipe through the bit patterns, and the square root and the
-// relative change use a refined hardware reciprocal (square root) estimate.
-// The result differs from the reference's operation order by a few ulps.
+// h up to the rounding of those coordinates), neighbours are chosen, signs flip
+// and maxima are taken on the integer pipe through the bit patterns, and the
+// square root uses the integer-pipe reciprocal root.  The result differs from
+// the reference's operation order by a few ulps.
 #include <algorithm>
 #include "m2cg_internal.h"
 
@@ -41,50 +41,40 @@ M2CG_DEV unsigned long long as_bits(double x) { return (unsigned long long)__dou
 
 M2CG_DEV bool ri_live(const ReinitState* st) { return st->run && st->detected; }
 
-// max(x, y, 0) through the bit patterns: non-negative doubles order like their
-// signed 64-bit patterns and every negative one (-0 included) falls below the
-// pattern of +0, so the comparison runs on the integer pipe.
-M2CG_DEV double max_with_zero(double x, double y) {
-  long long a = __double_as_longlong(x), b = __double_as_longlong(y);
-  long long m = a > b ? a : b;
-  return __longlong_as_double(m > 0 ? m : 0);
-}
-
 // x with its sign bit xor-ed with sb (0 or the sign bit): an exact negation
 // when sb is set, on the integer pipe.
 M2CG_DEV double flip(double x, long long sb) { return __longlong_as_double(__double_as_longlong(x) ^ sb); }
 
-// sqrt(x) for x >= 0 as x * rsqrt(x), the reciprocal square root from the
-// hardware estimate refined by Newton's iteration (one step, cubic term).
-M2CG_DEV double sqrt_nr(double x) {
-  if (!(x > 1e-300)) return sqrt(x);   // zero, subnormal (the estimate flushes it), NaN
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y * y, 1.0);
-  y = fma(y * e, fma(e, 0.375, 0.5), y);
-  return x * y;
-}
-
-// 1/x for x > 0 from the hardware estimate refined by Newton's iteration.
-M2CG_DEV double rcp_nr(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = fma(-x, r, 1.0);
-  return fma(r, fma(e, e, e), r);
+// Godunov's one-sided difference along one axis: max(p - m, p - n, 0), for
+// phi < 0 (sb set) max(m - p, n - p, 0).  Rounding is monotone, so the larger
+// difference is that of the smaller (larger) neighbour, chosen on the integer
+// pipe: one subtraction instead of two, the same bits.  A NaN neighbour gives
+// NaN.
+M2CG_DEV double one_sided(double p, double m, double n, long long sb) {
+  // the neighbours with their signs flipped for phi < 0; the smaller of the two
+  const double x = flip(m, sb), y = flip(n, sb);
+  const bool xl = i_key(x) <= i_key(y) ? !is_nan_bits(y) : is_nan_bits(x);
+  const double d = flip(p, sb) - (xl ? x : y);
+  const long long db = __double_as_longlong(d);
+  return __longlong_as_double(db > 0 ? db : 0);   // negative differences (-0 included) fall below +0
 }
 
 // |grad phi| - 1 by Godunov's upwind rule (LevelSetReinitializer.cpp:1009-1026).
 // For phi >= 0 the x term is max(max(a,0)^2, min(b,0)^2) with a, b the backward
 // and forward differences; it equals (max(p - p_{i-1}, p - p_{i+1}, 0) / h)^2.
 // For phi < 0 the differences change sign (phi = -0 counts as >= 0, as there).
-M2CG_DEV double ri_res(const double* __restrict__ q, int64_t c, int64_t sy, int64_t sz, const double* rh) {
+// With one spacing h the three squares share one product by 1/h.
+M2CG_DEV double ri_res(const double* __restrict__ q, int64_t c, int64_t sy, int64_t sz, const double* rh, bool cube) {
   const double p = q[c];
   const long long pb = __double_as_longlong(p);
   const long long sb = (pb < 0 && pb != (long long)0x8000000000000000ull) ? (long long)0x8000000000000000ull : 0ll;
-  const double gx = max_with_zero(flip(p - q[c - 1], sb), flip(p - q[c + 1], sb)) * rh[0];
-  const double gy = max_with_zero(flip(p - q[c - sy], sb), flip(p - q[c + sy], sb)) * rh[1];
-  const double gz = max_with_zero(flip(p - q[c - sz], sb), flip(p - q[c + sz], sb)) * rh[2];
-  return sqrt_nr(fma(gz, gz, fma(gy, gy, gx * gx))) - 1.0;
+  double gx = one_sided(p, q[c - 1], q[c + 1], sb);
+  double gy = one_sided(p, q[c - sy], q[c + sy], sb);
+  double gz = one_sided(p, q[c - sz], q[c + sz], sb);
+  if (!cube) { gx *= rh[0]; gy *= rh[1]; gz *= rh[2]; }
+  const double g2 = fma(gz, gz, fma(gy, gy, gx * gx));
+  const double g = if_rsqrt_range(if_hi(g2)) ? g2 * if_rsqrt_core(if_hi(g2), if_lo(g2)) : sqrt(g2);
+  return cube ? fma(g, rh[0], -1.0) : g - 1.0;
 }
 
 // Block maximum of non-negative bit patterns, one atomic per block.
@@ -185,6 +175,13 @@ __global__ void __launch_bounds__(RI_THREADS) k_ri_prep(ReinitArgs a) {
 //   S = 3: phi  = (phi/3 + 2 phi2/3) + 2 R/3, and the largest relative change
 // S = 1 also records max |res| over the untagged nodes; later sub-stages stop
 // once that is below the tolerance (the reference's loop exit).
+//
+// Bound by the FP64 pipe: about 13 FP64 instructions per node and sub-stage
+// (three differences, three squares, the root's product, the product by 1/h
+// with the -1, two for R, the combination; 30 before the choices, the root and
+// the sign of R moved to the integer pipe): 0.44 ms per sub-stage at
+// 256 x 224 x 192 against 1.02.  A warp covers 32 consecutive interior nodes of
+// the x-fastest order (rows of any length leave no idle lanes).
 template <int S>
 __global__ void __launch_bounds__(RI_THREADS) k_ri_stage(ReinitArgs a) {
   ReinitState* st = a.st;
@@ -195,37 +192,64 @@ __global__ void __launch_bounds__(RI_THREADS) k_ri_stage(ReinitArgs a) {
   double* out = S == 1 ? a.phi1 : (S == 2 ? a.phi2 : a.phi);
   const double mdt = -(st->cfl * a.hmin);
   const Grid& g = a.g;
-  const int64_t rows = (int64_t)g.ny * g.nz;
-  unsigned long long mx = 0;
-  for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
-    const int k = (int)(r / g.ny), j = (int)(r - (int64_t)k * g.ny);
-    const int64_t base = g.at(0, j, k);
-    for (int i = threadIdx.x; i < g.nx; i += RI_THREADS) {
-      const int64_t c = base + i;
+  const bool cube = a.rh[0] == a.rh[1] && a.rh[0] == a.rh[2];
+  const int64_t n = (int64_t)g.nx * g.ny * g.nz;
+  unsigned long long mx = 0;   // the thread's largest value
+  int mxw = 0;                 // the warp's largest high word so far
+  for (int64_t t0 = (int64_t)blockIdx.x * RI_THREADS + (threadIdx.x & ~31); t0 < n; t0 += (int64_t)gridDim.x * RI_THREADS) {
+    const int64_t t = t0 + (threadIdx.x & 31);
+    const bool in = t < n;
+    int i, j, k;
+    if (n <= 0x7fffffffll) {   // 32-bit divisions where they reach
+      const unsigned u = (unsigned)(in ? t : n - 1), r = u / (unsigned)g.nx;
+      i = (int)(u - r * (unsigned)g.nx); k = (int)(r / (unsigned)g.ny); j = (int)(r - (unsigned)k * (unsigned)g.ny);
+    } else {
+      const int64_t r = (in ? t : n - 1) / g.nx;
+      i = (int)((in ? t : n - 1) - r * g.nx); k = (int)(r / g.ny); j = (int)(r - (int64_t)k * g.ny);
+    }
+    const int64_t c = g.at(i, j, k);
+    double e = 0.0, anw = 1.0;
+    if (in) {
       double R = 0.0;
       if (!a.tag[c]) {
-        const double res = ri_res(src, c, g.sy, g.sz, a.rh);
+        const double res = ri_res(src, c, g.sy, g.sz, a.rh, cube);
         const double f = mdt * a.sign[c];
-        const double ares = fabs(res);
-        R = ares <= 1.0 ? f * res : (f * res) / ares;
-        if (S == 1) { const unsigned long long b = as_bits(ares); mx = b > mx ? b : mx; }
+        // f max(-1, min(1, res)): beyond 1 only the sign of res remains
+        const long long rb = __double_as_longlong(res) & (long long)0x8000000000000000ull;
+        const unsigned long long ab = as_bits(res) & 0x7fffffffffffffffull;
+        if (ab <= 0x3ff0000000000000ull) R = f * res;
+        else if (ab < 0x7ff0000000000000ull) R = flip(f, rb);
+        else R = (f * res) / fabs(res);   // infinite or NaN
+        if (S == 1) mx = ab > mx ? ab : mx;
       }
       if (S == 1) {
         const double p = src[c];
         if (restore) a.phi[c] = p;
         out[c] = p + R;
       } else if (S == 2) {
-        out[c] = (0.25 * src[c] + 0.75 * a.phi[c]) + 0.25 * R;
+        // products by 1/4 are exact: the fused forms round as the separate ones
+        out[c] = fma(0.25, R, fma(0.25, src[c], 0.75 * a.phi[c]));
       } else {
         const double old = out[c];
         const double nw = ((1.0 / 3.0) * old + (2.0 / 3.0) * src[c]) + (2.0 / 3.0) * R;
         out[c] = nw;
-        double e = fabs(nw - old);
-        const double anw = fabs(nw);
-        if (anw > 1e-300) e *= rcp_nr(anw);
-        else if (nw != 0.0) e /= anw;
-        const unsigned long long b = as_bits(e);
+        e = fabs(nw - old);
+        anw = fabs(nw);
+      }
+    }
+    if (S == 3) {
+      // The largest e / |nw|: a quotient's high word is at most the difference
+      // of the operands' plus 1.0's (the binary logarithm is above its chord),
+      // so nodes that cannot raise the warp's maximum skip the division.
+      const int cand = __double2hiint(e) - __double2hiint(anw) + 0x3ff00001;
+      const bool odd = !(anw > 1e-300) || (__double2hiint(e) & 0x7ff00000) == 0x7ff00000;
+      if (__any_sync(0xffffffffu, e != 0.0 && (cand >= mxw || odd))) {
+        double q = e;
+        if (anw > 1e-300) q = e * rcp_fast(anw);
+        else if (anw != 0.0) q = e / anw;
+        const unsigned long long b = as_bits(q);
         mx = b > mx ? b : mx;
+        mxw = __reduce_max_sync(0xffffffffu, (int)(mx >> 32));
       }
     }
   }
@@ -501,7 +525,8 @@ cudaError_t reinit_build_graph(cudaStream_t s, const ReinitArgs& a, int nsm, int
   if (e != cudaSuccess) return e;
   cudaGraphConditionalHandle h;
   const int64_t rows = (int64_t)a.g.ny * a.g.nz;
-  const int sblocks = (int)std::min<int64_t>(rows, (int64_t)nsm * 16);
+  const int64_t nreal = rows * a.g.nx;
+  const int sblocks = (int)std::max<int64_t>(1, std::min<int64_t>((nreal + RI_THREADS - 1) / RI_THREADS, (int64_t)nsm * 16));
   const int64_t nghost = 2 * ((int64_t)a.g.ny * a.g.nz + (int64_t)a.g.nx * a.g.nz + (int64_t)a.g.nx * a.g.ny);
   const int gblocks = (int)std::max<int64_t>(1, std::min<int64_t>((nghost + 255) / 256, (int64_t)nsm * 4));
   cudaGraphNodeParams np = {};
