@@ -15,8 +15,10 @@
 #include "m2cg_ens.h"
 
 namespace m2cg {
-void launch_reconstruct(cudaStream_t, const Params&, const StateSet&, const int32_t*, double* const*, unsigned long long*);
-void launch_face_flux(cudaStream_t, const Params&, const int32_t*, double* const*, double* const*, unsigned long long*);
+void launch_reconstruct(cudaStream_t, const Params&, const StateSet&, const int32_t*, double* const*, unsigned long long*,
+                        const Gate&);
+void launch_face_flux(cudaStream_t, const Params&, const int32_t*, double* const*, double* const*, unsigned long long*,
+                      const Gate&);
 void launch_update(cudaStream_t, const Params&, const StageArgs&, const int32_t*, int32_t*, double* const*,
                    const IfaceList&, const DevScalars*, int64_t*, unsigned long long*, int64_t, unsigned long long*);
 void launch_ls_residual(cudaStream_t, const Params&, const StateSet&, double*);
@@ -43,7 +45,7 @@ void launch_riemann_interfaces(cudaStream_t, const Params&, const Mats*, const S
                                unsigned long long*, const float*, unsigned long long*, const DevScalars*);
 void launch_riemann_stragglers(cudaStream_t, const Params&, const Mats*, const StateSet&, const int32_t*,
                                double* const*, const IfaceList&, int, double*, int, int, size_t, const int32_t*,
-                               const unsigned long long*, const float*, unsigned long long*, const DevScalars*, int);
+                               const unsigned long long*, const float*, unsigned long long*, const DevScalars*, int, int*);
 cudaError_t riemann_stragglers_reserve(size_t bytes);
 void mlp_warm_faces(m2cg_mlp*, cudaStream_t, int, const Params&, const StateSet&, const int32_t*, const IfaceList&,
                     __nv_bfloat16*, float*, float*, float*, const DevScalars*);
@@ -129,15 +131,10 @@ struct m2cg_ctx {
   int eval_limit = 24;
   int sblocks = 0;             // straggler blocks of 128 threads (one SM each; idle ones exit at once)
   int strag_lanes = 1;         // straggler faces packed per warp (1: one face per warp)
-  // Fused reconstruction + face flux (m2cg_tile.cu) for each state set, when
-  // the configuration allows it; the split kernels otherwise (or with
-  // M2CG_STAGE_KERNELS=split, for comparisons).
-  bool tile_ok = false;
-  int tile_z = 16;             // planes per CTA of the fused kernel (M2CG_TILE_Z)
-  TileMaps tmaps[3];
   size_t sreserve = 0;         // their dynamic shared-memory request
   int32_t* strag = nullptr;
   unsigned long long* strag_count = nullptr;
+  int* stalled = nullptr;      // per stage: did the stage before it leave stalled solves (Gate)
   cudaEvent_t ev_a = nullptr;  // end of the first pass
   long long hold_cycles = 40000;  // ~20 us head start for the straggler blocks
   // learned warm start (m2cg_set_warm_start): per interface face features,
@@ -325,6 +322,7 @@ static m2cg_status ctx_alloc(m2cg_ctx* x) {
   else CK(x->alloc(&x->scratch, (size_t)6 * x->path_cap * x->rblocks * x->rthreads));
   CK(x->alloc(&x->strag, L.cap));
   CK(x->alloc(&x->strag_count, 1));
+  CK(x->alloc(&x->stalled, 3));
   x->sblocks = std::max(1, std::min(x->nsm, x->rblocks));
   // tuning overrides: M2CG_RIEMANN_EVAL_LIMIT (first-pass budget, 0 = none),
   // M2CG_RIEMANN_STRAGGLER_SMS (blocks of the second pass, one SM each),
@@ -334,14 +332,6 @@ static m2cg_status ctx_alloc(m2cg_ctx* x) {
   if (const char* e = getenv("M2CG_RIEMANN_STRAGGLER_SMS")) x->sblocks = std::min(x->rblocks, std::max(1, atoi(e)));
   if (const char* e = getenv("M2CG_RIEMANN_HOLD_CYCLES")) x->hold_cycles = std::max(0ll, atoll(e));
   if (const char* e = getenv("M2CG_RIEMANN_STRAGGLER_LANES")) x->strag_lanes = std::min(32, std::max(1, atoi(e)));
-  {
-    const char* e = getenv("M2CG_STAGE_KERNELS");
-    bool want = !(e && strcmp(e, "split") == 0);
-    if (const char* z = getenv("M2CG_TILE_Z")) x->tile_z = std::max(1, atoi(z));
-    x->tile_ok = want && tile_supported(x->P) && tile_prepare() == cudaSuccess;
-    for (int s = 0; s < 3 && x->tile_ok; s++) x->tile_ok = tile_maps(x->P, x->S[s], &x->tmaps[s]);
-    cudaGetLastError();
-  }
   {
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
@@ -406,19 +396,15 @@ static StageArgs stage_args(m2cg_ctx* x, int stage, bool last, const StateSet& i
   return A;
 }
 
-// Reconstruction and same-material face fluxes of a stage input: the fused
-// tile kernel where available, else the split kernels.  Returns launches.
-static int64_t enqueue_recon_flux(m2cg_ctx* x, cudaStream_t s, const StateSet& in) {
-  if (x->tile_ok) {
-    for (int k = 0; k < 3; k++)
-      if (in.q[0] == x->S[k].q[0]) {
-        PHASE(PH_FLUX, launch_recon_flux_tile(s, x->tmaps[k], x->P, in, x->id, x->d_F, x->cnt, x->tile_z));
-        return 2;
-      }
-  }
-  PHASE(PH_RECON, launch_reconstruct(s, x->P, in, x->id, x->d_fs, x->cnt));
-  PHASE(PH_FLUX, launch_face_flux(s, x->P, x->id, x->d_fs, x->d_F, x->cnt));
-  return 3;
+// Reconstruction (unless done) and same-material face fluxes of a stage input.  Returns launches.
+static int64_t enqueue_recon_flux(m2cg_ctx* x, cudaStream_t s, const StateSet& in, bool recon, const Gate& gt) {
+  if (recon) PHASE(PH_RECON, launch_reconstruct(s, x->P, in, x->id, x->d_fs, x->cnt, gt));
+  PHASE(PH_FLUX, launch_face_flux(s, x->P, x->id, x->d_fs, x->d_F, x->cnt, gt));
+  return recon ? 3 : 1;
+}
+// Runge-Kutta stages of the configured scheme.
+static int rk_stages(const m2cg_ctx* x) {
+  return x->cfg.ts_type == M2CG_TS_FORWARD_EULER ? 1 : x->cfg.ts_type == M2CG_TS_RK2 ? 2 : 3;
 }
 
 // Enqueue one Runge-Kutta stage.
@@ -426,13 +412,18 @@ static int64_t enqueue_stage(m2cg_ctx* x, int stage, bool last, const StateSet& 
   cudaStream_t s = x->stream;
   const Params& P = x->P;
   int64_t n = 0;
-  // Interface Riemann solves on stream2: the budgeted first pass alone on the
-  // GPU, then the stragglers on a few reserved SMs while this stream
-  // reconstructs and evaluates the same-material face fluxes on the others.
-  // With ReconstructionAtInterface = Constant the solves read the cell-centre
-  // stage input and go first; otherwise they follow the reconstruction.
+  // Interface Riemann solves on stream2: the budgeted first pass, then the
+  // stragglers on a few reserved SMs while this stream reconstructs and
+  // evaluates the same-material face fluxes on the others.  With
+  // ReconstructionAtInterface = Constant the solves read the cell-centre stage
+  // input and go first; otherwise they follow the reconstruction.
+  // Where the stage before left no stalled solves, reconstruction and fluxes run
+  // beside the first pass (a latency-bound kernel: 128^3 stirred bubble 6.1 ->
+  // 5.1 ms a step); where it did, they wait for its end, so that the pass ends
+  // early and the stragglers, the longest chain of the stage, find empty SMs
+  // (256^3 bubble from rest: 165 against 172-196 ms).
   const bool after_recon = (P.mp_recon != M2CG_MPREC_CONSTANT);
-  if (after_recon) { PHASE(PH_RECON, launch_reconstruct(s, P, in, x->id, x->d_fs, x->cnt)); n += 2; }
+  if (after_recon) { PHASE(PH_RECON, launch_reconstruct(s, P, in, x->id, x->d_fs, x->cnt, Gate{})); n += 2; }
   cudaEventRecord(x->ev_fork, s);
   cudaStreamWaitEvent(x->stream2, x->ev_fork, 0);
   const float* warm = nullptr;
@@ -450,13 +441,13 @@ static int64_t enqueue_stage(m2cg_ctx* x, int stage, bool last, const StateSet& 
   PHASE_ON(PH_RIEMANN_B, x->stream2,
            launch_riemann_stragglers(x->stream2, P, x->d_mats, in, x->id, x->d_fs, x->L, stage == 0, x->scratch,
                                      x->path_cap, x->sblocks, x->sreserve, x->strag, x->strag_count, warm, x->cnt,
-                                     x->sc, x->strag_lanes));
+                                     x->sc, x->strag_lanes, &x->stalled[(stage + 1) % rk_stages(x)]));
   cudaEventRecord(x->ev_join, x->stream2);
   n += 2;
+  n += enqueue_recon_flux(x, s, in, !after_recon, Gate{&x->stalled[stage], 0});
   cudaStreamWaitEvent(s, x->ev_a, 0);
   if (x->hold_cycles > 0) { launch_hold(s, x->hold_cycles); n++; }
-  if (!after_recon) n += enqueue_recon_flux(x, s, in);
-  else { PHASE(PH_FLUX, launch_face_flux(s, P, x->id, x->d_fs, x->d_F, x->cnt)); n++; }
+  n += enqueue_recon_flux(x, s, in, !after_recon, Gate{&x->stalled[stage], 1});
   cudaStreamWaitEvent(s, x->ev_join, 0);
   StageArgs A = stage_args(x, stage, last, in, out);
   if (P.ls_fv) {   // the finite-volume level-set residual of the stage input
@@ -793,7 +784,7 @@ m2cg_status m2cg_compute_residual(m2cg_ctx* x, double* R) {
   cudaStream_t s = x->stream;
   CK(cudaMemsetAsync(x->L.count, 0, sizeof(unsigned long long), s));
   launch_compact(s, x->P, x->id, x->L, x->cnt, nullptr);
-  x->launches += enqueue_recon_flux(x, s, x->S[0]) - 3;
+  x->launches += enqueue_recon_flux(x, s, x->S[0], true, Gate{}) - 3;
   const float* warm = nullptr;
   if (x->mlp) {
     mlp_warm_faces(x->mlp, s, x->nsm, x->P, x->S[0], x->id, x->L, x->w_X, x->w_t, x->w_ref, x->w_p, nullptr);
@@ -803,7 +794,7 @@ m2cg_status m2cg_compute_residual(m2cg_ctx* x, double* R) {
   launch_riemann_interfaces(s, x->P, x->d_mats, x->S[0], x->id, x->d_fs, x->L, 1, x->scratch, x->path_cap, x->rblocks,
                             x->rthreads, x->eval_limit, x->strag, x->strag_count, warm, x->cnt, nullptr);
   launch_riemann_stragglers(s, x->P, x->d_mats, x->S[0], x->id, x->d_fs, x->L, 1, x->scratch, x->path_cap, x->sblocks,
-                            x->sreserve, x->strag, x->strag_count, warm, x->cnt, nullptr, x->strag_lanes);
+                            x->sreserve, x->strag, x->strag_count, warm, x->cnt, nullptr, x->strag_lanes, nullptr);
   StageArgs A;
   memset(&A, 0, sizeof(A));
   A.in = x->S[0];
@@ -1344,9 +1335,9 @@ void m2cg_host_free(void* p) {
 // run as one pool over the concatenated face lists.  The step is captured
 // once into a CUDA graph.
 namespace m2cg {
-void launch_k_reconstruct_ens(cudaStream_t, int64_t, const k_reconstruct_args*, const int64_t*, int);
-void launch_k_reconstruct_ghosts_ens(cudaStream_t, int64_t, const k_reconstruct_ghosts_args*, const int64_t*, int);
-void launch_k_face_flux_ens(cudaStream_t, int64_t, const k_face_flux_args*, const int64_t*, int);
+void launch_k_reconstruct_ens(cudaStream_t, int64_t, const k_reconstruct_args*, const int64_t*, int, const Gate&);
+void launch_k_reconstruct_ghosts_ens(cudaStream_t, int64_t, const k_reconstruct_ghosts_args*, const int64_t*, int, const Gate&);
+void launch_k_face_flux_ens(cudaStream_t, int64_t, const k_face_flux_args*, const int64_t*, int, const Gate&);
 void launch_k_update_ens(cudaStream_t, int64_t, const k_update_args*, const int64_t*, int);
 void launch_k_bc_ens(cudaStream_t, int64_t, const k_bc_args*, const int64_t*, int);
 void launch_k_dt_reduce_ens(cudaStream_t, int64_t, const k_dt_reduce_args*, const int64_t*, int);
@@ -1357,8 +1348,10 @@ void launch_k_commit_remaining_ens(cudaStream_t, int64_t, const k_commit_remaini
 void launch_k_swept_update_ens(cudaStream_t, int64_t, const k_swept_update_args*, const int64_t*, int);
 void launch_k_commit_ids_ens(cudaStream_t, int64_t, const k_commit_ids_args*, const int64_t*, int);
 void launch_reset_counters_ens(cudaStream_t, const CounterResetArgs*, int);
-void launch_riemann_ens(cudaStream_t, const RiemannEnsArgs*, int, int64_t*, double*, int, int, int, int64_t*,
-                        unsigned long long*, int, size_t, int);
+void launch_riemann_ens_first(cudaStream_t, const RiemannEnsArgs*, int, int64_t*, double*, int, int, int, int64_t*,
+                              unsigned long long*);
+void launch_riemann_ens_stragglers(cudaStream_t, const RiemannEnsArgs*, double*, int, const int64_t*,
+                                   const unsigned long long*, int, size_t, int, int*);
 cudaError_t riemann_stragglers_ens_reserve(size_t bytes);
 }  // namespace m2cg
 
@@ -1366,13 +1359,17 @@ struct m2cg_ensemble {
   std::vector<m2cg_ctx*> m;
   int nsm = 0;
   cudaStream_t stream = nullptr;
+  cudaStream_t stream2 = nullptr;   // interface Riemann work, as in a single domain (m2cg_ctx::stream2)
   cudaEvent_t e0 = nullptr, e1 = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_a = nullptr, ev_join = nullptr;
+  long long hold_cycles = 40000;
   double* scratch = nullptr;  // Riemann integration-path pool shared by the members
   int path_cap = 1024, rblocks = 0, sblocks = 0, eval_limit = 16;
   int strag_lanes = 1;         // straggler faces per warp (see m2cg_ctx::strag_lanes)
   size_t sreserve = 0;
   int64_t* strag = nullptr;
   unsigned long long* strag_count = nullptr;
+  int* stalled = nullptr;      // as m2cg_ctx::stalled
   int64_t* off = nullptr;
   std::vector<void*> dev;  // argument tables (device), in the order the step uses them
   size_t tab_i = 0;
@@ -1490,21 +1487,44 @@ static m2cg_status ens_enqueue_step(m2cg_ensemble* e, int64_t* nl) {
     ENS_TABLE(k_face_flux_args, ff);
     ENS_TABLE(k_update_args, up);
     ENS_TABLE(k_bc_args, bc);
-    const bool after_recon = (x0->P.mp_recon != M2CG_MPREC_CONSTANT);
-    auto recon = [&]() -> m2cg_status {
-      { int64_t nb_; int64_t* bo_ = ens_boff(e, ens_cell_threads, 128, &nb_); if (!bo_) { set_err("ensemble table"); return M2CG_ERR_CUDA; } if (!e->building) launch_k_reconstruct_ens(s, nb_, rc_d, bo_, D); }
-      { int64_t nb_; int64_t* bo_ = ens_boff(e, ens_ghosts, 128, &nb_); if (!bo_) { set_err("ensemble table"); return M2CG_ERR_CUDA; } if (!e->building) launch_k_reconstruct_ghosts_ens(s, nb_, rg_d, bo_, D); }
+    // The interface solves on stream2 beside reconstruction and fluxes, gated as in a single domain.
+    int64_t nb_rc, nb_rg, nb_ff;
+    int64_t* bo_rc = ens_boff(e, ens_cell_threads, 128, &nb_rc);
+    int64_t* bo_rg = ens_boff(e, ens_ghosts, 128, &nb_rg);
+    int64_t* bo_ff = ens_boff(e, ens_face_threads, 128, &nb_ff);
+    if (!bo_rc || !bo_rg || !bo_ff) { set_err("ensemble table"); return M2CG_ERR_CUDA; }
+    auto recon = [&](const Gate& gt) {
+      if (!e->building) launch_k_reconstruct_ens(s, nb_rc, rc_d, bo_rc, D, gt);
+      if (!e->building) launch_k_reconstruct_ghosts_ens(s, nb_rg, rg_d, bo_rg, D, gt);
       n += 2;
-      return M2CG_OK;
     };
-    if (after_recon) { m2cg_status st = recon(); if (st != M2CG_OK) return st; }
-    if (!e->building) launch_riemann_ens(s, ra_d, D, e->off, e->scratch, e->path_cap, e->rblocks, e->eval_limit, e->strag,
-                       e->strag_count, e->sblocks, e->sreserve, e->strag_lanes);
-    n += 3;
-    if (!after_recon) { m2cg_status st = recon(); if (st != M2CG_OK) return st; }
-    { int64_t nb_; int64_t* bo_ = ens_boff(e, ens_face_threads, 128, &nb_); if (!bo_) { set_err("ensemble table"); return M2CG_ERR_CUDA; } if (!e->building) launch_k_face_flux_ens(s, nb_, ff_d, bo_, D); }
+    const bool after_recon = (x0->P.mp_recon != M2CG_MPREC_CONSTANT);
+    auto recon_flux = [&](const Gate& gt) {
+      if (!after_recon) recon(gt);
+      if (!e->building) launch_k_face_flux_ens(s, nb_ff, ff_d, bo_ff, D, gt);
+      n++;
+    };
+    if (after_recon) recon(Gate{});
+    if (!e->building) {
+      cudaEventRecord(e->ev_fork, s);
+      cudaStreamWaitEvent(e->stream2, e->ev_fork, 0);
+      launch_riemann_ens_first(e->stream2, ra_d, D, e->off, e->scratch, e->path_cap, e->rblocks, e->eval_limit, e->strag,
+                               e->strag_count);
+      cudaEventRecord(e->ev_a, e->stream2);
+      launch_riemann_ens_stragglers(e->stream2, ra_d, e->scratch, e->path_cap, e->strag, e->strag_count, e->sblocks,
+                                    e->sreserve, e->strag_lanes, &e->stalled[(stage + 1) % nst]);
+      cudaEventRecord(e->ev_join, e->stream2);
+    }
+    recon_flux(Gate{&e->stalled[stage], 0});
+    if (!e->building) {
+      cudaStreamWaitEvent(s, e->ev_a, 0);
+      launch_hold(s, e->hold_cycles);
+    }
+    recon_flux(Gate{&e->stalled[stage], 1});
+    n += 4;
+    if (!e->building) cudaStreamWaitEvent(s, e->ev_join, 0);
     { int64_t nb_; int64_t* bo_ = ens_boff(e, ens_cell_threads, 128, &nb_); if (!bo_) { set_err("ensemble table"); return M2CG_ERR_CUDA; } if (!e->building) launch_k_update_ens(s, nb_, up_d, bo_, D); }
-    n += 2;
+    n++;
     if (!last) { { int64_t nb_; int64_t* bo_ = ens_boff(e, ens_ghosts, 128, &nb_); if (!bo_) { set_err("ensemble table"); return M2CG_ERR_CUDA; } if (!e->building) launch_k_bc_ens(s, nb_, bc_d, bo_, D); } n++; }
   }
   {
@@ -1563,9 +1583,11 @@ void m2cg_ensemble_destroy(m2cg_ensemble* e) {
   if (e->scratch) cudaFree(e->scratch);
   if (e->strag) cudaFree(e->strag);
   if (e->strag_count) cudaFree(e->strag_count);
+  if (e->stalled) cudaFree(e->stalled);
   if (e->off) cudaFree(e->off);
-  if (e->e0) cudaEventDestroy(e->e0);
-  if (e->e1) cudaEventDestroy(e->e1);
+  for (cudaEvent_t ev : {e->e0, e->e1, e->ev_fork, e->ev_a, e->ev_join})
+    if (ev) cudaEventDestroy(ev);
+  if (e->stream2) { cudaStreamSynchronize(e->stream2); cudaStreamDestroy(e->stream2); }
   if (e->stream) cudaStreamDestroy(e->stream);
   delete e;
 }
@@ -1607,10 +1629,18 @@ m2cg_status m2cg_ensemble_create(const m2cg_config* cfgs, int32_t n, m2cg_ensemb
   e->rblocks = e->nsm * 2;
   e->sblocks = e->nsm;
   if (const char* v = getenv("M2CG_RIEMANN_STRAGGLER_LANES")) e->strag_lanes = std::min(32, std::max(1, atoi(v)));
+  if (const char* v = getenv("M2CG_RIEMANN_HOLD_CYCLES")) e->hold_cycles = std::max(0ll, atoll(v));
+  int prio_low = 0, prio_high = 0;
   if (cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high) != cudaSuccess ||
+      cudaStreamCreateWithPriority(&e->stream2, cudaStreamNonBlocking, prio_high) != cudaSuccess ||
+      cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&e->ev_a, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&e->ev_join, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreate(&e->e0) != cudaSuccess || cudaEventCreate(&e->e1) != cudaSuccess ||
       cudaMalloc(&e->scratch, (size_t)6 * e->path_cap * e->rblocks * 128 * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&e->strag_count, sizeof(unsigned long long)) != cudaSuccess ||
+      cudaMalloc(&e->stalled, 3 * sizeof(int)) != cudaSuccess || cudaMemset(e->stalled, 0, 3 * sizeof(int)) != cudaSuccess ||
       cudaMalloc(&e->off, (size_t)(n + 1) * sizeof(int64_t)) != cudaSuccess) {
     set_err("ensemble set-up failed: %s", cudaGetErrorString(cudaGetLastError()));
     m2cg_ensemble_destroy(e);
@@ -1665,7 +1695,7 @@ m2cg_status m2cg_ensemble_run(m2cg_ensemble* e, int32_t n_steps, float* ms) {
     cudaError_t ce = cudaStreamEndCapture(s, &g);
     if (st != M2CG_OK) return st;
     CK(ce);
-    CK(cudaGraphInstantiate(&e->graph, g, 0));
+    CK(cudaGraphInstantiate(&e->graph, g, cudaGraphInstantiateFlagUseNodePriority));
     cudaGraphDestroy(g);
     e->launches_per_step = nl;
   }

@@ -33,28 +33,34 @@ struct Mats {
 // FP64-pipe slots too.  Sign and range tests on a double's bit pattern run on
 // the integer pipe instead (IEEE-754 binary64 orders like a sign-magnitude
 // integer).
+// The tests read the two 32-bit words: the compiler turns the same tests on the
+// 64-bit pattern back into FP64 comparisons (78 FP64 instructions per cell in
+// the reconstruction).
 M2CG_DEV long long bits(double x) { return __double_as_longlong(x); }
-M2CG_DEV bool is_finite_bits(double x) { return (bits(x) & 0x7ff0000000000000ll) != 0x7ff0000000000000ll; }
+M2CG_DEV int hi_word(double x) { return __double2hiint(x); }
+M2CG_DEV unsigned lo_word(double x) { return (unsigned)__double2loint(x); }
+M2CG_DEV bool is_finite_bits(double x) { return (hi_word(x) & 0x7ff00000) != 0x7ff00000; }
 // x <= 0 (both zeros included)
-M2CG_DEV bool le_zero_bits(double x) { return bits(x) <= 0; }
+M2CG_DEV bool le_zero_bits(double x) { return hi_word(x) < 0 || ((unsigned)hi_word(x) | lo_word(x)) == 0u; }
 // x < 0 (negative zero excluded)
-M2CG_DEV bool lt_zero_bits(double x) { long long b = bits(x); return b < 0 && b != (long long)0x8000000000000000ull; }
+M2CG_DEV bool lt_zero_bits(double x) { return hi_word(x) < 0 && (((unsigned)hi_word(x) << 1) | lo_word(x)) != 0u; }
 // |x| < c for a positive constant c
 M2CG_DEV bool abs_lt_bits(double x, double c) { return (bits(x) & 0x7fffffffffffffffll) < bits(c); }
-M2CG_DEV bool is_pos_inf(double x) { return bits(x) == 0x7ff0000000000000ll; }
-M2CG_DEV bool is_neg_inf(double x) { return bits(x) == (long long)0xfff0000000000000ull; }
+M2CG_DEV bool is_pos_inf(double x) { return hi_word(x) == 0x7ff00000 && lo_word(x) == 0u; }
+M2CG_DEV bool is_neg_inf(double x) { return hi_word(x) == (int)0xfff00000 && lo_word(x) == 0u; }
 // Comparisons, minima and maxima of any two doubles on the integer pipe: the
 // results of the FP64 instructions for every operand (an FP64 comparison costs
 // a full slot of the FP64 pipe, and 115 cycles of latency on a dependent chain).
-M2CG_DEV bool is_nan_bits(double x) { return (bits(x) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll; }
-M2CG_DEV bool i_le0(double x) {   // x <= 0: +0, or -0 down to -infinity
-  const unsigned long long u = (unsigned long long)bits(x);
-  return u == 0ull || u - 0x8000000000000000ull <= 0x7ff0000000000000ull;
+M2CG_DEV bool is_nan_bits(double x) {
+  const int h = hi_word(x) & 0x7fffffff;
+  return h > 0x7ff00000 || (h == 0x7ff00000 && lo_word(x) != 0u);
 }
-M2CG_DEV bool i_lt0(double x) {   // x < 0
-  return (unsigned long long)bits(x) - 0x8000000000000001ull <= 0x7fefffffffffffffull;
-}
-M2CG_DEV bool i_eq0(double x) { return ((unsigned long long)bits(x) << 1) == 0ull; }
+M2CG_DEV bool i_eq0(double x) { return (((unsigned)hi_word(x) << 1) | lo_word(x)) == 0u; }
+M2CG_DEV bool i_lt0(double x) { return hi_word(x) < 0 && !i_eq0(x) && !is_nan_bits(x); }             // x < 0
+M2CG_DEV bool i_le0(double x) { return i_eq0(x) || (hi_word(x) < 0 && !is_nan_bits(x)); }            // x <= 0
+M2CG_DEV bool i_gt0(double x) { return hi_word(x) >= 0 && !i_eq0(x) && !is_nan_bits(x); }            // x > 0
+M2CG_DEV bool i_ge0(double x) { return i_eq0(x) || (hi_word(x) >= 0 && !is_nan_bits(x)); }           // x >= 0
+M2CG_DEV double flip_sign(double x) { return __hiloint2double(hi_word(x) ^ (int)0x80000000, __double2loint(x)); }
 // order-preserving integer of a double that is not NaN (-0 just below +0)
 M2CG_DEV long long i_key(double x) {
   const int m = __double2hiint(x) >> 31;
@@ -64,13 +70,15 @@ M2CG_DEV bool i_special(double a, double b) {   // an infinity or NaN among the 
   return (__double2hiint(a) & 0x7ff00000) == 0x7ff00000 || (__double2hiint(b) & 0x7ff00000) == 0x7ff00000;
 }
 static __device__ __noinline__ bool lt_fp64(double a, double b) { return a < b; }
+static __device__ __noinline__ bool le_fp64(double a, double b) { return a <= b; }
+static __device__ __noinline__ double max_fp64(double a, double b) { return fmax(a, b); }
 static __device__ __noinline__ double min_fp64(double a, double b) { return fmin(a, b); }
 M2CG_DEV bool i_lt(double a, double b) {
   if (i_special(a, b)) return lt_fp64(a, b);
   return i_key(a) < i_key(b) && ((bits(a) | bits(b)) << 1) != 0;
 }
 M2CG_DEV bool i_le(double a, double b) {
-  if (i_special(a, b)) return lt_fp64(a, b) || a == b;
+  if (i_special(a, b)) return le_fp64(a, b);
   return i_key(a) <= i_key(b) || ((bits(a) | bits(b)) << 1) == 0;
 }
 M2CG_DEV double i_min(double a, double b) {
@@ -78,7 +86,7 @@ M2CG_DEV double i_min(double a, double b) {
   return i_key(a) <= i_key(b) ? a : b;
 }
 M2CG_DEV double i_max(double a, double b) {
-  if (i_special(a, b)) return -min_fp64(-a, -b);
+  if (i_special(a, b)) return max_fp64(a, b);
   return i_key(a) >= i_key(b) ? a : b;
 }
 // a b < 0: opposite signs, unless the product underflows to zero or an operand is zero or NaN
@@ -88,12 +96,12 @@ M2CG_DEV bool i_prod_lt0(double a, double b) {
   return (bits(a) ^ bits(b)) < 0;
 }
 
-M2CG_DEV bool i_ge0(double x) {   // x >= 0
-  const unsigned long long u = (unsigned long long)bits(x);
-  return u <= 0x7ff0000000000000ull || u == 0x8000000000000000ull;
+// a b > 0 likewise
+M2CG_DEV bool i_prod_gt0(double a, double b) {
+  const unsigned ea = (unsigned)(bits(a) >> 52) & 0x7ffu, eb = (unsigned)(bits(b) >> 52) & 0x7ffu;
+  if (ea + eb < 1100u || ea - 1u > 2045u || eb - 1u > 2045u) return __dmul_rn(a, b) > 0.0;
+  return (bits(a) ^ bits(b)) >= 0;
 }
-M2CG_DEV bool i_gt0(double x) { return (unsigned long long)bits(x) - 1ull <= 0x7fefffffffffffffull; }
-
 // Reciprocal and reciprocal square root to 0.51 ulp on the integer pipe
 // (m2cg_intfp.cuh: 68 and 99 cycles per warp against 204 and 369 for the
 // refined FP64 estimates, and none of them on the FP64 pipe that bounds the
@@ -225,7 +233,7 @@ M2CG_DEV bool eos_bad5_fast(const DevMat& M, const double* V) {
   if (!is_finite_bits(V[0]) || !is_finite_bits(V[1]) || !is_finite_bits(V[2]) || !is_finite_bits(V[3]) ||
       !is_finite_bits(V[4]))
     return true;
-  if (M.type == M2CG_EOS_SG || M.type == M2CG_EOS_NASG) return le_zero_bits(V[0]) || i_le(V[4], -M.Pstiff);   // p + Pstiff <= 0 without the addition
+  if (M.type == M2CG_EOS_SG || M.type == M2CG_EOS_NASG) return le_zero_bits(V[0]) || i_le(V[4], flip_sign(M.Pstiff));   // p + Pstiff <= 0 without the addition
   return eos_bad(M, V[0], V[4]);
 }
 M2CG_DEV bool eos_clip_fast(const DevMat& M, double* V) {
@@ -548,11 +556,26 @@ M2CG_DEV bool flux_genroe(const DevMat& M, int dir, const double* Vm, const doub
 }
 
 // ---- slope limiters (Reconstructor.h:96-111) ------------------------------------
-M2CG_DEV double gen_minmod(double alpha, double dq0, double dq1) {
+// The candidate of smallest magnitude on the integer pipe (equal signs order
+// like the bit patterns, and alpha min(|dq0|, |dq1|) rounds like the smaller of
+// the two products): two FP64 instructions against nine.  The same value as the
+// reference's form, whose comparisons make NaN differences give 0.
+static __device__ __noinline__ double gen_minmod_fp64(double alpha, double dq0, double dq1) {
   // uniform mesh: A = B = 1, so B/(A+1) = 0.5
   if (dq0 < 0.0 && dq1 < 0.0) return fmax(alpha * dq0, fmax(0.5 * (dq0 + dq1), alpha * dq1));
   if (dq0 > 0.0 && dq1 > 0.0) return fmin(alpha * dq0, fmin(0.5 * (dq0 + dq1), alpha * dq1));
   return 0.0;
+}
+static __device__ __noinline__ double gen_minmod(double alpha, double dq0, double dq1) {
+  const unsigned long long MAG = 0x7fffffffffffffffull;
+  const unsigned long long u0 = (unsigned long long)bits(dq0) & MAG, u1 = (unsigned long long)bits(dq1) & MAG;
+  if ((bits(dq0) ^ bits(dq1)) < 0 || u0 == 0ull || u1 == 0ull || is_nan_bits(dq0) || is_nan_bits(dq1)) return 0.0;
+  const double s = __dadd_rn(dq0, dq1);
+  const int es = __double2hiint(s) & 0x7ff00000;
+  if (es <= 0x00100000 || es == 0x7ff00000 || !(bits(alpha) > 0)) return gen_minmod_fp64(alpha, dq0, dq1);
+  const double h = __hiloint2double(__double2hiint(s) - 0x00100000, __double2loint(s));   // s / 2
+  const double t = __dmul_rn(alpha, u0 < u1 ? dq0 : dq1);
+  return ((unsigned long long)bits(h) & MAG) < ((unsigned long long)bits(t) & MAG) ? h : t;
 }
 // van Albada on the integer pipe (if_van_albada: 182 cycles per warp with one
 // FP64 multiplication, against 666 for the FP64 form with its ten); products

@@ -6,6 +6,18 @@
 
 namespace m2cg {
 
+// Member owning flat block b of a batched launch: largest d with boff[d] <= b
+// (members without blocks in the launch are never found).
+__device__ __forceinline__ int ens_member(const int64_t* __restrict__ boff, int D, int64_t b) {
+  int lo = 0, hi = D - 1;
+  while (lo < hi) {
+    int mid = (lo + hi + 1) >> 1;
+    if (boff[mid] <= b) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+
 struct k_reconstruct_args {
   Params P;
   StateSet S;

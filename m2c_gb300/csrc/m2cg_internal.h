@@ -1,7 +1,6 @@
 // Internal definitions shared by the kernels and the host API of libm2cg.
 #pragma once
 #include <cstdint>
-#include <cuda.h>   // CUtensorMap (encoded through the runtime's driver entry point)
 #include <cuda_runtime.h>
 #include "m2cg_device.cuh"
 #include "m2cg_riemann.cuh"
@@ -78,7 +77,7 @@ M2CG_DEV bool ghost_face_cell(const Grid& g, int64_t t, int& side, int& i, int& 
 enum {
   CNT_IFACE = 0, CNT_RERR, CNT_RITER, CNT_RSOLVE, CNT_CLIPCELL, CNT_CLIPFACE, CNT_BAD, CNT_SWEPT, CNT_UNRES,
   CNT_IF_OVERFLOW, CNT_PATH_CAPPED, CNT_SWEPT_OVERFLOW, CNT_BADID, CNT_FALLBACK, CNT_UNRES_FIXED,
-  CNT_UNRES_OVERFLOW, CNT_UNRES_REPAIRS, CNT_TILE_TIMEOUT, CNT_N
+  CNT_UNRES_OVERFLOW, CNT_UNRES_REPAIRS, CNT_N
 };
 
 // Scalars that live on the device for the whole run (no host round trip per step).
@@ -89,6 +88,7 @@ struct DevScalars {
   int pad;
   long long steps;
   double dt_in;     // the time step a caller gave m2cg_advance (its step graph reads it here)
+  double cf[3][3];  // per Runge-Kutta stage and direction: -area / volume times the stage's share of dt
 };
 
 struct Params {
@@ -120,6 +120,15 @@ struct Params {
   double fd3l[3][4], fd3r[3][4];
   double cfl, timestep, max_time;
   int ts_type;
+};
+
+// Reconstruction and fluxes are enqueued twice per stage, before and after the
+// wait for the first Riemann pass; a launch runs only where the device flag
+// (the previous stage left stalled solves) has the value it wants.
+struct Gate {
+  const int* flag;   // NULL: always run
+  int want;
+  M2CG_DEV bool closed() const { return flag && *flag != want; }
 };
 
 // A primitive state set: rho, u, v, w, p, phi (SoA, ghosted).
@@ -242,17 +251,5 @@ struct StageArgs {
   const double* rls_pre;      // level-set residual computed beforehand (finite volume), else NULL
   int residual_only;
 };
-
-// Tensor maps of the five primitive arrays of one state set for the fused
-// reconstruction + flux kernel (m2cg_tile.cu): 3D (x, y, z) over the ghosted
-// arrays, box 36 x 7 x 1.
-struct TileMaps {
-  CUtensorMap v[5];
-};
-bool tile_supported(const Params& P);
-bool tile_maps(const Params& P, const StateSet& S, TileMaps* out);
-cudaError_t tile_prepare();
-void launch_recon_flux_tile(cudaStream_t s, const TileMaps& maps, const Params& P, const StateSet& S,
-                            const int32_t* id, double* const* F, unsigned long long* cnt, int zchunk);
 
 }  // namespace m2cg

@@ -210,8 +210,8 @@ M2CG_INT_SLOW double dsqrt(double x) {
 // the smaller: a h, h = b (a + b) / (a^2 + b^2) in [1, 1.21], h in fixed point
 // from the significands (a's shifted to b's exponent: h depends on a / b to
 // 2^-60) and one binary64 multiplication; 0 for opposite signs and for a
-// product below 1e-16.  Returns 1 with the slope, or 0 where the product is
-// next to 1e-16 or an operand is special (the caller's FP64 form decides).
+// product below 1e-16.  Returns 1 with the slope, or 0 where the product rounds
+// at 1e-16 or an operand is special (the caller's FP64 form decides).
 M2CG_INT int if_van_albada(double x, double y, double& out) {
   const uint32_t xh = if_hi(x), yh = if_hi(y);
   const uint32_t ux = xh & 0x7fffffffu, uy = yh & 0x7fffffffu;
@@ -223,8 +223,14 @@ M2CG_INT int if_van_albada(double x, double y, double& out) {
   if (eb > 2000u) return 0;
   // the product lies in [2^(ea + eb - 2046), 4 x that); 1e-16 = 2^-53.15
   if (ea + eb <= 1990u) return 1;
-  if (ea + eb < 1994u) return 0;
   if ((int32_t)(ah ^ bh) < 0) return 1;
+  if (ea + eb < 1993u) {
+    // next to the threshold: the product to 2^-62 against 1e-16, undecided only
+    // within the rounding of the product
+    const uint64_t t = if_mulhi64(if_sig(ah, al), if_sig(bh, bl)), c = 16615349947311448064ull >> (ea + eb - 1991u);
+    if (t + 2048u < c) return 1;
+    if (t < c + 2048u) return 0;
+  }
   if (ea == 0u) return 0;
   const uint32_t sh = eb - ea;
   const uint64_t B = if_sig(bh, bl), A = if_sig(ah, al) >> (sh < 63u ? sh : 63u);

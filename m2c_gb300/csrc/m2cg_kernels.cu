@@ -11,32 +11,32 @@
 
 namespace m2cg {
 
-// Member owning flat block b of a batched launch: largest d with boff[d] <= b.
-__device__ __forceinline__ int ens_member(const int64_t* __restrict__ boff, int D, int64_t b) {
-  int lo = 0, hi = D - 1;
-  while (lo < hi) {
-    int mid = (lo + hi + 1) >> 1;
-    if (boff[mid] <= b) lo = mid;
-    else hi = mid - 1;
-  }
-  return lo;
-}
-
-
 __device__ __forceinline__ void atomic_inc(unsigned long long* c, unsigned long long v = 1ull) {
   atomicAdd(c, v);
 }
 
+// (i, j, k) of flat index t over an ex x ey x ez space, x fastest; 32-bit
+// divisions where the space allows (a 64-bit one takes five times as many
+// instructions).
+__device__ __forceinline__ bool flat_index(int ex, int ey, int ez, int64_t t, int& i, int& j, int& k) {
+  const int64_t exy = (int64_t)ex * ey, n = exy * ez;
+  if (t >= n) return false;
+  if (n <= 0x7fffffffll) {
+    const unsigned u = (unsigned)t, row = u / (unsigned)ex;
+    i = (int)(u - row * (unsigned)ex);
+    k = (int)(row / (unsigned)ey);
+    j = (int)(row - (unsigned)k * (unsigned)ey);
+    return true;
+  }
+  k = (int)(t / exy);
+  const int64_t r = t - (int64_t)k * exy;
+  j = (int)(r / ex);
+  i = (int)(r - (int64_t)j * ex);
+  return true;
+}
 // Linear index of a real cell from a flat thread id over nx*ny*nz.
 __device__ __forceinline__ bool real_cell(const Grid& g, int64_t t, int& i, int& j, int& k) {
-  int64_t n = (int64_t)g.nx * g.ny * g.nz;
-  if (t >= n) return false;
-  int64_t nxy = (int64_t)g.nx * g.ny;
-  k = (int)(t / nxy);
-  int64_t r = t - (int64_t)k * nxy;
-  j = (int)(r / g.nx);
-  i = (int)(r - (int64_t)j * g.nx);
-  return true;
+  return flat_index(g.nx, g.ny, g.nz, t, i, j, k);
 }
 
 // Real cell of this thread in block bx of a cell kernel (the grid's block shape).
@@ -72,7 +72,8 @@ __device__ __forceinline__ void store_faces(const DevMat& M, const double* q, do
 // ---------------------------------------------------------------------------
 // K1: MUSCL reconstruction of the six face states of every real cell
 // (Reconstructor.cpp:426-782) followed by CheckReconstructedStates
-// (SpaceOperator.cpp:2446-2484).  fs[f*5+p]: f = vl, vr, vb, vt, vk, vf.
+// (SpaceOperator.cpp:2446-2484).  fs[f*5+p]: f = vl, vr, vb, vt, vk, vf.  One
+// direction at a time, so that a thread holds two face states, not six.
 __device__ __forceinline__ void k_reconstruct_body(const Params& P, const StateSet& S, const int32_t* __restrict__ id, double* const* fs, unsigned long long* cnt, unsigned bx_, unsigned gx_) {
   int i, j, k;
   if (!block_cell(P.g, bx_, i, j, k)) return;
@@ -83,17 +84,19 @@ __device__ __forceinline__ void k_reconstruct_body(const Params& P, const StateS
   for (int p = 0; p < 5; p++) q[p] = S.q[p][c];
   const int myid = id[c];
   const DevMat& M = P.mats.m[myid];
-  double face[6][5];
-  if (P.rec_type == M2CG_REC_CONSTANT) {
+  const int64_t st[3] = {1, g.sy, g.sz};
+  bool done = false;   // the cell's revert chain, carried across directions
+  int nclip = 0, nbad = 0;
 #pragma unroll
-    for (int f = 0; f < 6; f++)
+  for (int d = 0; d < 3; d++) {
+    double vm[5], vp[5];
+    bool badm, badp;
+    if (P.rec_type == M2CG_REC_CONSTANT) {
 #pragma unroll
-      for (int p = 0; p < 5; p++) face[f][p] = q[p];
-  } else {
-    const int64_t st[3] = {1, g.sy, g.sz};
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      bool zero = P.slope_zero && (id[c - st[d]] != myid || id[c + st[d]] != myid);
+      for (int p = 0; p < 5; p++) { vm[p] = q[p]; vp[p] = q[p]; }
+      badm = badp = eos_bad5_fast(M, q);
+    } else {
+      const bool zero = P.slope_zero && (id[c - st[d]] != myid || id[c + st[d]] != myid);
 #pragma unroll
       for (int p = 0; p < 5; p++) {
         double dq0 = q[p] - S.q[p][c - st[d]];
@@ -103,29 +106,56 @@ __device__ __forceinline__ void k_reconstruct_body(const Params& P, const StateS
         else if (P.limiter == M2CG_LIM_GENERALIZED_MINMOD) s = gen_minmod(P.minmod_coeff, dq0, dq1);
         else s = 0.5 * (dq0 + dq1);
         if (zero) s = 0.0;
-        face[2 * d][p] = fma(-0.5, s, q[p]);
-        face[2 * d + 1][p] = fma(0.5, s, q[p]);
+        vm[p] = fma(-0.5, s, q[p]);
+        vp[p] = fma(0.5, s, q[p]);
       }
-    }
-    // Reconstructor.cpp:722-778: the first nonphysical face state reverts to the cell value
-    bool done = false;
+      // Reconstructor.cpp:722-778: the first nonphysical face state reverts to the cell value
+      badm = eos_bad5_fast(M, vm);
+      badp = eos_bad5_fast(M, vp);
+      if (!done && badm) {
 #pragma unroll
-    for (int f = 0; f < 6; f++) {
-      bool bad = !done && eos_bad5_fast(M, face[f]);
-      if (bad) {
+        for (int p = 0; p < 5; p++) vm[p] = q[p];
+        badm = eos_bad5_fast(M, vm);
+        done = true;
+      }
+      if (!done && badp) {
 #pragma unroll
-        for (int p = 0; p < 5; p++) face[f][p] = q[p];
+        for (int p = 0; p < 5; p++) vp[p] = q[p];
+        badp = eos_bad5_fast(M, vp);
         done = true;
       }
     }
+    // CheckReconstructedStates (SpaceOperator.cpp:2446-2484)
+    double t[5] = {vm[0], vm[1], vm[2], vm[3], vm[4]};
+    if (eos_clip_fast(M, t)) {
+#pragma unroll
+      for (int p = 0; p < 5; p++) vm[p] = q[p];
+      badm = eos_bad5_fast(M, vm);
+      nclip++;
+    }
+#pragma unroll
+    for (int p = 0; p < 5; p++) t[p] = vp[p];
+    if (eos_clip_fast(M, t)) {
+#pragma unroll
+      for (int p = 0; p < 5; p++) vp[p] = q[p];
+      badp = eos_bad5_fast(M, vp);
+      nclip++;
+    }
+    nbad += (int)badm + (int)badp;
+#pragma unroll
+    for (int p = 0; p < 5; p++) { fs[(2 * d) * 5 + p][c] = vm[p]; fs[(2 * d + 1) * 5 + p][c] = vp[p]; }
   }
-  store_faces(M, q, face, fs, c, cnt);
+  if (nclip) atomic_inc(&cnt[CNT_CLIPFACE], nclip);
+  if (nbad) atomic_inc(&cnt[CNT_BAD], nbad);
 }
-__global__ void __launch_bounds__(128) k_reconstruct(Params P, StateSet S, const int32_t* __restrict__ id,
-                                                     double* const* fs, unsigned long long* cnt) { k_reconstruct_body(P, S, id, fs, cnt, blockIdx.x, gridDim.x); }
+__global__ void __launch_bounds__(128, 8) k_reconstruct(Params P, StateSet S, const int32_t* __restrict__ id,
+                                                        double* const* fs, unsigned long long* cnt, Gate gt) {
+  if (!gt.closed()) k_reconstruct_body(P, S, id, fs, cnt, blockIdx.x, gridDim.x);
+}
 // batched: the launch's blocks are the members' blocks back to back
 // (boff: exclusive prefix of the members' block counts)
-__global__ void __launch_bounds__(128) k_reconstruct_ens(const k_reconstruct_args* __restrict__ ea, const int64_t* __restrict__ boff, int D, int64_t nvb) {
+__global__ void __launch_bounds__(128, 6) k_reconstruct_ens(const k_reconstruct_args* __restrict__ ea, const int64_t* __restrict__ boff, int D, int64_t nvb, Gate gt) {
+  if (gt.closed()) return;
   // persistent: the launch's blocks take the members' blocks in turn
   for (int64_t b = blockIdx.x; b < nvb; b += gridDim.x) {
     const int d = ens_member(boff, D, b);
@@ -305,8 +335,9 @@ __device__ __forceinline__ void reconstruct_var_cell(const Params& P, const Stat
 
 template <int VT>
 __global__ void __launch_bounds__(128) k_reconstruct_var(Params P, StateSet S, const int32_t* __restrict__ id,
-                                                         double* const* fs, unsigned long long* cnt) {
+                                                         double* const* fs, unsigned long long* cnt, Gate gt) {
   int i, j, k;
+  if (gt.closed()) return;
   if (!real_cell(P.g, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
   const int64_t c = P.g.at(i, j, k);
   double q[5];
@@ -350,10 +381,13 @@ __device__ __forceinline__ void k_reconstruct_ghosts_body(const Params& P, const
   for (int p = 0; p < 5; p++) fs[inward * 5 + p][c] = t[p];
 }
 __global__ void k_reconstruct_ghosts(Params P, StateSet S, const int32_t* __restrict__ id, double* const* fs,
-                                     unsigned long long* cnt) { k_reconstruct_ghosts_body(P, S, id, fs, cnt, blockIdx.x, gridDim.x); }
+                                     unsigned long long* cnt, Gate gt) {
+  if (!gt.closed()) k_reconstruct_ghosts_body(P, S, id, fs, cnt, blockIdx.x, gridDim.x);
+}
 // batched: the launch's blocks are the members' blocks back to back
 // (boff: exclusive prefix of the members' block counts)
-__global__ void k_reconstruct_ghosts_ens(const k_reconstruct_ghosts_args* __restrict__ ea, const int64_t* __restrict__ boff, int D) {
+__global__ void k_reconstruct_ghosts_ens(const k_reconstruct_ghosts_args* __restrict__ ea, const int64_t* __restrict__ boff, int D, Gate gt) {
+  if (gt.closed()) return;
   const int d = ens_member(boff, D, blockIdx.x);
   const k_reconstruct_ghosts_args& e = ea[d];
   k_reconstruct_ghosts_body(e.P, e.S, e.id, e.fs, e.cnt, (unsigned)(blockIdx.x - boff[d]), (unsigned)(boff[d + 1] - boff[d]));
@@ -376,14 +410,7 @@ __device__ __forceinline__ void k_face_flux_body(const Params& P, const int32_t*
   if (g.tile[0]) {
     if (!tiled_index(g.nx + 1, g.ny + 1, g.nz + 1, g.tile, bx_, threadIdx.x, i, j, k)) return;
   } else {
-    int64_t t = (int64_t)bx_ * blockDim.x + threadIdx.x;
-    int64_t ex = g.nx + 1, ey = g.ny + 1;
-    int64_t n = ex * ey * (g.nz + 1);
-    if (t >= n) return;
-    k = (int)(t / (ex * ey));
-    int64_t r = t - (int64_t)k * ex * ey;
-    j = (int)(r / ex);
-    i = (int)(r - (int64_t)j * ex);
+    if (!flat_index(g.nx + 1, g.ny + 1, g.nz + 1, (int64_t)bx_ * blockDim.x + threadIdx.x, i, j, k)) return;
   }
   int64_t c = g.at(i, j, k);
   const int64_t st[3] = {1, g.sy, g.sz};
@@ -405,10 +432,13 @@ __device__ __forceinline__ void k_face_flux_body(const Params& P, const int32_t*
   if (bad) atomic_inc(&cnt[CNT_BAD], bad);
 }
 __global__ void __launch_bounds__(128) k_face_flux(Params P, const int32_t* __restrict__ id, double* const* fs, double* const* F,
-                            unsigned long long* cnt) { k_face_flux_body(P, id, fs, F, cnt, blockIdx.x, gridDim.x); }
+                            unsigned long long* cnt, Gate gt) {
+  if (!gt.closed()) k_face_flux_body(P, id, fs, F, cnt, blockIdx.x, gridDim.x);
+}
 // batched: the launch's blocks are the members' blocks back to back
 // (boff: exclusive prefix of the members' block counts)
-__global__ void __launch_bounds__(128) k_face_flux_ens(const k_face_flux_args* __restrict__ ea, const int64_t* __restrict__ boff, int D, int64_t nvb) {
+__global__ void __launch_bounds__(128) k_face_flux_ens(const k_face_flux_args* __restrict__ ea, const int64_t* __restrict__ boff, int D, int64_t nvb, Gate gt) {
+  if (gt.closed()) return;
   // persistent: the launch's blocks take the members' blocks in turn
   for (int64_t b = blockIdx.x; b < nvb; b += gridDim.x) {
     const int d = ens_member(boff, D, b);
@@ -431,24 +461,26 @@ __device__ __forceinline__ double ls_residual(const Params& P, const double* __r
   double term[3];
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    int64_t s = st[d];
+    // the third-order stencil on the upwind side, its coefficients and start
+    // selected (lanes of a warp with different flow directions stay together):
+    // left-biased over c-2 .. c+1, right-biased over c-1 .. c+2
+    const int64_t s = st[d];
+    const bool left = i_ge0(vel[d]);
+    // the reference's right-biased y coefficients are 3rd order only when
+    // i < NY-1 (GradientCalculatorFD3.cpp:409 tests i, not j)
+    const bool right_third = (d == 1) ? (i < g.ny - 1) : (pos[d] < n[d] - 1);
     double gr;
-    if (vel[d] >= 0) {
-      if (pos[d] - 2 >= -1)
-        gr = P.fd3l[d][0] * phi[c - 2 * s] + P.fd3l[d][1] * phi[c - s] + P.fd3l[d][2] * phi[c] + P.fd3l[d][3] * phi[c + s];
-      else
-        gr = (phi[c] - phi[c - s]) / h[d];
+    if (left ? pos[d] - 2 >= -1 : (pos[d] + 2 <= n[d] && right_third)) {
+      const double* q = phi + c - (left ? 2 * s : s);
+      const double k0 = left ? P.fd3l[d][0] : P.fd3r[d][0], k1 = left ? P.fd3l[d][1] : P.fd3r[d][1];
+      const double k2 = left ? P.fd3l[d][2] : P.fd3r[d][2], k3 = left ? P.fd3l[d][3] : P.fd3r[d][3];
+      gr = k0 * q[0] + k1 * q[s] + k2 * q[2 * s] + k3 * q[3 * s];
+    } else if (left) {
+      gr = (phi[c] - phi[c - s]) / h[d];
+    } else if (pos[d] + 2 <= n[d]) {
+      gr = 0.0 * phi[c - s] + (-1.0 / h[d]) * phi[c] + (1.0 / h[d]) * phi[c + s] + 0.0 * phi[c + 2 * s];
     } else {
-      if (pos[d] + 2 <= n[d]) {
-        // the reference's right-biased y coefficients are 3rd order only when
-        // i < NY-1 (GradientCalculatorFD3.cpp:409 tests i, not j)
-        bool third = (d == 1) ? (i < g.ny - 1) : (pos[d] < n[d] - 1);
-        if (third)
-          gr = P.fd3r[d][0] * phi[c - s] + P.fd3r[d][1] * phi[c] + P.fd3r[d][2] * phi[c + s] + P.fd3r[d][3] * phi[c + 2 * s];
-        else
-          gr = 0.0 * phi[c - s] + (-1.0 / h[d]) * phi[c] + (1.0 / h[d]) * phi[c + s] + 0.0 * phi[c + 2 * s];
-      } else
-        gr = (phi[c + s] - phi[c]) / h[d];
+      gr = (phi[c + s] - phi[c]) / h[d];
     }
     term[d] = gr * vel[d];
   }
@@ -474,12 +506,13 @@ __device__ __forceinline__ void k_update_body(const Params& P, const StageArgs& 
   // -F_minus*A (x, y, z) then +F_plus*A (SpaceOperator.cpp:1703-1705, 1863-1865,
   // 2022-2024); differencing first gives the same value to rounding and an exact
   // zero wherever the two fluxes of a direction are equal, as the reference does
-  // for a uniform flux.
+  // for a uniform flux.  In a step the areas come scaled by the stage's share
+  // of dt over the volume (DevScalars::cf), which saves the products by both.
   double f[5] = {0, 0, 0, 0, 0};
 #pragma unroll
   for (int d = 0; d < 3; d++) {
     int64_t m = c - st[d], pc = c + st[d];
-    const double a = P.area[d];
+    const double a = A.residual_only ? P.area[d] : sc->cf[A.stage][d];
     double fm[5], fp[5];
     if (id[m] != myid) {
       int s = L.slot[d][c];
@@ -498,14 +531,11 @@ __device__ __forceinline__ void k_update_body(const Params& P, const StageArgs& 
       for (int p = 0; p < 5; p++) fp[p] = F[d * 5 + p][pc];
     }
 #pragma unroll
-    for (int p = 0; p < 5; p++) f[p] += (fp[p] - fm[p]) * a;
+    for (int p = 0; p < 5; p++) f[p] = d == 0 ? (fp[p] - fm[p]) * a : fma(fp[p] - fm[p], a, f[p]);
   }
-  double R[5];
-#pragma unroll
-  for (int p = 0; p < 5; p++) R[p] = f[p] * P.inv_negvol;
   if (A.residual_only) {
 #pragma unroll
-    for (int p = 0; p < 5; p++) A.R[p][c] = R[p];
+    for (int p = 0; p < 5; p++) A.R[p][c] = f[p] * P.inv_negvol;
     return;
   }
   const double dt = sc->dt;
@@ -521,11 +551,10 @@ __device__ __forceinline__ void k_update_body(const Params& P, const StageArgs& 
       for (int p = 0; p < 5; p++) A.Un[p][c] = Un[p];
     }
 #pragma unroll
-    for (int p = 0; p < 5; p++) U[p] = Un[p] + dt * R[p];
+    for (int p = 0; p < 5; p++) U[p] = Un[p] + f[p];
   } else {
-    const double cdt = A.c_dt * dt;
 #pragma unroll
-    for (int p = 0; p < 5; p++) U[p] = (A.a_own * A.Us[p][c] + A.b_un * A.Un[p][c]) + cdt * R[p];
+    for (int p = 0; p < 5; p++) U[p] = (A.a_own * A.Us[p][c] + A.b_un * A.Un[p][c]) + f[p];
   }
   double V[5];
   cons_to_prim_fast(M, U, V);
@@ -553,8 +582,8 @@ __device__ __forceinline__ void k_update_body(const Params& P, const StageArgs& 
     if (A.last) {
       // sign change (MultiPhaseOperator.cpp:190-222) -> new ID or "remaining" tag (negative)
       int nid = myid;
-      if (!(ph * phin > 0.0)) {
-        if (ph < 0) nid = P.ls_matid;
+      if (!i_prod_gt0(ph, phin)) {
+        if (i_lt0(ph)) nid = P.ls_matid;
         else nid = -1 - myid;  // resolved from the neighbors after this kernel
         unsigned long long s = atomicAdd(swept_count, 1ull);
         if ((int64_t)s < swept_cap) swept[s] = c;
@@ -804,6 +833,10 @@ __device__ __forceinline__ void k_dt_finalize_body(const Params& P, DevScalars* 
   sc->active = 1;
   sc->dt = dt;
   sc->cfl = cfl;
+  for (int st = 0; st < 3; st++) {
+    const double w = st == 0 ? 1.0 : P.ts_type == M2CG_TS_RK2 ? 0.5 : st == 1 ? 0.25 : 2.0 / 3.0;   // stage_args' c_dt
+    for (int d = 0; d < 3; d++) sc->cf[st][d] = (P.area[d] * P.inv_negvol) * (w * dt);
+  }
   sc->time = t + dt;
   sc->steps += 1;
 }
@@ -1003,16 +1036,8 @@ __global__ void k_commit_ids_ens(const k_commit_ids_args* __restrict__ ea, const
 __device__ __forceinline__ void k_compact_interfaces_body(const Params& P, const int32_t* __restrict__ id, const IfaceList& L, unsigned long long* cnt, const DevScalars* sc, unsigned bx_, unsigned gx_) {
   if (sc && !sc->active) return;
   const Grid& g = P.g;
-  int64_t t = (int64_t)bx_ * blockDim.x + threadIdx.x;
-  int64_t ex = g.nx + 1, ey = g.ny + 1;
-  int64_t n = ex * ey * (g.nz + 1);
-  bool valid = t < n;
   int i = 0, j = 0, k = 0;
-  if (valid) {
-    k = (int)(t / (ex * ey));
-    int64_t r = t - (int64_t)k * ex * ey;
-    j = (int)(r / ex); i = (int)(r - (int64_t)j * ex);
-  }
+  const bool valid = flat_index(g.nx + 1, g.ny + 1, g.nz + 1, (int64_t)bx_ * blockDim.x + threadIdx.x, i, j, k);
   const int64_t st[3] = {1, g.sy, g.sz};
   for (int d = 0; d < 3; d++) {
     bool is_if = false;
@@ -1104,22 +1129,22 @@ __global__ void k_pack(Params P, StateSet S, const int32_t* id, double* Vh, int3
 static inline int nblk(int64_t n, int b) { return (int)((n + b - 1) / b); }
 
 void launch_reconstruct(cudaStream_t s, const Params& P, const StateSet& S, const int32_t* id, double* const* fs,
-                        unsigned long long* cnt) {
+                        unsigned long long* cnt, const Gate& gt) {
   int64_t n = (int64_t)P.g.nx * P.g.ny * P.g.nz;
   if (P.rec_type == M2CG_REC_CONSTANT || P.rec_var == M2CG_VAR_PRIMITIVE)
-    k_reconstruct<<<(unsigned)shaped_blocks(P.g, P.g.nx, P.g.ny, P.g.nz), 128, 0, s>>>(P, S, id, fs, cnt);
+    k_reconstruct<<<(unsigned)shaped_blocks(P.g, P.g.nx, P.g.ny, P.g.nz), 128, 0, s>>>(P, S, id, fs, cnt, gt);
   else if (P.rec_var == M2CG_VAR_CONSERVATIVE)
-    k_reconstruct_var<M2CG_VAR_CONSERVATIVE><<<nblk(n, 128), 128, 0, s>>>(P, S, id, fs, cnt);
+    k_reconstruct_var<M2CG_VAR_CONSERVATIVE><<<nblk(n, 128), 128, 0, s>>>(P, S, id, fs, cnt, gt);
   else if (P.rec_var == M2CG_VAR_PRIMITIVE_CHARACTERISTIC)
-    k_reconstruct_var<M2CG_VAR_PRIMITIVE_CHARACTERISTIC><<<nblk(n, 128), 128, 0, s>>>(P, S, id, fs, cnt);
+    k_reconstruct_var<M2CG_VAR_PRIMITIVE_CHARACTERISTIC><<<nblk(n, 128), 128, 0, s>>>(P, S, id, fs, cnt, gt);
   else
-    k_reconstruct_var<M2CG_VAR_CONSERVATIVE_CHARACTERISTIC><<<nblk(n, 128), 128, 0, s>>>(P, S, id, fs, cnt);
+    k_reconstruct_var<M2CG_VAR_CONSERVATIVE_CHARACTERISTIC><<<nblk(n, 128), 128, 0, s>>>(P, S, id, fs, cnt, gt);
   int64_t ng = 2 * ((int64_t)P.g.ny * P.g.nz + (int64_t)P.g.nx * P.g.nz + (int64_t)P.g.nx * P.g.ny);
-  k_reconstruct_ghosts<<<nblk(ng, 128), 128, 0, s>>>(P, S, id, fs, cnt);
+  k_reconstruct_ghosts<<<nblk(ng, 128), 128, 0, s>>>(P, S, id, fs, cnt, gt);
 }
 void launch_face_flux(cudaStream_t s, const Params& P, const int32_t* id, double* const* fs, double* const* F,
-                      unsigned long long* cnt) {
-  k_face_flux<<<(unsigned)shaped_blocks(P.g, P.g.nx + 1, P.g.ny + 1, P.g.nz + 1), 128, 0, s>>>(P, id, fs, F, cnt);
+                      unsigned long long* cnt, const Gate& gt) {
+  k_face_flux<<<(unsigned)shaped_blocks(P.g, P.g.nx + 1, P.g.ny + 1, P.g.nz + 1), 128, 0, s>>>(P, id, fs, F, cnt, gt);
 }
 void launch_update(cudaStream_t s, const Params& P, const StageArgs& A, const int32_t* id, int32_t* id_new,
                    double* const* F, const IfaceList& L, const DevScalars* sc, int64_t* swept,
@@ -1215,9 +1240,17 @@ static int persistent_grid(KF kernel, int block) {
     static const int grid = persistent_grid(K##_ens, B);                                                \
     if (blocks > 0 && D > 0) K##_ens<<<(unsigned)std::min<int64_t>(blocks, grid), B, 0, s>>>(t, boff, D, blocks); \
   }
-M2CG_ENS_PERSISTENT_LAUNCHER(k_reconstruct, 128)
-M2CG_ENS_LAUNCHER(k_reconstruct_ghosts, 128)
-M2CG_ENS_PERSISTENT_LAUNCHER(k_face_flux, 128)
+#define M2CG_ENS_PERSISTENT_GATED_LAUNCHER(K, B)                                                       \
+  void launch_##K##_ens(cudaStream_t s, int64_t blocks, const K##_args* t, const int64_t* boff, int D, const Gate& gt) { \
+    static const int grid = persistent_grid(K##_ens, B);                                                \
+    if (blocks > 0 && D > 0) K##_ens<<<(unsigned)std::min<int64_t>(blocks, grid), B, 0, s>>>(t, boff, D, blocks, gt); \
+  }
+M2CG_ENS_PERSISTENT_GATED_LAUNCHER(k_reconstruct, 128)
+void launch_k_reconstruct_ghosts_ens(cudaStream_t s, int64_t blocks, const k_reconstruct_ghosts_args* t,
+                                     const int64_t* boff, int D, const Gate& gt) {
+  if (blocks > 0 && D > 0) k_reconstruct_ghosts_ens<<<(unsigned)blocks, 128, 0, s>>>(t, boff, D, gt);
+}
+M2CG_ENS_PERSISTENT_GATED_LAUNCHER(k_face_flux, 128)
 M2CG_ENS_PERSISTENT_LAUNCHER(k_update, 128)
 M2CG_ENS_LAUNCHER(k_bc, 128)
 M2CG_ENS_LAUNCHER(k_dt_reduce, 256)

@@ -23,6 +23,7 @@
 //
 // Compiled without floating-point contraction, like the other interface kernels,
 // so its results equal m2cg_riemann_batch's for the same path-cache capacity.
+#include <cuda.h>
 #include <mutex>
 #include "m2cg_internal.h"
 

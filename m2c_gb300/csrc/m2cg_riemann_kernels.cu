@@ -276,10 +276,12 @@ __global__ void __launch_bounds__(128) k_riemann_stragglers(Params P, const Mats
                                                             IfaceList L, int store, double* scratch, int path_cap,
                                                             size_t reserve_bytes, const int32_t* __restrict__ strag,
                                                             const unsigned long long* strag_count, const float* warm,
-                                                            unsigned long long* cnt, const DevScalars* sc, int lanes) {
+                                                            unsigned long long* cnt, const DevScalars* sc, int lanes,
+                                                            int* stalled) {
   extern __shared__ __align__(16) double s_path[];
   if (sc && !sc->active) return;
   int64_t n = (int64_t)min((unsigned long long)L.cap, *strag_count);
+  if (stalled && blockIdx.x == 0 && threadIdx.x == 0) *stalled = n > 0;   // the next stage's Gate
   const int64_t W = straggler_warps(n, (int64_t)gridDim.x * (blockDim.x >> 5), lanes);
   const int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int64_t lane = threadIdx.x & 31;
@@ -399,9 +401,11 @@ __global__ void k_riemann_interfaces_ens(const RiemannEnsArgs* __restrict__ a, i
 __global__ void __launch_bounds__(128) k_riemann_stragglers_ens(const RiemannEnsArgs* __restrict__ a, double* scratch,
                                                                 int path_cap, size_t reserve_bytes,
                                                                 const int64_t* __restrict__ strag,
-                                                                const unsigned long long* strag_count, int lanes) {
+                                                                const unsigned long long* strag_count, int lanes,
+                                                                int* stalled) {
   extern __shared__ __align__(16) double s_path[];
   const int64_t n = (int64_t)*strag_count;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *stalled = n > 0;   // the next stage's Gate
   const int64_t W = straggler_warps(n, (int64_t)gridDim.x * (blockDim.x >> 5), lanes);
   const int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int64_t lane = threadIdx.x & 31;
@@ -445,13 +449,17 @@ __global__ void __launch_bounds__(128) k_riemann_stragglers_ens(const RiemannEns
   }
 }
 
-void launch_riemann_ens(cudaStream_t s, const RiemannEnsArgs* a, int D, int64_t* off, double* scratch, int path_cap,
-                        int blocks, int eval_limit, int64_t* strag, unsigned long long* strag_count, int sblocks,
-                        size_t reserve_smem, int lanes) {
+void launch_riemann_ens_first(cudaStream_t s, const RiemannEnsArgs* a, int D, int64_t* off, double* scratch,
+                              int path_cap, int blocks, int eval_limit, int64_t* strag,
+                              unsigned long long* strag_count) {
   k_ens_iface_prefix<<<1, 1, 0, s>>>(a, D, off, strag_count);
   k_riemann_interfaces_ens<<<blocks, 128, 0, s>>>(a, D, off, scratch, path_cap, eval_limit, strag, strag_count);
+}
+void launch_riemann_ens_stragglers(cudaStream_t s, const RiemannEnsArgs* a, double* scratch, int path_cap,
+                                   const int64_t* strag, const unsigned long long* strag_count, int sblocks,
+                                   size_t reserve_smem, int lanes, int* stalled) {
   k_riemann_stragglers_ens<<<sblocks, 128, reserve_smem, s>>>(a, scratch, path_cap, reserve_smem, strag, strag_count,
-                                                              lanes);
+                                                              lanes, stalled);
 }
 cudaError_t riemann_stragglers_ens_reserve(size_t bytes) {
   return cudaFuncSetAttribute(k_riemann_stragglers_ens, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -573,9 +581,9 @@ void launch_riemann_stragglers(cudaStream_t s, const Params& P, const Mats* md, 
                                double* const* fs, const IfaceList& L, int store, double* scratch, int path_cap,
                                int blocks, size_t reserve_smem, const int32_t* strag,
                                const unsigned long long* strag_count, const float* warm, unsigned long long* cnt,
-                               const DevScalars* sc, int lanes) {
+                               const DevScalars* sc, int lanes, int* stalled) {
   k_riemann_stragglers<<<blocks, 128, reserve_smem, s>>>(P, md, S, id, fs, L, store, scratch, path_cap, reserve_smem,
-                                                         strag, strag_count, warm, cnt, sc, lanes);
+                                                         strag, strag_count, warm, cnt, sc, lanes, stalled);
 }
 // One block that holds one SM for a fixed number of clock cycles (bounded
 // loop, waits on nothing).  Launched on the main stream between the first
