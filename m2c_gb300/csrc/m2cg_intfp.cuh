@@ -87,8 +87,8 @@ M2CG_INT uint64_t if_recip(uint64_t D) {
   return ((uint64_t)r24 << 39) + (uint64_t)(c >> 12);
 }
 
-// 2^63 / sqrt(m) for M = m 2^62, m in [1, 4): at most the true value (to 1/8
-// unit), at least it - 8.
+// 2^63 / sqrt(m) for M = m 2^62, m in [1, 4): at most the true value, at least
+// it - 10.
 M2CG_INT uint64_t if_rsqrt(uint64_t M) {
   // binary32 argument just above m, exponent 127 or 128
   const uint32_t Mh = (uint32_t)(M >> 32);
@@ -100,7 +100,7 @@ M2CG_INT uint64_t if_rsqrt(uint64_t M) {
   const uint32_t r24 = (rb & 0x7fffffu) | 0x800000u;
   const uint64_t S = ((uint64_t)r24 * r24) << 16;            // y^2 2^64
   const uint64_t P = if_mulhi64(M, S);                       // m y^2 2^62, cut
-  int64_t es = (int64_t)(0x3ffffffffffffffcull - P) << 20;   // (e / 2) 2^83
+  int64_t es = (int64_t)(0x3ffffffffffffffaull - P) << 20;   // (e / 2) 2^83
   const int32_t eh = (int32_t)(es >> 32);                    // e 2^50
   es += ((int64_t)eh * (eh * 3)) >> 20;                      // + 3 e^2 / 8
   const int64_t c = (int64_t)(int32_t)r24 * (int32_t)(es >> 32) + if_mulhi(r24, (uint32_t)es);
@@ -166,21 +166,31 @@ M2CG_INT_SLOW double ddiv(double a, double b) {
   const uint64_t D = if_sig(if_hi(b), if_lo(b));
   return if_div_core(a, b, D, if_recip(D));
 }
-// ddiv for a chain that waits for each result (few active lanes): where the
-// estimate's error bound cannot reach the next 54-bit quotient, the remainder
-// is skipped (97 % of the quotients).
-M2CG_INT_SLOW double ddiv_lat(double a, double b) {
-  if (!if_div_range(a, b)) return a / b;
-  const uint32_t ah = if_hi(a), al = if_lo(a), bh = if_hi(b);
-  const uint64_t D = if_sig(bh, if_lo(b));
-  const uint64_t T = if_mulhi64(if_sig(ah, al), if_recip(D));
-  const uint32_t s = ((uint32_t)(T >> 62) ^ 1u) & 1u;
-  uint64_t Q = T >> (9u - s);
-  if ((((uint32_t)T + 8u) & (0x1ffu >> s)) < 8u)   // the floor of T + 8 may be one more
-    Q += ((uint64_t)(al << (21u + s)) << 32) - Q * (D >> 11) >= (D >> 11) ? 1u : 0u;
-  return if_pack(((ah ^ bh) & 0x80000000u) + ((((ah >> 20) & 0x7ffu) - ((bh >> 20) & 0x7ffu) + 1022u - s) << 20),
-                 (Q + 1u) >> 1);
+// The same for a chain that waits for each result (one problem per warp): the
+// estimate is rounded at once, and the exact remainder is formed only where the
+// estimate's error bound reaches the rounding boundary (8 of 512 or 1024
+// values); 250 cycles of latency against 385.  D and R as in if_div_core, so
+// that a divisor's reciprocal can be started before the dividend is known.
+M2CG_INT_SLOW double if_div_edge(double a, double b, uint64_t D, uint64_t R) {
+  return if_div_range(a, b) ? if_div_core(a, b, D, R) : a / b;
 }
+M2CG_INT double if_div_lat(double a, double b, uint64_t D, uint64_t R) {
+  const uint32_t ah = if_hi(a), bh = if_hi(b);
+  const uint64_t T = if_mulhi64(if_sig(ah, if_lo(a)), R);     // in (a / d 2^62 - 8, a / d 2^62]
+  const bool one = (uint32_t)(T >> 32) >= 0x40000000u;        // a / d >= 1
+  const uint64_t X0 = T + 512u, X1 = T + 256u;
+  const uint64_t m = one ? X0 >> 10 : X1 >> 9;
+  const bool edge = one ? (((uint32_t)X0 + 8u) & 1023u) < 8u : (((uint32_t)X1 + 8u) & 511u) < 8u;
+  const uint32_t ex = ((ah >> 20) & 0x7ffu) - ((bh >> 20) & 0x7ffu);
+  double r = if_pack(((ah ^ bh) & 0x80000000u) + ((ex + (one ? 1022u : 1021u)) << 20), m);
+  if (edge || !if_div_range(a, b)) r = if_div_edge(a, b, D, R);
+  return r;
+}
+M2CG_INT double if_div_lat(double a, double b) {
+  const uint64_t D = if_sig(if_hi(b), if_lo(b));
+  return if_div_lat(a, b, D, if_recip(D));
+}
+M2CG_INT_SLOW double ddiv_lat(double a, double b) { return if_div_lat(a, b); }
 M2CG_INT void ddiv2(double a, double b, double c, double d, double& q, double& r) {
   const bool ok = if_div_range(a, b) && if_div_range(c, d);
   const uint64_t D = if_sig(if_hi(b), if_lo(b)), E = if_sig(if_hi(d), if_lo(d));
@@ -203,6 +213,15 @@ M2CG_INT_SLOW double dsqrt(double x) {
   const uint64_t rem = ((uint64_t)(lo << (23u - even)) << 32) - Q * Q;   // m 2^106 - Q^2 modulo 2^64
   const uint64_t m = (Q + 1u + (rem > 2u * Q ? 1u : 0u)) >> 1;
   return if_pack((1022u + (uint32_t)(((int32_t)E - 1023) >> 1)) << 20, m);
+}
+
+M2CG_INT double if_sqrt_lat(double x) {   // as if_div_lat
+  const uint32_t hi = if_hi(x), lo = if_lo(x), E = hi >> 20;
+  const uint64_t M = if_sig(hi, lo) >> (E & 1u);
+  const uint64_t X = if_mulhi64(M, if_rsqrt(M)) + 256u;       // T in (sqrt(m) 2^61 - 13, sqrt(m) 2^61]
+  double r = if_pack((1022u + (uint32_t)(((int32_t)E - 1023) >> 1)) << 20, X >> 9);
+  if ((((uint32_t)X + 13u) & 511u) < 13u || !if_rsqrt_range(hi)) r = dsqrt(x);
+  return r;
 }
 
 // ---- van Albada's limited slope ------------------------------------------------

@@ -195,21 +195,26 @@ struct ExactRiemannDevT {
     return false;
   }
 
-  // c^2 at (rho, p): eos_e then eos_c2, a Noble-Abel gas's independent
-  // quotients in separate lanes.
-  __device__ __noinline__ static double c2_coop(const DevMat& M, double rho, double p) {
+  // c^2 at (rho, p): eos_e then eos_c2.  The reciprocal of rho is formed beside
+  // the first quotient; a Noble-Abel gas's independent quotients take separate
+  // lanes.
+  M2CG_DEV static double c2_coop(const DevMat& M, double rho, double p) {
+    const uint64_t D = if_sig(if_hi(rho), if_lo(rho)), R = if_recip(D);
     if (M.type == M2CG_EOS_SG) {
       const double g = M.gam1 * rho;
-      const double e = ddiv_lat(p + M.gamPs, g);
-      return M.gam1 * e + ddiv_lat(g * e - M.gamPs, rho) * M.gam1;
+      const double e = if_div_lat(p + M.gamPs, g);
+      return M.gam1 * e + if_div_lat(g * e - M.gamPs, rho, D, R) * M.gam1;
     }
+    return c2_coop_general(M, rho, p, D, R);
+  }
+  __device__ __noinline__ static double c2_coop_general(const DevMat& M, double rho, double p, uint64_t D, uint64_t R) {
     if (M.type == M2CG_EOS_NASG) {
-      const double V = ddiv_lat(1.0, rho), vb = V - M.b;
+      const double V = if_div_lat(1.0, rho, D, R), vb = V - M.b;
       const double e1 = (M.invgam1 * (p + M.gamPs) * vb + M.q) - M.q;
       const int l = lane();
       const double n1 = M.gam1 * V * V * e1, d1 = vb * vb, d2 = 1.0 - M.b * rho, n0 = M.gam1 * e1;
-      const double q = ddiv_lat(l == 0 ? n0 : l == 1 ? n1 : M.gam1, l == 0 ? vb : l == 1 ? d1 : d2);
-      return bc(q, 1) + ddiv_lat(bc(q, 0) - M.gamPs, rho) * bc(q, 2);
+      const double q = if_div_lat(l == 0 ? n0 : l == 1 ? n1 : M.gam1, l == 0 ? vb : l == 1 ? d1 : d2);
+      return bc(q, 1) + if_div_lat(bc(q, 0) - M.gamPs, rho, D, R) * bc(q, 2);
     }
     return eos_c2(M, rho, eos_e(M, rho, p));
   }
@@ -231,13 +236,13 @@ struct ExactRiemannDevT {
     if (!memo_get(M, rho_0, p_0, c2, c0)) {
       c2 = c2_coop(M, rho_0, p_0);
       if (i_le0(rho_0) || i_lt0(c2)) return false;
-      memo_start = EosMemo{&M, rho_0, p_0, c2, dsqrt(c2)};
+      memo_start = EosMemo{&M, rho_0, p_0, c2, if_sqrt_lat(c2)};
     }
     double S = j < 5 ? rho_0 : 0.0, cq = c2, rq = rho_0;
     for (int k = 0; k < 6; k++) {
       const double a = rk45_a[k][j], ad = a * dp;
       const bool on = a != 0.0;
-      const double q = ddiv_lat(on ? (j < 5 ? ad : a) : 1.0, c2);
+      const double q = if_div_lat(on ? (j < 5 ? ad : a) : 1.0, c2);
       const double S1 = S + q;
       if (on) S = S1;
       if (k == 5) break;
@@ -247,7 +252,7 @@ struct ExactRiemannDevT {
       if (rk45_stage[j9] == k + 1) { cq = c2; rq = rk; }
     }
     const double D = S * dp;
-    const double w = ddiv_lat(ddiv_lat(rk45_u[j9], dsqrt(cq)), rq);
+    const double w = if_div_lat(if_div_lat(rk45_u[j9], if_sqrt_lat(cq)), rq);
     const int b = l == 0 ? 0 : 4;
     double T = bc(w, b) + bc(w, b + 1) + bc(w, b + 2) + bc(w, b + 3);
     const double T1 = T + bc(w, 8);
@@ -262,7 +267,7 @@ struct ExactRiemannDevT {
     u = (wave == 1) ? u_0 - du : u_0 + du;
     const double ce = c2_coop(M, rho, p);
     if (i_le0(rho) || i_lt0(ce)) return false;
-    const double c = dsqrt(ce);
+    const double c = if_sqrt_lat(ce);
     memo_end = EosMemo{&M, rho, p, ce, c};
     xi = (wave == 1) ? u - c : u + c;
     return true;
@@ -279,12 +284,12 @@ struct ExactRiemannDevT {
     if (!memo_get(M, rho_0, p_0, c2, c0)) {
       c2 = c2_coop(M, rho_0, p_0);
       if (i_le0(rho_0) || i_lt0(c2)) return false;
-      memo_start = EosMemo{&M, rho_0, p_0, c2, dsqrt(c2)};
+      memo_start = EosMemo{&M, rho_0, p_0, c2, if_sqrt_lat(c2)};
     }
     const double pm = p_0 + hdp, pe = p_0 + dp;
     double cq = c2, rq = rho_0, rr = 0.0;
     for (int k = 0; k < 4; k++) {
-      const double q = ddiv_lat((l == 0 && k < 3) ? (k < 2 ? hdp : dp) : 1.0, c2);
+      const double q = if_div_lat((l == 0 && k < 3) ? (k < 2 ? hdp : dp) : 1.0, c2);
       const double r1 = bc(q, 1);
       if (l == k) rr = r1;
       if (k == 3) break;
@@ -293,7 +298,7 @@ struct ExactRiemannDevT {
       if (i_le0(rk) || i_lt0(c2)) return false;
       if (l == k + 1) { cq = c2; rq = rk; }
     }
-    const double w = ddiv_lat(ddiv_lat(1.0, dsqrt(cq)), rq);
+    const double w = if_div_lat(if_div_lat(1.0, if_sqrt_lat(cq)), rq);
     // every lane takes part in every shuffle; lane 0 sums the density's terms, lane 1 the velocity's
     const double r0 = bc(rr, 0), r1 = bc(rr, 1), r2 = bc(rr, 2), r3 = bc(rr, 3);
     const double w0 = bc(w, 0), w1 = bc(w, 1), w2 = bc(w, 2), w3 = bc(w, 3);
@@ -306,7 +311,7 @@ struct ExactRiemannDevT {
     u = (wave == 1) ? u_0 - du : u_0 + du;
     const double ce = c2_coop(M, rho, p);
     if (i_le0(rho) || i_lt0(ce)) return false;
-    const double c = dsqrt(ce);
+    const double c = if_sqrt_lat(ce);
     memo_end = EosMemo{&M, rho, p, ce, c};
     xi = (wave == 1) ? u - c : u + c;
     return true;
@@ -512,12 +517,12 @@ struct ExactRiemannDevT {
     double es, oors;
     if (Coop && M.type == M2CG_EOS_SG) {
       const bool o = lane() & 1;
-      const double q = ddiv_lat(o ? 1.0 : ps + M.gamPs, o ? rhos : M.gam1 * rhos);
+      const double q = if_div_lat(o ? 1.0 : ps + M.gamPs, o ? rhos : M.gam1 * rhos);
       es = bc(q, 0);
       oors = bc(q, 1);
     } else if (M.type == M2CG_EOS_SG) ddiv2(ps + M.gamPs, M.gam1 * rhos, 1.0, rhos, es, oors);
     else if (M.type == M2CG_EOS_NASG) {   // 1 / rho serves both terms
-      oors = ddiv(1.0, rhos);
+      oors = Coop ? if_div_lat(1.0, rhos) : ddiv(1.0, rhos);
       es = M.invgam1 * (ps + M.gamPs) * (oors - M.b) + M.q;
     } else { es = eos_e(M, rhos, ps); oors = ddiv(1.0, rhos); }
     return es - e + pavg * (oors - one_over_rho);
@@ -685,7 +690,7 @@ struct ExactRiemannDevT {
         drho = rhos1 - rhos0;
         int it;
         for (it = 0; it < P.maxIts_shock; it++) {
-          rhos2 = rhos2 - (Coop ? ddiv_lat(f2 * drho, f1 - f0) : ddiv(f2 * drho, f1 - f0));
+          rhos2 = rhos2 - (Coop ? if_div_lat(f2 * drho, f1 - f0) : ddiv(f2 * drho, f1 - f0));
           if (i_le(rhos1, rhos2) || i_le(rhos2, rhos0)) rhos2 = rhos0 + 0.5 * drho;
           f2 = hugo(M, e, pavg, oor, ps, rhos2);
           if (i_eq0(f2)) { s_first = s_second = rhos2; break; }

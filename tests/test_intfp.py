@@ -80,10 +80,11 @@ int main() {
       div += !same(q, a / b) + !same(w, b / a);
       double x = fabs(a);
       if ((i & 7) == 5 && b == b) x = b * b;
-      root += !same(dsqrt(x), sqrt(x));
+      root += !same(dsqrt(x), sqrt(x)) + !same(if_sqrt_lat(x), sqrt(x));
       if (if_rcp_range(if_hi(b)) && fabs(b) < 1e300) { double d = ulps(if_rcp_core(if_hi(b), if_lo(b)), 1.0L / b); er = d > er ? d : er; }
       if (if_rsqrt_range(if_hi(x))) { double d = ulps(if_rsqrt_core(if_hi(x), if_lo(x)), 1.0L / sqrtl(x)); es = d > es ? d : es; }
       double p = mk(r1, 960 + (r3 >> 20) % 100), t = mk(r2, 960 + (r3 >> 40) % 100), o;
+      if ((i & 63) == 1) t = copysign(1e-16 / fabs(p), p) * (1 + 0x1p-52 * ((int)(r3 >> 56) - 128));
       if (i & 2) t = copysign(p, t) * (1 + 1e-3 * ((r3 >> 50) & 7));
       if (if_van_albada(p, t, o)) {
         const bool zero = p * t <= 0 || fabs(p * t) < 1e-16;
