@@ -129,7 +129,7 @@ struct m2cg_ctx {
   // it) on stream2, which has the highest priority so that the straggler
   // blocks are placed on empty SMs before the reconstruction kernel's.
   int eval_limit = 24;
-  int sblocks = 0;             // straggler blocks of 128 threads (one SM each; idle ones exit at once)
+  int sblocks = 0;             // straggler blocks of 256 threads (one SM each; idle ones exit at once)
   int strag_lanes = 1;         // straggler faces packed per warp (1: one face per warp)
   size_t sreserve = 0;         // their dynamic shared-memory request
   int32_t* strag = nullptr;
@@ -323,13 +323,13 @@ static m2cg_status ctx_alloc(m2cg_ctx* x) {
   CK(x->alloc(&x->strag, L.cap));
   CK(x->alloc(&x->strag_count, 1));
   CK(x->alloc(&x->stalled, 3));
-  x->sblocks = std::max(1, std::min(x->nsm, x->rblocks));
+  x->sblocks = std::max(1, std::min(x->nsm, x->rblocks / 2));   // 256-thread blocks on the first pass's scratch
   // tuning overrides: M2CG_RIEMANN_EVAL_LIMIT (first-pass budget, 0 = none),
   // M2CG_RIEMANN_STRAGGLER_SMS (blocks of the second pass, one SM each),
   // M2CG_RIEMANN_HOLD_CYCLES (head start of the second pass, SM clock cycles) and
   // M2CG_RIEMANN_STRAGGLER_LANES (second-pass faces per warp, 1..32)
   if (const char* e = getenv("M2CG_RIEMANN_EVAL_LIMIT")) x->eval_limit = std::max(0, atoi(e));
-  if (const char* e = getenv("M2CG_RIEMANN_STRAGGLER_SMS")) x->sblocks = std::min(x->rblocks, std::max(1, atoi(e)));
+  if (const char* e = getenv("M2CG_RIEMANN_STRAGGLER_SMS")) x->sblocks = std::min(x->rblocks / 2, std::max(1, atoi(e)));
   if (const char* e = getenv("M2CG_RIEMANN_HOLD_CYCLES")) x->hold_cycles = std::max(0ll, atoll(e));
   if (const char* e = getenv("M2CG_RIEMANN_STRAGGLER_LANES")) x->strag_lanes = std::min(32, std::max(1, atoi(e)));
   {

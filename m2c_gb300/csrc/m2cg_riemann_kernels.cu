@@ -245,33 +245,49 @@ __global__ void k_riemann_interfaces(Params P, const Mats* __restrict__ md, Stat
   iface_counts(cnt, acc);
 }
 
-// Warps the second pass spreads its n faces over: all W launched warps (one
-// face per warp) when lanes <= 1, else just enough warps to hold `lanes` faces
-// each.  Lanes of a warp that follow different faces take turns only where
-// their control flow differs; the stalled solves that reach this pass mostly
-// run the same secant loop, so packing several into one warp costs little
-// latency and frees the SMs the pass would otherwise hold.  Face k runs on
-// warp k mod W, lane k / W (k / W < 32 for every k < n).
-__device__ __forceinline__ int64_t straggler_warps(int64_t n, int64_t W, int lanes) {
-  if (lanes <= 1 || n <= 0) return W;
-  int64_t need = (n + lanes - 1) / lanes;
-  int64_t floor32 = (n + 31) / 32;   // never fewer warps than 32 lanes can hold
-  need = need < floor32 ? floor32 : need;
-  return need < W ? need : W;
+// Layout of the second pass: which warps of a 256-thread block work, the warp's
+// index w among the W working ones, and whether it keeps its path caches in the
+// reserved shared memory.  Half of the block's warps (one per sub-partition)
+// while these are enough, all of them beyond that; with lanes > 1 just enough
+// warps to hold `lanes` faces each.  Face k runs on warp k mod W, and there on
+// lane k / W where there are more faces than warps.
+struct StragglerWarps {
+  int64_t W, w;
+  bool works, shared;
+};
+__device__ __forceinline__ StragglerWarps straggler_warps(int64_t n, int lanes, size_t per_warp, size_t reserve_bytes) {
+  const int warp = (int)(threadIdx.x >> 5), all = (int)(blockDim.x >> 5), half = all / 2;
+  const int use = n <= (int64_t)gridDim.x * half ? half : all;
+  StragglerWarps r;
+  r.W = (int64_t)gridDim.x * use;
+  r.w = (int64_t)blockIdx.x * use + warp;
+  if (lanes > 1 && n > 0) {
+    int64_t need = (n + lanes - 1) / lanes;
+    const int64_t floor32 = (n + 31) / 32;   // never fewer warps than 32 lanes can hold
+    need = need < floor32 ? floor32 : need;
+    r.W = need < r.W ? need : r.W;
+  }
+  r.works = warp < use && r.w < r.W;
+  r.shared = warp < half && (size_t)half * per_warp * sizeof(double) <= reserve_bytes;
+  return r;
 }
 
 // Second pass: the listed faces solved without a budget.  Each is one long
-// chain of dependent binary64 operations, so the faces are dealt round-robin
-// over the warps (lane-major), which puts as few as possible in one warp: lanes
-// of a warp that follow different faces diverge and take turns.  The launch
-// asks for (and never touches) nearly all of an SM's shared memory, so no block
-// of another kernel shares an SM -- and its FP64 unit -- with these chains while
-// the reconstruction and face-flux kernels run concurrently on the other SMs.
-// That request also takes most of the SM's L1, so lane 0 of each warp -- the
-// one lane in use while there are no more faces than warps -- keeps its
-// integration-path caches in the reserved shared memory instead of going
-// through L1 to the global scratch.
-__global__ void __launch_bounds__(128) k_riemann_stragglers(Params P, const Mats* __restrict__ md, StateSet S,
+// chain of dependent operations, dealt over the warps: one face per warp while
+// there are no more faces than warps (its lanes solve it together), else
+// lane-major, which puts as few as possible in one warp: lanes that follow
+// different faces diverge and take turns.  A block of 256 threads at 255
+// registers takes an SM's whole register file, so that no block of another
+// kernel shares the SM -- and its FP64 units -- with these chains while
+// reconstruction and fluxes run on the other SMs.  The shared memory it asks
+// for holds the path caches of half its warps (of a warp's first lane when
+// there are several faces per warp); the rest go through L1 to the scratch.
+// Eight warps an SM instead of four, and none of the path caches shared by the
+// upper four, cost a chain little (it waits for latencies) and halve the rounds
+// where more than 608 faces stall: five steps of the bubble cluster (1,100 to
+// 1,600 stalled faces) 241, 222, 272, 350 ms for four sets of states against
+// 286, 251, 283, 380.
+__global__ void __launch_bounds__(256) k_riemann_stragglers(Params P, const Mats* __restrict__ md, StateSet S,
                                                             const int32_t* __restrict__ id, double* const* fs,
                                                             IfaceList L, int store, double* scratch, int path_cap,
                                                             size_t reserve_bytes, const int32_t* __restrict__ strag,
@@ -282,35 +298,26 @@ __global__ void __launch_bounds__(128) k_riemann_stragglers(Params P, const Mats
   if (sc && !sc->active) return;
   int64_t n = (int64_t)min((unsigned long long)L.cap, *strag_count);
   if (stalled && blockIdx.x == 0 && threadIdx.x == 0) *stalled = n > 0;   // the next stage's Gate
-  const int64_t W = straggler_warps(n, (int64_t)gridDim.x * (blockDim.x >> 5), lanes);
-  const int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const size_t per_warp = (size_t)6 * path_cap;  // doubles: two waves x cap entries x {p, rho, u}
+  const StragglerWarps sw = straggler_warps(n, lanes, per_warp, reserve_bytes);
+  if (!sw.works) return;
   const int64_t lane = threadIdx.x & 31;
   int64_t T = (int64_t)gridDim.x * blockDim.x;
   int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t per_warp = (size_t)6 * path_cap;  // doubles: two waves x cap entries x {p, rho, u}
-  if (lanes <= 1 && coop_pass(n)) {   // one face per warp: its lanes solve it together
-    if (w >= n) return;
+  unsigned long long acc[6] = {0, 0, 0, 0, 0, 0};
+  if (lanes <= 1 && n <= sw.W) {   // one face per warp: its lanes solve it together
+    if (sw.w >= n) return;
     ExactRiemannCoop rc;
-    if ((size_t)(blockDim.x >> 5) * per_warp * sizeof(double) <= reserve_bytes)
-      init_coop(rc, md, P.rp, s_path, path_cap, threadIdx.x >> 5);
-    else
-      init_coop(rc, md, P.rp, scratch, path_cap, w);
-    unsigned long long acc[6] = {0, 0, 0, 0, 0, 0};
-    iface_solve(P, S, id, fs, L, store, warm, strag[w], rc, acc);
+    if (sw.shared) init_coop(rc, md, P.rp, s_path, path_cap, threadIdx.x >> 5);
+    else init_coop(rc, md, P.rp, scratch, path_cap, sw.w);
+    iface_solve(P, S, id, fs, L, store, warm, strag[sw.w], rc, acc);
     if (lane == 0) iface_counts(cnt, acc);
     return;
   }
   ExactRiemannDev rs;
   init_solver(rs, md, P.rp, scratch, path_cap, tid, T);
-  if (lane == 0 && (size_t)(blockDim.x >> 5) * per_warp * sizeof(double) <= reserve_bytes) {
-    rs.path1.base = s_path + (threadIdx.x >> 5) * per_warp;
-    rs.path1.stride = 1;
-    rs.path3.base = rs.path1.base + (size_t)3 * path_cap;
-    rs.path3.stride = 1;
-  }
-  unsigned long long acc[6] = {0, 0, 0, 0, 0, 0};
-  if (w < W)
-    for (int64_t k = lane * W + w; k < n; k += 32 * W) iface_solve(P, S, id, fs, L, store, warm, strag[k], rs, acc);
+  if (lane == 0 && sw.shared) init_solver(rs, md, P.rp, s_path + (threadIdx.x >> 5) * per_warp, path_cap, 0, 1);
+  for (int64_t k = lane * sw.W + sw.w; k < n; k += 32 * sw.W) iface_solve(P, S, id, fs, L, store, warm, strag[k], rs, acc);
   iface_counts(cnt, acc);
 }
 
@@ -398,7 +405,7 @@ __global__ void k_riemann_interfaces_ens(const RiemannEnsArgs* __restrict__ a, i
 // The listed faces of all members, dealt lane-major over the warps as in
 // k_riemann_stragglers (one face per warp while there are no more faces than
 // warps).
-__global__ void __launch_bounds__(128) k_riemann_stragglers_ens(const RiemannEnsArgs* __restrict__ a, double* scratch,
+__global__ void __launch_bounds__(256) k_riemann_stragglers_ens(const RiemannEnsArgs* __restrict__ a, double* scratch,
                                                                 int path_cap, size_t reserve_bytes,
                                                                 const int64_t* __restrict__ strag,
                                                                 const unsigned long long* strag_count, int lanes,
@@ -406,38 +413,28 @@ __global__ void __launch_bounds__(128) k_riemann_stragglers_ens(const RiemannEns
   extern __shared__ __align__(16) double s_path[];
   const int64_t n = (int64_t)*strag_count;
   if (blockIdx.x == 0 && threadIdx.x == 0) *stalled = n > 0;   // the next stage's Gate
-  const int64_t W = straggler_warps(n, (int64_t)gridDim.x * (blockDim.x >> 5), lanes);
-  const int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const size_t per_warp = (size_t)6 * path_cap;
+  const StragglerWarps sw = straggler_warps(n, lanes, per_warp, reserve_bytes);
+  if (!sw.works) return;
   const int64_t lane = threadIdx.x & 31;
   int64_t T = (int64_t)gridDim.x * blockDim.x;
   int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t per_warp = (size_t)6 * path_cap;
-  if (lanes <= 1 && coop_pass(n)) {
-    if (w >= n) return;
-    ExactRiemannCoop rc;
-    if ((size_t)(blockDim.x >> 5) * per_warp * sizeof(double) <= reserve_bytes)
-      init_coop(rc, a[0].md, a[0].P.rp, s_path, path_cap, threadIdx.x >> 5);
-    else
-      init_coop(rc, a[0].md, a[0].P.rp, scratch, path_cap, w);
-    unsigned long long acc[6] = {0, 0, 0, 0, 0, 0};
-    const int64_t v = strag[w];
+  unsigned long long acc[6] = {0, 0, 0, 0, 0, 0};
+  if (lanes <= 1 && n <= sw.W) {
+    if (sw.w >= n) return;
+    const int64_t v = strag[sw.w];
     const RiemannEnsArgs& e = a[(int)(v >> 40)];
-    rc.mats = e.md;
-    rc.P = e.P.rp;
+    ExactRiemannCoop rc;
+    if (sw.shared) init_coop(rc, e.md, e.P.rp, s_path, path_cap, threadIdx.x >> 5);
+    else init_coop(rc, e.md, e.P.rp, scratch, path_cap, sw.w);
     iface_solve(e.P, e.S, e.id, e.fs, e.L, e.store, e.warm, v & ((1ll << 40) - 1), rc, acc);
     if (lane == 0) iface_counts(e.cnt, acc);
     return;
   }
   ExactRiemannDev rs;
   init_solver(rs, a[0].md, a[0].P.rp, scratch, path_cap, tid, T);
-  if (lane == 0 && (size_t)(blockDim.x >> 5) * per_warp * sizeof(double) <= reserve_bytes) {
-    rs.path1.base = s_path + (threadIdx.x >> 5) * per_warp;
-    rs.path1.stride = 1;
-    rs.path3.base = rs.path1.base + (size_t)3 * path_cap;
-    rs.path3.stride = 1;
-  }
-  unsigned long long acc[6] = {0, 0, 0, 0, 0, 0};
-  for (int64_t k = lane * W + w; w < W && k < n; k += 32 * W) {
+  if (lane == 0 && sw.shared) init_solver(rs, a[0].md, a[0].P.rp, s_path + (threadIdx.x >> 5) * per_warp, path_cap, 0, 1);
+  for (int64_t k = lane * sw.W + sw.w; k < n; k += 32 * sw.W) {
     int64_t v = strag[k];
     int d = (int)(v >> 40);
     int64_t s = v & ((1ll << 40) - 1);
@@ -458,14 +455,17 @@ void launch_riemann_ens_first(cudaStream_t s, const RiemannEnsArgs* a, int D, in
 void launch_riemann_ens_stragglers(cudaStream_t s, const RiemannEnsArgs* a, double* scratch, int path_cap,
                                    const int64_t* strag, const unsigned long long* strag_count, int sblocks,
                                    size_t reserve_smem, int lanes, int* stalled) {
-  k_riemann_stragglers_ens<<<sblocks, 128, reserve_smem, s>>>(a, scratch, path_cap, reserve_smem, strag, strag_count,
+  k_riemann_stragglers_ens<<<sblocks, 256, reserve_smem, s>>>(a, scratch, path_cap, reserve_smem, strag, strag_count,
                                                               lanes, stalled);
 }
 cudaError_t riemann_stragglers_ens_reserve(size_t bytes) {
   return cudaFuncSetAttribute(k_riemann_stragglers_ens, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-// Batched independent problems (device arrays, AoS rows of 5 / 3).
+// Batched independent problems (device arrays, AoS rows of 5 / 3): one per
+// warp or one per thread (coop_pass; two kernels, since one that held both
+// solvers spilt 3.4 kB a thread and took 9.8 ms instead of 9.3 for 20,000 problems).
+template <bool Coop>
 __global__ void k_riemann_batch(const Mats* __restrict__ md, RiemannPrm rp, int64_t n, const double* __restrict__ Vm,
                                 const int32_t* __restrict__ idm, const double* __restrict__ Vp,
                                 const int32_t* __restrict__ idp, const double* __restrict__ dir, double* Vs,
@@ -473,22 +473,11 @@ __global__ void k_riemann_batch(const Mats* __restrict__ md, RiemannPrm rp, int6
                                 int path_cap, const double* warm) {
   int64_t T = (int64_t)gridDim.x * blockDim.x;
   int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (coop_pass(n)) {   // one warp per problem
-    const int64_t q = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-    if (q >= n) return;
-    ExactRiemannCoop rc;
-    init_coop(rc, md, rp, scratch, path_cap, q);
-    int oid = 0;
-    rc.warm_p = warm ? warm[q] : 0.0;
-    const int e = rc.solve(&dir[q * 3], &Vm[q * 5], idm[q], &Vp[q * 5], idp[q], &Vs[q * 5], oid, &Vsm[q * 5], &Vsp[q * 5]);
-    id[q] = oid;
-    if (iters) iters[q] = rc.evals;
-    if (err) err[q] = e;
-    return;
-  }
-  ExactRiemannDev rs;
-  init_solver(rs, md, rp, scratch, path_cap, tid, T);
-  for (int64_t q = tid; q < n; q += T) {
+  ExactRiemannDevT<Coop> rs;
+  const int64_t w = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;   // < T / 32
+  if constexpr (Coop) init_coop(rs, md, rp, scratch, path_cap, w);
+  else init_solver(rs, md, rp, scratch, path_cap, tid, T);
+  for (int64_t q = Coop ? w : tid; q < n; q += T) {
     int oid = 0;
     rs.warm_p = warm ? warm[q] : 0.0;
     int e = rs.solve(&dir[q * 3], &Vm[q * 5], idm[q], &Vp[q * 5], idp[q], &Vs[q * 5], oid, &Vsm[q * 5], &Vsp[q * 5]);
@@ -538,7 +527,8 @@ __device__ __forceinline__ void riemann_eos_problem(Solver& rs, Mats& mats, int6
 // Independent 1D problems, each with its own material pair (the warm-start
 // training and evaluation sets): W rows {rho_l, u_l, p_l, rho_r, u_r, p_r},
 // E rows {type, gamma, pc, b, q} left then right; out rows {p*, u*, rho*_l,
-// rho*_r}.  One thread per problem, grid-stride.
+// rho*_r}.  One warp or one thread per problem, as k_riemann_batch.
+template <bool Coop>
 __global__ void k_riemann_batch_eos(RiemannPrm rp, int64_t n, const double* __restrict__ W,
                                     const double* __restrict__ E, const double* __restrict__ warm, double* out,
                                     int32_t* iters, int32_t* err, double* scratch, int path_cap) {
@@ -546,17 +536,11 @@ __global__ void k_riemann_batch_eos(RiemannPrm rp, int64_t n, const double* __re
   int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   Mats mats;
   const double dir[3] = {1.0, 0.0, 0.0};
-  if (coop_pass(n)) {   // one warp per problem
-    const int64_t q = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-    if (q >= n) return;
-    ExactRiemannCoop rc;
-    init_coop(rc, &mats, rp, scratch, path_cap, q);
-    riemann_eos_problem(rc, mats, q, W, E, warm, dir, out, iters, err);
-    return;
-  }
-  ExactRiemannDev rs;
-  init_solver(rs, &mats, rp, scratch, path_cap, tid, T);
-  for (int64_t q = tid; q < n; q += T) riemann_eos_problem(rs, mats, q, W, E, warm, dir, out, iters, err);
+  ExactRiemannDevT<Coop> rs;
+  const int64_t w = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;   // < T / 32
+  if constexpr (Coop) init_coop(rs, &mats, rp, scratch, path_cap, w);
+  else init_solver(rs, &mats, rp, scratch, path_cap, tid, T);
+  for (int64_t q = Coop ? w : tid; q < n; q += T) riemann_eos_problem(rs, mats, q, W, E, warm, dir, out, iters, err);
 }
 
 __global__ void k_flux_batch(Params P, int64_t n, const int32_t* __restrict__ dir, const double* __restrict__ Vm,
@@ -575,14 +559,14 @@ void launch_riemann_interfaces(cudaStream_t s, const Params& P, const Mats* md, 
   k_riemann_interfaces<<<blocks, threads, 0, s>>>(P, md, S, id, fs, L, store, scratch, path_cap, eval_limit, strag,
                                                   strag_count, warm, cnt, sc);
 }
-// blocks * 128 threads must not exceed the first pass's thread count (the
+// blocks * 256 threads must not exceed the first pass's thread count (the
 // path-cache scratch is shared); reserve_smem: dynamic shared memory per block.
 void launch_riemann_stragglers(cudaStream_t s, const Params& P, const Mats* md, const StateSet& S, const int32_t* id,
                                double* const* fs, const IfaceList& L, int store, double* scratch, int path_cap,
                                int blocks, size_t reserve_smem, const int32_t* strag,
                                const unsigned long long* strag_count, const float* warm, unsigned long long* cnt,
                                const DevScalars* sc, int lanes, int* stalled) {
-  k_riemann_stragglers<<<blocks, 128, reserve_smem, s>>>(P, md, S, id, fs, L, store, scratch, path_cap, reserve_smem,
+  k_riemann_stragglers<<<blocks, 256, reserve_smem, s>>>(P, md, S, id, fs, L, store, scratch, path_cap, reserve_smem,
                                                          strag, strag_count, warm, cnt, sc, lanes, stalled);
 }
 // One block that holds one SM for a fixed number of clock cycles (bounded
@@ -606,13 +590,15 @@ void launch_riemann_batch(cudaStream_t s, const Params& P, const Mats* md, int64
                           const double* Vp, const int32_t* idp, const double* dir, double* Vs, int32_t* id,
                           double* Vsm, double* Vsp, int32_t* iters, int32_t* err, double* scratch, int path_cap,
                           int blocks, int threads, const double* warm) {
-  k_riemann_batch<<<blocks, threads, 0, s>>>(md, P.rp, n, Vm, idm, Vp, idp, dir, Vs, id, Vsm, Vsp, iters, err,
+  const auto k = n <= (int64_t)blocks * (threads / 32) ? k_riemann_batch<true> : k_riemann_batch<false>;
+  k<<<blocks, threads, 0, s>>>(md, P.rp, n, Vm, idm, Vp, idp, dir, Vs, id, Vsm, Vsp, iters, err,
                                              scratch, path_cap, warm);
 }
 void launch_riemann_batch_eos(cudaStream_t s, const Params& P, int64_t n, const double* W, const double* E,
                               const double* warm, double* out, int32_t* iters, int32_t* err, double* scratch,
                               int path_cap, int blocks, int threads) {
-  k_riemann_batch_eos<<<blocks, threads, 0, s>>>(P.rp, n, W, E, warm, out, iters, err, scratch, path_cap);
+  const auto k = n <= (int64_t)blocks * (threads / 32) ? k_riemann_batch_eos<true> : k_riemann_batch_eos<false>;
+  k<<<blocks, threads, 0, s>>>(P.rp, n, W, E, warm, out, iters, err, scratch, path_cap);
 }
 void launch_flux_batch(cudaStream_t s, const Params& P, int64_t n, const int32_t* dir, const double* Vm,
                        const double* Vp, const int32_t* id, double* F) {
