@@ -9,10 +9,22 @@
 // operands staged in shared memory and FP32 accumulators in tensor memory, one
 // 128-row tile per CTA pass.  The scalar head (64 -> 1), biases, SiLU, the
 // loss and Adam run on the CUDA cores in FP32.  Training runs forward and
-// backward for a tile in one kernel, keeping the three pre-activations in
-// TMEM for the backward pass, and accumulates the weight gradients with FP32
-// atomics; Adam then updates the FP32 master weights and k_pack_bf16 writes
-// the BF16 copies the GEMMs read.
+// backward for a tile in one kernel and accumulates the weight gradients with
+// FP32 atomics; Adam then updates the FP32 master weights and the BF16 copies
+// the GEMMs read.
+//
+// A tile is a short serial chain (three GEMMs of 2 x 128 x 64 x 64 operations
+// and their epilogues, eight in training), so the time is latency: of the
+// shared-memory traffic around the GEMMs, the activations and the barriers.
+// 16 warps share a tile, each thread holding one row's 16 columns: one 64-byte
+// TMEM load per layer, two 16-byte stores into the operand tile, which the
+// next GEMM reads K-major and the weight-gradient GEMM, transposed by its
+// descriptor, M-major from the same bytes.  SiLU' is kept in registers from
+// the forward pass, column sums are taken while the GEMMs run.  (With one row
+// per thread, element-wise stores, transposed copies and 320 shuffles per row
+// for the column sums, 32 training batches of 16,384 rows took 4.2 ms, 3.0 of
+// them in this kernel, and a forward pass over 262,144 rows 216 us; now 1.8 ms,
+// most of it the host's permutation of the rows, and 61 us.)
 //
 // Inputs are dimensionless groups of the two states relative to the
 // impedance-weighted pressure p_ref = (C_r p_l + C_l p_r) / (C_l + C_r), with
@@ -56,58 +68,101 @@ constexpr int OFF_W1 = 0, OFF_B1 = OFF_W1 + NH * NF, OFF_W2 = OFF_B1 + NH, OFF_B
               NPARAM = OFF_B4 + 1;
 static_assert(NPARAM == M2CG_MLP_PARAMS, "parameter count");
 // BF16 GEMM operands: W1f [64][16], W2f, W3f [64][64] (out x in, the forward
-// B operands) and W2b, W3b [64][64] (in x out, the backward B operands)
+// B operands) and W2b, W3b [64][64] (in x out, the backward B operands), each
+// in the operand layout of shared memory, so that a CTA's copy is one run of
+// 16-byte words
 constexpr int BF_W1F = 0, BF_W2F = BF_W1F + NH * NF, BF_W3F = BF_W2F + NH * NH, BF_W2B = BF_W3F + NH * NH,
               BF_W3B = BF_W2B + NH * NH, NBF = BF_W3B + NH * NH;
 
 constexpr long long MAX_POLLS = 1ll << 26;  // mbarrier wait limit (the MMAs take microseconds)
 
-// shared-memory layout of the tile kernels (byte offsets, 1024-aligned)
-constexpr int S_W1F = 0, S_W2F = S_W1F + 2048, S_W3F = S_W2F + 8192, S_W2B = S_W3F + 8192, S_W3B = S_W2B + 8192,
-              S_XA = S_W3B + 8192, S_H1A = S_XA + 4096, S_H2A = S_H1A + 16384, S_HT = S_H2A + 16384,
-              S_DZA = S_HT + 32768, S_DZT = S_DZA + 16384, S_F32 = S_DZT + 16384,
-              // fp32: b1 b2 b3 w4 (4 x 64), reductions db1 db2 db3 dw4 (4 x 64), b4, loss, db4
-              S_END = S_F32 + (8 * 64 + 4) * 4;
-constexpr int SMEM_FWD = S_H2A + 16384 + (8 * 64 + 4) * 4;  // forward: weights, Xa, H1a, H2a (+ floats)
-constexpr int SMEM_TRAIN = S_END;
+// Threads of a tile: row r = thread % 128 (the TMEM lane its warp can reach),
+// columns 16 (thread / 128) .. + 15.
+constexpr int NTHR = 512;
+constexpr int CG = 16;         // columns per thread
+constexpr int NGRP = NH / CG;  // column groups
+static_assert(NTHR == TILE * NGRP, "one thread per row and column group");
 
-__device__ __forceinline__ float silu(float z) { return z / (1.0f + expf(-z)); }
-__device__ __forceinline__ float dsilu(float z) {
-  float s = 1.0f / (1.0f + expf(-z));
-  return s * (1.0f + z * (1.0f - s));
+// shared-memory layout of the tile kernels (byte offsets, 1024-aligned): the
+// weights as in global memory, the operand tiles, then floats.  As the M-major
+// operand of a weight-gradient GEMM a tile is read as 128 features, of which
+// it has 64 (or 16): the rest, up to 1,792 bytes behind its end, only reach
+// accumulator rows that nobody reads.
+constexpr int S_W = 0, S_XA = S_W + 2 * NBF, S_H1A = S_XA + 4096, S_H2A = S_H1A + 16384,
+              S_FWD_END = S_H2A + 16384, S_DZ3 = S_FWD_END, S_DZ2 = S_DZ3 + 16384, S_DZ1 = S_DZ2 + 16384,
+              S_TRAIN_END = S_DZ1 + 16384;
+static_assert(S_XA % 1024 == 0, "tile alignment");
+// the last hidden layer's activations [64][128] in FP32 for the head: where the
+// operand tiles are free at that time
+constexpr int S_H3_FWD = S_H1A, S_H3_TRAIN = S_DZ2;
+// floats behind them: b1 b2 b3 w4 (4 x 64), b4, padding; in training the rows'
+// outputs, the column sums of the four warps of each column: db1 db2 db3 dw4,
+// then loss and db4 of the warps of group 0
+constexpr int F_B4 = 256, F_OUT = 260, F_SUM = F_OUT + TILE, F_LOSS = F_SUM + 4 * 4 * NH, F_END = F_LOSS + 8;
+constexpr int SMEM_FWD = S_FWD_END + F_OUT * 4;
+constexpr int SMEM_TRAIN = S_TRAIN_END + F_END * 4;
+
+// s = 1 / (1 + exp(-z)) and z / (1 + exp(-z)), the latter from z s by two exact
+// residuals (the first makes it faithful, the second correctly rounded:
+// Markstein, IBM J. Res. Dev. 34, 1990); where the residual is no number (an
+// infinity) z s is the quotient.
+__device__ __forceinline__ float silu(float z, float& s) {
+  const float d = 1.0f + expf(-z);
+  s = __frcp_rn(d);
+  float q = z * s, r = fmaf(-q, d, z);
+  if (r == r) {
+    q = fmaf(r, s, q);
+    q = fmaf(fmaf(-q, d, z), s, q);
+  }
+  return q;
 }
-__device__ __forceinline__ void st_bf16(unsigned char* base, uint32_t off, float v) {
-  *reinterpret_cast<__nv_bfloat16*>(base + off) = __float2bfloat16_rn(v);
-}
+__device__ __forceinline__ float dsilu(float z, float s) { return s * (1.0f + z * (1.0f - s)); }
 
 // ---- features ---------------------------------------------------------------
 // f[0..15] and p_ref of one problem: states (rho, u, p) per side, EOS rows
-// {type, gamma, pc, b, q}.
+// {type, gamma, pc, b, q}.  Bound by the binary64 pipe (64 cycles per warp
+// instruction and sub-partition; five logarithms, three asinh): the ten
+// quotients and two roots run on the integer pipe instead, rounded alike, and a
+// row leaves in two 16-byte stores (262,144 problems 258 -> 199 us).
 __device__ double problem_features(double rl, double ul, double pl, const double* el, double rr, double ur,
                                    double pr, const double* er, float* f) {
   pl = fmax(pl, 1.0);
   pr = fmax(pr, 1.0);
-  double c2l = el[1] * (pl + el[2]) / (rl * (1.0 - el[3] * rl));
-  double c2r = er[1] * (pr + er[2]) / (rr * (1.0 - er[3] * rr));
+  double c2l = ddiv(el[1] * (pl + el[2]), rl * (1.0 - el[3] * rl));
+  double c2r = ddiv(er[1] * (pr + er[2]), rr * (1.0 - er[3] * rr));
   c2l = c2l > 0.0 ? c2l : 1.0;
   c2r = c2r > 0.0 ? c2r : 1.0;
-  double Cl = rl * sqrt(c2l), Cr = rr * sqrt(c2r);
-  double pref = (Cr * pl + Cl * pr) / (Cl + Cr);
-  double a = (ul - ur) * Cl * Cr / ((Cl + Cr) * pref);
+  double Cl = rl * dsqrt(c2l), Cr = rr * dsqrt(c2r);
+  double pref = ddiv(Cr * pl + Cl * pr, Cl + Cr);
+  double a = ddiv((ul - ur) * Cl * Cr, (Cl + Cr) * pref);
   f[0] = (float)(asinh(a) * 0.25);
-  f[1] = (float)(log(pl / pref) * 0.25);
-  f[2] = (float)(log(pr / pref) * 0.25);
-  f[3] = (float)(log(Cl / Cr) * 0.25);
-  f[4] = (float)((el[1] - 4.0) / 1.7);
-  f[5] = (float)((er[1] - 4.0) / 1.7);
-  f[6] = (float)(asinh(el[2] / pref) * 0.125);
-  f[7] = (float)(asinh(er[2] / pref) * 0.125);
+  f[1] = (float)(log(ddiv(pl, pref)) * 0.25);
+  f[2] = (float)(log(ddiv(pr, pref)) * 0.25);
+  f[3] = (float)(log(ddiv(Cl, Cr)) * 0.25);
+  f[4] = (float)ddiv(el[1] - 4.0, 1.7);
+  f[5] = (float)ddiv(er[1] - 4.0, 1.7);
+  f[6] = (float)(asinh(ddiv(el[2], pref)) * 0.125);
+  f[7] = (float)(asinh(ddiv(er[2], pref)) * 0.125);
   f[8] = (float)(2.0 * el[3] * rl - 1.0);
   f[9] = (float)(2.0 * er[3] * rr - 1.0);
-  f[10] = (float)(log(rl * c2l / pref) * 0.25);
-  f[11] = (float)(log(rr * c2r / pref) * 0.25);
+  f[10] = (float)(log(ddiv(rl * c2l, pref)) * 0.25);
+  f[11] = (float)(log(ddiv(rr * c2r, pref)) * 0.25);
   for (int i = 12; i < NF; i++) f[i] = 0.f;
   return pref;
+}
+
+// A row of 16 features -> bf16, two 16-byte stores.
+__device__ __forceinline__ void put_row(__nv_bfloat16* X, int64_t row, const float* f) {
+  uint4 w[2];
+  uint32_t* u = reinterpret_cast<uint32_t*>(w);
+#pragma unroll
+  for (int i = 0; i < NF / 2; i++) {
+    const __nv_bfloat162 b = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+    u[i] = *reinterpret_cast<const uint32_t*>(&b);
+  }
+  uint4* x = reinterpret_cast<uint4*>(X) + row * 2;
+  x[0] = w[0];
+  x[1] = w[1];
 }
 
 // 1D problems: W rows {rho_l, u_l, p_l, rho_r, u_r, p_r}, E rows {type, gamma,
@@ -119,7 +174,7 @@ __global__ void k_features(int64_t n, const double* __restrict__ W, const double
   const double* w = &W[q * 6];
   float f[NF];
   double pr = problem_features(w[0], w[1], w[2], &E[q * 10], w[3], w[4], w[5], &E[q * 10 + 5], f);
-  for (int i = 0; i < NF; i++) X[q * NF + i] = __float2bfloat16_rn(f[i]);
+  put_row(X, q, f);
   if (pref) pref[q] = (float)pr;
   if (t && pstar) t[q] = (float)(log(fmax(pstar[q], 1e-300) / pr) * 0.25);
 }
@@ -142,7 +197,7 @@ __global__ void k_features_faces(Params P, StateSet S, const int32_t* __restrict
     double er[5] = {(double)MR.type, MR.gam, MR.Pstiff, MR.type == M2CG_EOS_NASG ? MR.b : 0.0, 0.0};
     float f[NF];
     double pr = problem_features(S.q[0][m], S.q[1 + d][m], S.q[4][m], el, S.q[0][c], S.q[1 + d][c], S.q[4][c], er, f);
-    for (int i = 0; i < NF; i++) X[s * NF + i] = __float2bfloat16_rn(f[i]);
+    put_row(X, s, f);
     pref[s] = (float)pr;
   }
 }
@@ -163,37 +218,26 @@ __global__ void k_to_pressure(int64_t n, const float* __restrict__ t, const floa
 // ---- tile machinery -----------------------------------------------------------
 struct TileCtx {
   unsigned char* sm;
-  float* f32;  // b1 b2 b3 w4 | db1 db2 db3 dw4 | b4, loss, db4
+  float* f32;
   uint64_t* bar;
   uint32_t tm;
   uint32_t phase;
   bool ok;
+  int r, g, j0;   // this thread's row, column group and first column
 };
 
-__device__ void load_weights(TileCtx& c, const __nv_bfloat16* __restrict__ wbf, const float* __restrict__ prm,
-                             bool backward) {
-  int t = threadIdx.x;
-  for (int i = t; i < NH * NF; i += blockDim.x) {
-    int n = i / NF, k = i % NF;
-    *reinterpret_cast<__nv_bfloat16*>(c.sm + S_W1F + umma::kmajor_offset(n, k, NF)) = wbf[BF_W1F + i];
+__device__ __forceinline__ void load_weights(TileCtx& c, const __nv_bfloat16* __restrict__ wbf,
+                                             const float* __restrict__ prm, bool backward) {
+  const int t = threadIdx.x;
+  const uint4* src = reinterpret_cast<const uint4*>(wbf);
+  uint4* dst = reinterpret_cast<uint4*>(c.sm + S_W);
+  const int n = (backward ? NBF : BF_W2B) / 8;
+  for (int i = t; i < n; i += NTHR) dst[i] = src[i];
+  if (t < 256) {
+    const int off[4] = {OFF_B1, OFF_B2, OFF_B3, OFF_W4};
+    c.f32[t] = prm[off[t >> 6] + (t & 63)];
   }
-  for (int i = t; i < NH * NH; i += blockDim.x) {
-    int n = i / NH, k = i % NH;
-    uint32_t o = umma::kmajor_offset(n, k, NH);
-    *reinterpret_cast<__nv_bfloat16*>(c.sm + S_W2F + o) = wbf[BF_W2F + i];
-    *reinterpret_cast<__nv_bfloat16*>(c.sm + S_W3F + o) = wbf[BF_W3F + i];
-    if (backward) {
-      *reinterpret_cast<__nv_bfloat16*>(c.sm + S_W2B + o) = wbf[BF_W2B + i];
-      *reinterpret_cast<__nv_bfloat16*>(c.sm + S_W3B + o) = wbf[BF_W3B + i];
-    }
-  }
-  for (int i = t; i < NH; i += blockDim.x) {
-    c.f32[i] = prm[OFF_B1 + i];
-    c.f32[64 + i] = prm[OFF_B2 + i];
-    c.f32[128 + i] = prm[OFF_B3 + i];
-    c.f32[192 + i] = prm[OFF_W4 + i];
-  }
-  if (t == 0) c.f32[512] = prm[OFF_B4];
+  if (t == 0) c.f32[F_B4] = prm[OFF_B4];
 }
 
 // Orders generic shared-memory writes before MMAs issued after the barrier,
@@ -205,71 +249,109 @@ __device__ __forceinline__ void sync_for_mma() {
   umma::fence_after_sync();
 }
 
-__device__ __forceinline__ void commit_wait(TileCtx& c) {
-  if (threadIdx.x == 0) umma::mma_commit(c.bar);
-  bool ok = umma::mbar_wait(c.bar, c.phase, MAX_POLLS);
+// Waits for the MMAs up to the last commit.
+__device__ __forceinline__ void wait_mma(TileCtx& c) {
+  c.ok = umma::mbar_wait(c.bar, c.phase, MAX_POLLS) && c.ok;
   c.phase ^= 1u;
-  c.ok = __syncthreads_and(ok) && c.ok;
   umma::fence_after_sync();
 }
 
-// TMEM address of this thread's row (lane) at column col.
+// TMEM address of this thread's row (lane) at column col + j0.
 __device__ __forceinline__ uint32_t trow(const TileCtx& c, int col) {
-  return c.tm + ((uint32_t)(threadIdx.x & ~31) << 16) + (uint32_t)col;
+  return c.tm + ((uint32_t)(c.r & ~31) << 16) + (uint32_t)(col + c.j0);
 }
 
-// Layer epilogue: H = bf16(SiLU(acc + bias)) into an A tile (K = 64).
-__device__ void epilogue_silu(const TileCtx& c, int col, const float* bias, unsigned char* dst) {
-  const int r = threadIdx.x;
-  for (int j0 = 0; j0 < NH; j0 += 16) {
-    float v[16];
-    umma::tmem_ld16(trow(c, col + j0), v);
+// 16 values of this thread's row and columns -> bf16 in a [128][64] operand tile.
+__device__ __forceinline__ void store16(const TileCtx& c, unsigned char* tile, const float (&h)[CG]) {
 #pragma unroll
-    for (int i = 0; i < 16; i++) st_bf16(dst, umma::kmajor_offset(r, j0 + i, NH), silu(v[i] + bias[j0 + i]));
+  for (int q = 0; q < 2; q++) {
+    uint4 w;
+    uint32_t* u = reinterpret_cast<uint32_t*>(&w);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const __nv_bfloat162 b = __floats2bfloat162_rn(h[8 * q + 2 * i], h[8 * q + 2 * i + 1]);
+      u[i] = *reinterpret_cast<const uint32_t*>(&b);
+    }
+    *reinterpret_cast<uint4*>(tile + umma::kmajor_offset(c.r, c.j0 + 8 * q, NH)) = w;
   }
 }
 
-// Forward through the three GEMM layers for the tile already in S_XA; leaves
-// Z1..Z3 accumulators (bias not added) in TMEM columns 0, 64, 128.
-__device__ void forward_tile(TileCtx& c) {
-  sync_for_mma();
-  if (threadIdx.x == 0) umma::gemm_128xN(c.tm + 0, c.sm + S_XA, c.sm + S_W1F, NH, NF, false);
-  commit_wait(c);
-  epilogue_silu(c, 0, c.f32 + 0, c.sm + S_H1A);
-  sync_for_mma();
-  if (threadIdx.x == 0) umma::gemm_128xN(c.tm + 64, c.sm + S_H1A, c.sm + S_W2F, NH, NH, false);
-  commit_wait(c);
-  epilogue_silu(c, 64, c.f32 + 64, c.sm + S_H2A);
-  sync_for_mma();
-  if (threadIdx.x == 0) umma::gemm_128xN(c.tm + 128, c.sm + S_H2A, c.sm + S_W3F, NH, NH, false);
-  commit_wait(c);
+// Half a network input row (8 features, 16 bytes) per thread of the first 256.
+__device__ __forceinline__ uint4 read_x(const __nv_bfloat16* __restrict__ X, int64_t row, bool valid) {
+  return valid ? reinterpret_cast<const uint4*>(X)[row * 2 + (threadIdx.x & 1)] : make_uint4(0, 0, 0, 0);
+}
+__device__ __forceinline__ void store_x(const TileCtx& c, uint4 x) {
+  *reinterpret_cast<uint4*>(c.sm + S_XA + umma::kmajor_offset(threadIdx.x >> 1, (threadIdx.x & 1) * 8, NF)) = x;
 }
 
-// Scalar head on the CUDA cores: out = b4 + sum_j SiLU(z3_j + b3_j) w4_j.
-__device__ float head(const TileCtx& c) {
-  float out = c.f32[512];
-  for (int j0 = 0; j0 < NH; j0 += 16) {
-    float v[16];
-    umma::tmem_ld16(trow(c, 128 + j0), v);
+// Hidden layer l (0, 1): its GEMM, then H = bf16(SiLU(Z + b)) into the operand
+// tile dst; ds: SiLU'(Z + b) of this thread's row and columns (training).
+template <bool Train>
+__device__ __forceinline__ void hidden_layer(TileCtx& c, int l, const unsigned char* in, const unsigned char* w, int K,
+                                             unsigned char* dst, float (&ds)[CG]) {
+  sync_for_mma();
+  if (threadIdx.x == 0) {
+    umma::gemm_128xN(c.tm + 64 * l, in, w, NH, K, false);
+    umma::mma_commit(c.bar);
+  }
+  wait_mma(c);
+  float v[CG];
+  umma::tmem_ld16(trow(c, 64 * l), v);
+  const float* b = c.f32 + 64 * l + c.j0;
 #pragma unroll
-    for (int i = 0; i < 16; i++) out += silu(v[i] + c.f32[128 + j0 + i]) * c.f32[192 + j0 + i];
+  for (int i = 0; i < CG; i++) {
+    const float z = v[i] + b[i];
+    float s;
+    v[i] = silu(z, s);
+    if (Train) ds[i] = dsilu(z, s);
+  }
+  store16(c, dst, v);
+}
+
+// The network for the tile in S_XA: returns, in the threads of group 0, the
+// output of the row (the scalar head out = b4 + sum_j SiLU(z3_j + b3_j) w4_j,
+// summed in this order by one thread); in training h3, ds1..ds3 of the row's 16
+// columns as well.
+template <bool Train>
+__device__ __forceinline__ float forward_tile(TileCtx& c, float (&h3)[CG], float (&ds1)[CG], float (&ds2)[CG],
+                                              float (&ds3)[CG]) {
+  const unsigned char* w = c.sm + S_W;
+  hidden_layer<Train>(c, 0, c.sm + S_XA, w + 2 * BF_W1F, NF, c.sm + S_H1A, ds1);
+  hidden_layer<Train>(c, 1, c.sm + S_H1A, w + 2 * BF_W2F, NH, c.sm + S_H2A, ds2);
+  sync_for_mma();
+  if (threadIdx.x == 0) {
+    umma::gemm_128xN(c.tm + 128, c.sm + S_H2A, w + 2 * BF_W3F, NH, NH, false);
+    umma::mma_commit(c.bar);
+  }
+  wait_mma(c);
+  umma::tmem_ld16(trow(c, 128), h3);
+  float* hb = reinterpret_cast<float*>(c.sm + (Train ? S_H3_TRAIN : S_H3_FWD)) + c.r;
+#pragma unroll
+  for (int i = 0; i < CG; i++) {
+    const float z = h3[i] + c.f32[128 + c.j0 + i];
+    float s;
+    h3[i] = silu(z, s);
+    if (Train) ds3[i] = dsilu(z, s);
+    hb[(c.j0 + i) * TILE] = h3[i];
+  }
+  __syncthreads();
+  float out = c.f32[F_B4];
+  if (c.g == 0) {
+#pragma unroll 16
+    for (int j = 0; j < NH; j++) out = fmaf(hb[j * TILE], c.f32[192 + j], out);
   }
   return out;
 }
 
-__device__ void load_x_row(TileCtx& c, const __nv_bfloat16* __restrict__ X, int64_t row, bool valid) {
-  const int r = threadIdx.x;
-  for (int k = 0; k < NF; k++) {
-    __nv_bfloat16 v = valid ? X[row * NF + k] : __float2bfloat16_rn(0.f);
-    *reinterpret_cast<__nv_bfloat16*>(c.sm + S_XA + umma::kmajor_offset(r, k, NF)) = v;
-  }
-}
-
-__device__ void tile_setup(TileCtx& c, unsigned char* sm, uint64_t* bar, uint32_t* tslot) {
+__device__ __forceinline__ void tile_setup(TileCtx& c, unsigned char* sm, float* f32, uint64_t* bar, uint32_t* tslot) {
   c.sm = sm;
+  c.f32 = f32;
   c.bar = bar;
   c.phase = 0;
   c.ok = true;
+  c.r = threadIdx.x & (TILE - 1);
+  c.g = threadIdx.x / TILE;
+  c.j0 = CG * c.g;
   if (threadIdx.x == 0) umma::mbar_init(bar, 1);
   if (threadIdx.x < 32) umma::tmem_alloc(tslot, 256);
   umma::fence_before_sync();
@@ -278,7 +360,7 @@ __device__ void tile_setup(TileCtx& c, unsigned char* sm, uint64_t* bar, uint32_
   c.tm = *tslot;
 }
 
-__device__ void tile_teardown(TileCtx& c) {
+__device__ __forceinline__ void tile_teardown(TileCtx& c) {
   umma::fence_before_sync();
   __syncthreads();
   if (threadIdx.x < 32) umma::tmem_dealloc(c.tm, 256);
@@ -287,7 +369,9 @@ __device__ void tile_teardown(TileCtx& c) {
 // ---- inference ----------------------------------------------------------------
 // Persistent: CTA b handles tiles b, b + grid, ...  out[row] = network output.
 // rows = min(n, *count) when count is given (the device-side interface count).
-__global__ void __launch_bounds__(TILE, 1) k_forward(int64_t n, const unsigned long long* count,
+// Two CTAs per SM (256 TMEM columns each), one working while the other waits;
+// the next tile's inputs are fetched during the current one.
+__global__ void __launch_bounds__(NTHR, 2) k_forward(int64_t n, const unsigned long long* count,
                                                       const __nv_bfloat16* __restrict__ X,
                                                       const __nv_bfloat16* __restrict__ wbf,
                                                       const float* __restrict__ prm, float* out, int* err,
@@ -300,57 +384,65 @@ __global__ void __launch_bounds__(TILE, 1) k_forward(int64_t n, const unsigned l
   int64_t ntiles = (n + TILE - 1) / TILE;
   if ((int64_t)blockIdx.x >= ntiles) return;
   TileCtx c;
-  c.f32 = reinterpret_cast<float*>(sm + SMEM_FWD - (8 * 64 + 4) * 4);
-  tile_setup(c, sm, &bar, &tslot);
+  tile_setup(c, sm, reinterpret_cast<float*>(sm + S_FWD_END), &bar, &tslot);
+  const bool loads = threadIdx.x < 2 * TILE;
+  int64_t xrow = (int64_t)blockIdx.x * TILE + (threadIdx.x >> 1);
+  uint4 x = read_x(X, xrow, loads && xrow < n);
   load_weights(c, wbf, prm, false);
   for (int64_t tile = blockIdx.x; tile < ntiles && c.ok; tile += gridDim.x) {
-    int64_t row = tile * TILE + threadIdx.x;
-    load_x_row(c, X, row, row < n);
-    forward_tile(c);
-    float o = head(c);
-    if (row < n) out[row] = o;
-    umma::fence_before_sync();
-    __syncthreads();  // TMEM reads done before the next tile's MMAs
-    umma::fence_after_sync();
+    if (loads) store_x(c, x);
+    xrow += (int64_t)gridDim.x * TILE;
+    x = read_x(X, xrow, loads && xrow < n);
+    float h3[CG], none[CG];
+    const float o = forward_tile<false>(c, h3, none, none, none);
+    const int64_t row = tile * TILE + c.r;
+    if (c.g == 0 && row < n) out[row] = o;
+    c.ok = __syncthreads_and(c.ok);   // (also: the head's activations are read)
   }
   if (!c.ok && threadIdx.x == 0) atomicExch(err, 1);
   tile_teardown(c);
 }
 
 // ---- training -------------------------------------------------------------------
-// Warp-reduce v over the 32 rows of this warp, then add into s[j] (shared).
-__device__ __forceinline__ void col_reduce_add(float* s, int j, float v) {
+// Sums of v[0..15] over the 32 rows of the warp into s[0..15]: each step of
+// the butterfly also halves the columns a lane keeps, 16 shuffles in all.
+__device__ __forceinline__ void col_sums(float* s, const float (&v)[CG]) {
+  const int lane = threadIdx.x & 31;
+  float a[CG];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(&s[j], v);
-}
-
-// dZ (fp32, per row) -> bf16 A tile dZa [row][j] and B tile dZT [j][row].
-__device__ __forceinline__ void store_dz(const TileCtx& c, int j, float dz) {
-  const int r = threadIdx.x;
-  st_bf16(c.sm + S_DZA, umma::kmajor_offset(r, j, NH), dz);
-  st_bf16(c.sm + S_DZT, umma::kmajor_offset(j, r, TILE), dz);
-}
-
-// Weight-gradient readout: TMEM columns 192..255 hold D[i][j] for input
-// feature i = row (< n_in); grad[off + j * n_in + i] += D[i][j].
-__device__ void dw_readout(const TileCtx& c, float* grad, int off, int n_in) {
-  const int i = threadIdx.x;
-  if ((threadIdx.x >> 5) * 32 >= n_in) return;  // warp-uniform: no rows of interest in this warp
-  for (int j0 = 0; j0 < NH; j0 += 16) {
-    float v[16];
-    umma::tmem_ld16(trow(c, 192 + j0), v);
-    if (i < n_in) {
+  for (int i = 0; i < CG; i++) a[i] = v[i];
 #pragma unroll
-      for (int q = 0; q < 16; q++) atomicAdd(&grad[off + (j0 + q) * n_in + i], v[q]);
+  for (int n = CG / 2, o = 16; n > 0; n >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < n; i++) {
+      const float give = up ? a[i] : a[i + n], keep = up ? a[i + n] : a[i];
+      a[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
     }
+  }
+  a[0] += __shfl_xor_sync(0xffffffffu, a[0], 1);
+  if ((lane & 1) == 0) s[lane >> 1] = a[0];
+}
+
+// Weight-gradient readout: 64 TMEM columns from col on hold D[i][j] for input
+// feature i = row (< n_in); grad[off + j * n_in + i] += D[i][j].
+__device__ __forceinline__ void dw_readout(const TileCtx& c, int col, float* grad, int off, int n_in) {
+  if ((c.r & ~31) >= n_in) return;  // warp-uniform: no rows of interest in this warp
+  float v[CG];
+  umma::tmem_ld16(trow(c, col), v);
+  if (c.r < n_in) {
+#pragma unroll
+    for (int q = 0; q < CG; q++) atomicAdd(&grad[off + (c.j0 + q) * n_in + c.r], v[q]);
   }
 }
 
 // One 128-row tile of the batch: forward, squared-error loss on the target,
 // backward; gradients (of the mean loss over the batch) and the loss sum are
-// accumulated into grad[] and loss[0].
-__global__ void __launch_bounds__(TILE, 1) k_train(int64_t batch, const int32_t* __restrict__ idx,
+// accumulated into grad[] and loss[0].  TMEM columns: Z1 0, Z2 64, Z3 128; then
+// dW3 192, dH2 128, dW2 0, dH1 64, dW1 128.  Each layer's input gradient is
+// issued and committed before its weight gradient, which runs on while the next
+// layer's dZ is computed (its own operand tile) and is read after the next wait.
+__global__ void __launch_bounds__(NTHR, 1) k_train(int64_t batch, const int32_t* __restrict__ idx,
                                                     const __nv_bfloat16* __restrict__ X, const float* __restrict__ y,
                                                     const __nv_bfloat16* __restrict__ wbf,
                                                     const float* __restrict__ prm, float* grad, float* loss,
@@ -359,120 +451,117 @@ __global__ void __launch_bounds__(TILE, 1) k_train(int64_t batch, const int32_t*
   __shared__ uint64_t bar;
   __shared__ uint32_t tslot;
   TileCtx c;
-  c.f32 = reinterpret_cast<float*>(sm + S_F32);
-  const int r = threadIdx.x;
-  const int64_t brow = (int64_t)blockIdx.x * TILE + r;
-  const bool valid = brow < batch;
-  const int64_t row = valid ? (idx ? (int64_t)idx[brow] : brow) : 0;
-  tile_setup(c, sm, &bar, &tslot);
+  tile_setup(c, sm, reinterpret_cast<float*>(sm + S_TRAIN_END), &bar, &tslot);
+  const int64_t b0 = (int64_t)blockIdx.x * TILE;
+  uint4 x = make_uint4(0, 0, 0, 0);
+  if (threadIdx.x < 2 * TILE) {
+    const int64_t xb = b0 + (threadIdx.x >> 1);
+    x = read_x(X, xb < batch ? (idx ? (int64_t)idx[xb] : xb) : 0, xb < batch);
+  }
+  const bool valid = b0 + c.r < batch;
+  const float target = valid ? y[idx ? (int64_t)idx[b0 + c.r] : b0 + c.r] : 0.f;
   load_weights(c, wbf, prm, true);
-  for (int i = r; i < 4 * 64; i += TILE) c.f32[256 + i] = 0.f;  // reductions db1 db2 db3 dw4
-  if (r == 0) { c.f32[513] = 0.f; c.f32[514] = 0.f; }             // loss, db4 (f32[512] holds b4)
-  // HT rows 64..127 (padding of the feature dimension) stay zero
-  for (int i = r; i < 32768 / 4; i += TILE) reinterpret_cast<uint32_t*>(sm + S_HT)[i] = 0u;
-  load_x_row(c, X, row, valid);
-  forward_tile(c);
-  // head, loss and dOut
-  float out = head(c);
-  float d = 0.f;
-  if (valid) {
-    float e = out - y[row];
-    d = 2.f * e / (float)batch;
-    atomicAdd(&c.f32[513], e * e);
-    atomicAdd(&c.f32[514], d);
-  }
-  float* sdb1 = c.f32 + 256;
-  float* sdb2 = c.f32 + 320;
-  float* sdb3 = c.f32 + 384;
-  float* sdw4 = c.f32 + 448;
-  // layer 3: dZ3 = d w4 SiLU'(z3); dw4 = sum d h3; H2^T into HT
-  for (int j0 = 0; j0 < NH; j0 += 16) {
-    float v[16];
-    umma::tmem_ld16(trow(c, 128 + j0), v);
-#pragma unroll
-    for (int q = 0; q < 16; q++) {
-      int j = j0 + q;
-      float z = v[q] + c.f32[128 + j];
-      float dz = d * c.f32[192 + j] * dsilu(z);
-      store_dz(c, j, dz);
-      col_reduce_add(sdb3, j, dz);
-      col_reduce_add(sdw4, j, d * silu(z));
-    }
-  }
-  for (int i = 0; i < NH; i++)
-    *reinterpret_cast<__nv_bfloat16*>(sm + S_HT + umma::kmajor_offset(i, r, TILE)) =
-        *reinterpret_cast<const __nv_bfloat16*>(sm + S_H2A + umma::kmajor_offset(r, i, NH));
-  sync_for_mma();
-  if (r == 0) {
-    umma::gemm_128xN(c.tm + 192, sm + S_HT, sm + S_DZT, NH, TILE, false);  // dW3[i][j]
-    umma::gemm_128xN(c.tm + 128, sm + S_DZA, sm + S_W3B, NH, NH, false);  // dH2[r][i]
-  }
-  commit_wait(c);
-  dw_readout(c, grad, OFF_W3, NH);
-  // layer 2: dZ2 = dH2 SiLU'(z2); H1^T into HT
-  for (int j0 = 0; j0 < NH; j0 += 16) {
-    float g[16], v[16];
-    umma::tmem_ld16(trow(c, 128 + j0), g);
-    umma::tmem_ld16(trow(c, 64 + j0), v);
-#pragma unroll
-    for (int q = 0; q < 16; q++) {
-      int j = j0 + q;
-      float dz = g[q] * dsilu(v[q] + c.f32[64 + j]);
-      store_dz(c, j, dz);
-      col_reduce_add(sdb2, j, dz);
-    }
-  }
-  for (int i = 0; i < NH; i++)
-    *reinterpret_cast<__nv_bfloat16*>(sm + S_HT + umma::kmajor_offset(i, r, TILE)) =
-        *reinterpret_cast<const __nv_bfloat16*>(sm + S_H1A + umma::kmajor_offset(r, i, NH));
-  sync_for_mma();
-  if (r == 0) {
-    umma::gemm_128xN(c.tm + 192, sm + S_HT, sm + S_DZT, NH, TILE, false);  // dW2
-    umma::gemm_128xN(c.tm + 64, sm + S_DZA, sm + S_W2B, NH, NH, false);   // dH1
-  }
-  commit_wait(c);
-  dw_readout(c, grad, OFF_W2, NH);
-  // layer 1: dZ1 = dH1 SiLU'(z1); X^T into HT (feature rows 16..63 zeroed)
-  for (int j0 = 0; j0 < NH; j0 += 16) {
-    float g[16], v[16];
-    umma::tmem_ld16(trow(c, 64 + j0), g);
-    umma::tmem_ld16(trow(c, 0 + j0), v);
-#pragma unroll
-    for (int q = 0; q < 16; q++) {
-      int j = j0 + q;
-      float dz = g[q] * dsilu(v[q] + c.f32[j]);
-      st_bf16(sm + S_DZT, umma::kmajor_offset(j, r, TILE), dz);
-      col_reduce_add(sdb1, j, dz);
-    }
-  }
-  for (int i = 0; i < NH; i++) {
-    __nv_bfloat16 v = (i < NF) ? *reinterpret_cast<const __nv_bfloat16*>(sm + S_XA + umma::kmajor_offset(r, i, NF))
-                               : __float2bfloat16_rn(0.f);
-    *reinterpret_cast<__nv_bfloat16*>(sm + S_HT + umma::kmajor_offset(i, r, TILE)) = v;
-  }
-  sync_for_mma();
-  if (r == 0) umma::gemm_128xN(c.tm + 192, sm + S_HT, sm + S_DZT, NH, TILE, false);  // dW1
-  commit_wait(c);
-  dw_readout(c, grad, OFF_W1, NF);
+  if (threadIdx.x < 2 * TILE) store_x(c, x);
+  float h3[CG], ds1[CG], ds2[CG], ds3[CG];
+  const float o = forward_tile<true>(c, h3, ds1, ds2, ds3);
+  if (c.g == 0) c.f32[F_OUT + c.r] = o;
   __syncthreads();
-  if (r < NH) {
-    atomicAdd(&grad[OFF_B1 + r], sdb1[r]);
-    atomicAdd(&grad[OFF_B2 + r], sdb2[r]);
-    atomicAdd(&grad[OFF_B3 + r], sdb3[r]);
-    atomicAdd(&grad[OFF_W4 + r], sdw4[r]);
+  const float e = valid ? c.f32[F_OUT + c.r] - target : 0.f;
+  const float d = 2.f * e / (float)batch;
+  const int lane = threadIdx.x & 31, wr = c.r >> 5;
+  float* sums = c.f32 + F_SUM + wr * NH + c.j0;   // + 4 NH per quantity
+  // layer 3: dZ3 = d w4 SiLU'(z3); dw4 = sum d h3
+  float dz[CG];
+#pragma unroll
+  for (int q = 0; q < CG; q++) {
+    dz[q] = d * c.f32[192 + c.j0 + q] * ds3[q];
+    h3[q] *= d;
   }
-  if (r == 0) {
-    atomicAdd(&grad[OFF_B4], c.f32[514]);
-    atomicAdd(loss, c.f32[513]);
-    if (!c.ok) atomicExch(err, 1);
+  store16(c, sm + S_DZ3, dz);
+  sync_for_mma();
+  if (threadIdx.x == 0) {
+    umma::gemm_128xN(c.tm + 128, sm + S_DZ3, sm + S_W + 2 * BF_W3B, NH, NH, false);   // dH2[r][i]
+    umma::mma_commit(c.bar);
+    umma::gemm_tn_128xN(c.tm + 192, sm + S_H2A, NH, sm + S_DZ3, NH, TILE);            // dW3[i][j]
   }
+  col_sums(sums + 2 * 4 * NH, dz);
+  col_sums(sums + 3 * 4 * NH, h3);
+  if (c.g == 0) {
+    float l = e * e, db = d;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      l += __shfl_xor_sync(0xffffffffu, l, o);
+      db += __shfl_xor_sync(0xffffffffu, db, o);
+    }
+    if (lane == 0) { c.f32[F_LOSS + wr] = l; c.f32[F_LOSS + 4 + wr] = db; }
+  }
+  wait_mma(c);
+  // layer 2: dZ2 = dH2 SiLU'(z2)
+  umma::tmem_ld16(trow(c, 128), dz);
+#pragma unroll
+  for (int q = 0; q < CG; q++) dz[q] *= ds2[q];
+  store16(c, sm + S_DZ2, dz);
+  sync_for_mma();
+  if (threadIdx.x == 0) {
+    umma::gemm_128xN(c.tm + 64, sm + S_DZ2, sm + S_W + 2 * BF_W2B, NH, NH, false);    // dH1
+    umma::mma_commit(c.bar);
+    umma::gemm_tn_128xN(c.tm + 0, sm + S_H1A, NH, sm + S_DZ2, NH, TILE);              // dW2
+  }
+  col_sums(sums + 1 * 4 * NH, dz);
+  wait_mma(c);
+  // layer 1: dZ1 = dH1 SiLU'(z1)
+  umma::tmem_ld16(trow(c, 64), dz);
+#pragma unroll
+  for (int q = 0; q < CG; q++) dz[q] *= ds1[q];
+  store16(c, sm + S_DZ1, dz);
+  sync_for_mma();
+  if (threadIdx.x == 0) {
+    umma::gemm_tn_128xN(c.tm + 128, sm + S_XA, NF, sm + S_DZ1, NH, TILE);             // dW1
+    umma::mma_commit(c.bar);
+  }
+  col_sums(sums, dz);
+  dw_readout(c, 192, grad, OFF_W3, NH);   // complete: committed with dH1
+  wait_mma(c);
+  dw_readout(c, 0, grad, OFF_W2, NH);
+  dw_readout(c, 128, grad, OFF_W1, NF);
+  __syncthreads();
+  if (threadIdx.x < 256) {
+    const int k = threadIdx.x >> 6, j = threadIdx.x & 63;
+    const int off[4] = {OFF_B1, OFF_B2, OFF_B3, OFF_W4};
+    const float* s = c.f32 + F_SUM + k * 4 * NH + j;
+    atomicAdd(&grad[off[k] + j], (s[0] + s[NH]) + (s[2 * NH] + s[3 * NH]));
+  } else if (threadIdx.x < 258) {
+    const float* s = c.f32 + F_LOSS + 4 * (threadIdx.x - 256);
+    atomicAdd(threadIdx.x == 256 ? loss : &grad[OFF_B4], (s[0] + s[1]) + (s[2] + s[3]));
+  }
+  if (!c.ok) atomicExch(err, 1);
   tile_teardown(c);
 }
 
-// Adam on the FP32 master weights; clears the gradient.  bc1 = 1 - beta1^step,
-// bc2 = 1 - beta2^step.  k_pack_bf16 then refreshes the BF16 GEMM copies.
-__global__ void k_adam(float* prm, float* grad, float* m, float* v, float lr, float b1, float b2, float eps, float bc1,
-                       float bc2) {
+// Where parameter i is a GEMM weight: its BF16 copies (forward and transposed).
+__device__ __forceinline__ void pack_param(int i, float v, __nv_bfloat16* wbf) {
+  const __nv_bfloat16 b = __float2bfloat16_rn(v);
+  unsigned char* w = reinterpret_cast<unsigned char*>(wbf);
+  auto put = [&](int base, int r, int k, int K) {
+    *reinterpret_cast<__nv_bfloat16*>(w + 2 * base + umma::kmajor_offset(r, k, K)) = b;
+  };
+  if (i < OFF_B1) {
+    put(BF_W1F, i / NF, i % NF, NF);
+  } else if (i >= OFF_W2 && i < OFF_B2) {
+    const int o = (i - OFF_W2) / NH, in = (i - OFF_W2) % NH;   // W[o][in]
+    put(BF_W2F, o, in, NH);
+    put(BF_W2B, in, o, NH);
+  } else if (i >= OFF_W3 && i < OFF_B3) {
+    const int o = (i - OFF_W3) / NH, in = (i - OFF_W3) % NH;
+    put(BF_W3F, o, in, NH);
+    put(BF_W3B, in, o, NH);
+  }
+}
+
+// Adam on the FP32 master weights and their BF16 copies; clears the gradient.
+// bc1 = 1 - beta1^step, bc2 = 1 - beta2^step.
+__global__ void k_adam(float* prm, float* grad, float* m, float* v, __nv_bfloat16* wbf, float lr, float b1, float b2,
+                       float eps, float bc1, float bc2) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= NPARAM) return;
   float g = grad[i];
@@ -480,22 +569,15 @@ __global__ void k_adam(float* prm, float* grad, float* m, float* v, float lr, fl
   float vi = b2 * v[i] + (1.f - b2) * g * g;
   m[i] = mi;
   v[i] = vi;
-  prm[i] = prm[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+  const float p = prm[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+  prm[i] = p;
   grad[i] = 0.f;
+  pack_param(i, p, wbf);
 }
 
-// BF16 copies of the three GEMM weight matrices (forward and transposed).
 __global__ void k_pack_bf16(const float* __restrict__ prm, __nv_bfloat16* wbf) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < NH * NF) wbf[BF_W1F + i] = __float2bfloat16_rn(prm[OFF_W1 + i]);
-  if (i < NH * NH) {
-    int o = i / NH, in = i % NH;  // W[o][in]
-    __nv_bfloat16 w2 = __float2bfloat16_rn(prm[OFF_W2 + i]), w3 = __float2bfloat16_rn(prm[OFF_W3 + i]);
-    wbf[BF_W2F + i] = w2;
-    wbf[BF_W3F + i] = w3;
-    wbf[BF_W2B + in * NH + o] = w2;
-    wbf[BF_W3B + in * NH + o] = w3;
-  }
+  if (i < NPARAM) pack_param(i, prm[i], wbf);
 }
 
 }  // namespace mlp
@@ -604,7 +686,7 @@ m2cg_status m2cg_mlp_set_params(m2cg_mlp* m, const float* params) {
   MCK(cudaMemsetAsync(m->adam_m, 0, NPARAM * sizeof(float), m->stream));
   MCK(cudaMemsetAsync(m->adam_v, 0, NPARAM * sizeof(float), m->stream));
   MCK(cudaMemsetAsync(m->err, 0, sizeof(int), m->stream));
-  k_pack_bf16<<<(NH * NH + 255) / 256, 256, 0, m->stream>>>(m->prm, m->wbf);
+  k_pack_bf16<<<(NPARAM + 255) / 256, 256, 0, m->stream>>>(m->prm, m->wbf);
   MCK(cudaGetLastError());
   m->step = 0;
   MCK(cudaStreamSynchronize(m->stream));
@@ -617,8 +699,8 @@ m2cg_status m2cg_mlp_adam_step(m2cg_mlp* m, const float* grad, float lr) {
   MCK(cudaMemcpyAsync(m->grad, grad, NPARAM * sizeof(float), cudaMemcpyHostToDevice, m->stream));
   m->step++;
   const float bc1 = 1.f - std::pow(b1, (float)m->step), bc2 = 1.f - std::pow(b2, (float)m->step);
-  k_adam<<<(NPARAM + 255) / 256, 256, 0, m->stream>>>(m->prm, m->grad, m->adam_m, m->adam_v, lr, b1, b2, eps, bc1, bc2);
-  k_pack_bf16<<<(NH * NH + 255) / 256, 256, 0, m->stream>>>(m->prm, m->wbf);
+  k_adam<<<(NPARAM + 127) / 128, 128, 0, m->stream>>>(m->prm, m->grad, m->adam_m, m->adam_v, m->wbf, lr, b1, b2, eps,
+                                                      bc1, bc2);
   MCK(cudaGetLastError());
   MCK(cudaStreamSynchronize(m->stream));
   return M2CG_OK;
@@ -706,13 +788,12 @@ m2cg_status m2cg_mlp_train(m2cg_mlp* m, int32_t epochs, int32_t batch, float lr,
     MCK(cudaMemcpyAsync(m->perm, perm.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, m->stream));
     MCK(cudaMemsetAsync(m->loss, 0, sizeof(float), m->stream));
     for (int64_t b0 = 0; b0 + batch <= n; b0 += batch) {  // whole batches only
-      k_train<<<(unsigned)((batch + TILE - 1) / TILE), TILE, SMEM_TRAIN, m->stream>>>(
+      k_train<<<(unsigned)((batch + TILE - 1) / TILE), NTHR, SMEM_TRAIN, m->stream>>>(
           batch, m->perm + b0, m->X, m->y, m->wbf, m->prm, m->grad, m->loss, m->err);
       m->step++;
       float bc1 = 1.f - std::pow(b1, (float)m->step), bc2 = 1.f - std::pow(b2, (float)m->step);
-      k_adam<<<(NPARAM + 255) / 256, 256, 0, m->stream>>>(m->prm, m->grad, m->adam_m, m->adam_v, lr_ep, b1, b2,
+      k_adam<<<(NPARAM + 127) / 128, 128, 0, m->stream>>>(m->prm, m->grad, m->adam_m, m->adam_v, m->wbf, lr_ep, b1, b2,
                                                           eps, bc1, bc2);
-      k_pack_bf16<<<(NH * NH + 255) / 256, 256, 0, m->stream>>>(m->prm, m->wbf);
     }
     MCK(cudaGetLastError());
     if (loss_per_epoch) {
@@ -742,7 +823,7 @@ m2cg_status m2cg_mlp_grad(m2cg_mlp* m, int64_t n, const float* X, const float* t
   MCK(cudaMemcpyAsync(dt, t, n * sizeof(float), cudaMemcpyHostToDevice, m->stream));
   MCK(cudaMemsetAsync(m->grad, 0, NPARAM * sizeof(float), m->stream));
   MCK(cudaMemsetAsync(m->loss, 0, sizeof(float), m->stream));
-  k_train<<<(unsigned)((n + TILE - 1) / TILE), TILE, SMEM_TRAIN, m->stream>>>(n, nullptr, dX, dt, m->wbf, m->prm,
+  k_train<<<(unsigned)((n + TILE - 1) / TILE), NTHR, SMEM_TRAIN, m->stream>>>(n, nullptr, dX, dt, m->wbf, m->prm,
                                                                               m->grad, m->loss, m->err);
   MCK(cudaGetLastError());
   MCK(cudaMemcpyAsync(grad, m->grad, NPARAM * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
@@ -766,8 +847,8 @@ m2cg_status m2cg_mlp_forward(m2cg_mlp* m, int64_t n, const float* X, float* t) {
   MCK(cudaMalloc(&dt, n * sizeof(float)));
   MCK(cudaMemcpyAsync(dX, h.data(), n * NF * sizeof(__nv_bfloat16), cudaMemcpyHostToDevice, m->stream));
   int64_t ntiles = (n + TILE - 1) / TILE;
-  int grid = (int)std::min<int64_t>(ntiles, m->nsm);
-  k_forward<<<grid, TILE, SMEM_FWD, m->stream>>>(n, nullptr, dX, m->wbf, m->prm, dt, m->err, nullptr);
+  int grid = (int)std::min<int64_t>(ntiles, 2 * m->nsm);
+  k_forward<<<grid, NTHR, SMEM_FWD, m->stream>>>(n, nullptr, dX, m->wbf, m->prm, dt, m->err, nullptr);
   MCK(cudaGetLastError());
   MCK(cudaMemcpyAsync(t, dt, n * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
   MCK(cudaStreamSynchronize(m->stream));
@@ -797,8 +878,8 @@ m2cg_status m2cg_mlp_predict(m2cg_mlp* m, int64_t n, const double* W, const doub
   MCK(cudaEventRecord(e0, m->stream));
   k_features<<<(unsigned)((n + 255) / 256), 256, 0, m->stream>>>(n, dW, dE, nullptr, dX, dref, nullptr);
   int64_t ntiles = (n + TILE - 1) / TILE;
-  int grid = (int)std::min<int64_t>(ntiles, m->nsm);
-  k_forward<<<grid, TILE, SMEM_FWD, m->stream>>>(n, nullptr, dX, m->wbf, m->prm, dt, m->err, nullptr);
+  int grid = (int)std::min<int64_t>(ntiles, 2 * m->nsm);
+  k_forward<<<grid, NTHR, SMEM_FWD, m->stream>>>(n, nullptr, dX, m->wbf, m->prm, dt, m->err, nullptr);
   k_to_pressure<<<(unsigned)std::min<int64_t>((n + 255) / 256, 65535), 256, 0, m->stream>>>(n, dt, dref, dp,
                                                                                               nullptr, nullptr, nullptr);
   MCK(cudaEventRecord(e1, m->stream));
@@ -822,8 +903,8 @@ void mlp_warm_faces(m2cg_mlp* m, cudaStream_t s, int nsm, const Params& P, const
                     const IfaceList& L, __nv_bfloat16* X, float* t, float* pref, float* warm, const DevScalars* sc) {
   k_features_faces<<<nsm * 4, 128, 0, s>>>(P, S, id, L, X, pref, sc);
   int64_t ntiles = (L.cap + TILE - 1) / TILE;
-  int grid = (int)std::min<int64_t>(ntiles, nsm);
-  k_forward<<<grid, TILE, SMEM_FWD, s>>>(L.cap, L.count, X, m->wbf, m->prm, t, m->err, sc);
+  int grid = (int)std::min<int64_t>(ntiles, 2 * nsm);
+  k_forward<<<grid, NTHR, SMEM_FWD, s>>>(L.cap, L.count, X, m->wbf, m->prm, t, m->err, sc);
   k_to_pressure<<<nsm * 4, 128, 0, s>>>(L.cap, t, pref, nullptr, warm, sc, L.count);
 }
 cudaError_t mlp_prepare() { return mlp_set_smem(); }

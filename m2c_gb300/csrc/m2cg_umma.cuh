@@ -13,6 +13,12 @@
 //
 // D[M x N] (fp32, TMEM lanes = rows, columns = n) += A[M x K] * B[N x K]^T
 // with one tcgen05.mma per 16 elements of K.
+//
+// The same bytes are also the M-major (transposed) operand of R for K: an
+// M-major core matrix is 8 K-rows of 8 consecutive M elements, which is what a
+// core matrix above is with r as K and k as M.  The descriptor then gives as SBO
+// the step between 8-element groups of M (128 B) and as LBO the step between
+// 8-row groups of K ((width/8) * 128 B).
 #pragma once
 #include <cstdint>
 #include <cuda_bf16.h>
@@ -108,6 +114,18 @@ __device__ __forceinline__ void gemm_128xN(uint32_t d_tmem, const void* a, const
     mma_bf16(d_tmem, smem_desc(ia + kk * 256, 128, sbo), smem_desc(ib + kk * 256, 128, sbo), idesc,
              (accumulate || kk > 0) ? 1u : 0u);
   }
+}
+
+// D[128 x N] = A^T[128 x K] * B^T[N x K]^T for A and B stored as K rows of
+// wa / wb elements in the K-major layout above (rows along this product's K, a
+// multiple of 16; N = wb).  With wa < 128 accumulator rows wa..127 are whatever
+// lies up to (16 - wa / 8) * 128 bytes behind A.  Issued by one thread.
+__device__ __forceinline__ void gemm_tn_128xN(uint32_t d_tmem, const void* a, int wa, const void* b, int wb, int K) {
+  const uint32_t ia = smem_u32(a), ib = smem_u32(b);
+  const uint32_t la = (uint32_t)(wa >> 3) << 7, lb = (uint32_t)(wb >> 3) << 7;
+  const uint32_t idesc = idesc_bf16_f32(128, wb) | (1u << 15) | (1u << 16);   // A and B M-major
+  for (int kk = 0; kk < K / 16; kk++)
+    mma_bf16(d_tmem, smem_desc(ia + kk * 2 * la, la, 128), smem_desc(ib + kk * 2 * lb, lb, 128), idesc, kk > 0 ? 1u : 0u);
 }
 
 // ---- TMEM -> registers ------------------------------------------------------

@@ -240,3 +240,46 @@ def test_fv_step_with_warm_start():
     assert cw["riemann_iterations"] < 3 * cc["riemann_iterations"]
     warm.set_warm_start(None)
     cold.close(); warm.close(); net.close(); solver.close()
+
+
+@gpu
+@pytest.mark.parametrize("n", [1, 31, 127, 129])
+def test_tile_edges(n):
+    """Batches around one 128-row tile: outputs and the gradient's blocks
+    against the reference.  The operands are the same BF16 values on both sides
+    except where binary32 and binary64 activations round to different BF16
+    neighbours (2^-8 apart, a few per thousand of 64 terms a layer): 2^-8 / 4 of
+    the largest output, 2^-8 of a block's largest gradient, twice that where a
+    single row is not averaged."""
+    rng = np.random.default_rng(n)
+    net = ws.WarmStartMLP(7)
+    p = net.params.astype(np.float64)
+    for lo in (mlp_ref.OFF_B1, mlp_ref.OFF_B2, mlp_ref.OFF_B3):
+        p[lo:lo + 64] = rng.normal(0, 0.1, 64)
+    net.params = p.astype(np.float32)
+    p = net.params.astype(np.float64)
+    X = rng.normal(0, 1, (n, 16)).astype(np.float32)
+    t = rng.normal(0, 1, n).astype(np.float32)
+    out_ref, loss_ref, g_ref = mlp_ref.forward_backward(p, X, t)
+    assert np.max(np.abs(net.forward(X) - out_ref)) <= 2.0 ** -10 * max(1.0, np.max(np.abs(out_ref)))
+    g, loss = net.grad(X, t)
+    assert abs(loss - loss_ref) <= 2.0 ** -8 * loss_ref + 2.0 ** -18
+    for lo, hi in mlp_ref.BLOCKS.values():
+        assert np.max(np.abs(g[lo:hi] - g_ref[lo:hi])) <= 2.0 ** -7 * np.max(np.abs(g_ref[lo:hi]))
+    net.close()
+
+
+@gpu
+def test_rows_do_not_depend_on_their_tile():
+    """More tiles than resident blocks and a ragged end: every output is, bit
+    for bit, the one of the same row in a batch of its own tile alone."""
+    n = 128 * 700 + 5
+    rng = np.random.default_rng(2)
+    net = ws.WarmStartMLP(7)
+    X = rng.normal(0, 1, (n, 16)).astype(np.float32)
+    out = net.forward(X)
+    for lo in (0, 128 * 151, 128 * 303, 128 * 304, 128 * 608, 128 * 700):
+        rows = X[lo:lo + 128]
+        assert np.array_equal(out[lo:lo + 128], net.forward(rows))
+        assert np.array_equal(out[lo:lo + 1], net.forward(rows[:1]))
+    net.close()
