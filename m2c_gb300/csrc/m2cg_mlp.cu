@@ -22,9 +22,7 @@
 // descriptor, M-major from the same bytes.  SiLU' is kept in registers from
 // the forward pass, column sums are taken while the GEMMs run.  (With one row
 // per thread, element-wise stores, transposed copies and 320 shuffles per row
-// for the column sums, 32 training batches of 16,384 rows took 4.2 ms, 3.0 of
-// them in this kernel, and a forward pass over 262,144 rows 216 us; now 1.8 ms,
-// most of it the host's permutation of the rows, and 61 us.)
+// for the column sums, a training batch of 16,384 rows took 94 us and a forward pass over 262,144 rows 216 us; now 14 and 61 us.)
 //
 // Inputs are dimensionless groups of the two states relative to the
 // impedance-weighted pressure p_ref = (C_r p_l + C_l p_r) / (C_l + C_r), with
@@ -42,6 +40,7 @@
 #include <vector>
 #include <random>
 #include <algorithm>
+#include <mutex>
 #include "m2cg_internal.h"
 #include "m2cg_umma.cuh"
 
@@ -601,8 +600,21 @@ struct m2cg_mlp {
   int64_t n_data = 0;
   __nv_bfloat16* X = nullptr;
   float* y = nullptr;
-  int32_t* perm = nullptr;
+  int32_t* perm = nullptr;         // two epochs' permutations of the rows
+  // training: the next epoch's permutation is copied beside the current epoch
+  cudaStream_t copies = nullptr;
+  cudaEvent_t copied = nullptr;            // the last permutation has arrived
+  cudaEvent_t used[2] = {nullptr, nullptr};  // the epoch that read perm + k n is done
+  float* epoch_loss = nullptr;
+  int epoch_cap = 0;
+  // m2cg_mlp_predict's buffers, kept between calls up to WS_KEEP bytes (one
+  // call at a time holds them): six allocations and releases a call were 0.4 of
+  // 1.0 ms for 262,144 rows
+  std::mutex ws_lock;
+  void* ws = nullptr;
+  size_t ws_bytes = 0;
 };
+constexpr size_t WS_KEEP = size_t(256) << 20;
 
 namespace {
 m2cg_status mlp_check(m2cg_mlp* m) {
@@ -637,6 +649,10 @@ m2cg_status m2cg_mlp_create(uint64_t seed, m2cg_mlp** out) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&m->nsm, cudaDevAttrMultiProcessorCount, dev);
   if (cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&m->copies, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&m->copied, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&m->used[0], cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&m->used[1], cudaEventDisableTiming) != cudaSuccess ||
       cudaMalloc(&m->prm, NPARAM * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&m->grad, NPARAM * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&m->adam_m, NPARAM * sizeof(float)) != cudaSuccess ||
@@ -673,8 +689,11 @@ void m2cg_mlp_destroy(m2cg_mlp* m) {
   if (!m) return;
   if (m->stream) cudaStreamSynchronize(m->stream);
   for (void* p : {(void*)m->prm, (void*)m->grad, (void*)m->adam_m, (void*)m->adam_v, (void*)m->wbf, (void*)m->loss,
-                  (void*)m->err, (void*)m->X, (void*)m->y, (void*)m->perm})
+                  (void*)m->err, (void*)m->X, (void*)m->y, (void*)m->perm, (void*)m->epoch_loss, m->ws})
     if (p) cudaFree(p);
+  for (cudaEvent_t e : {m->copied, m->used[0], m->used[1]})
+    if (e) cudaEventDestroy(e);
+  if (m->copies) cudaStreamDestroy(m->copies);
   if (m->stream) cudaStreamDestroy(m->stream);
   delete m;
 }
@@ -752,7 +771,7 @@ m2cg_status m2cg_mlp_set_data(m2cg_mlp* m, int64_t n, const double* W, const dou
   double *dW, *dE, *dp;
   MCK(cudaMalloc(&m->X, n * NF * sizeof(__nv_bfloat16)));
   MCK(cudaMalloc(&m->y, n * sizeof(float)));
-  MCK(cudaMalloc(&m->perm, n * sizeof(int32_t)));
+  MCK(cudaMalloc(&m->perm, 2 * n * sizeof(int32_t)));
   MCK(cudaMalloc(&dW, n * 6 * sizeof(double)));
   MCK(cudaMalloc(&dE, n * 10 * sizeof(double)));
   MCK(cudaMalloc(&dp, n * sizeof(double)));
@@ -773,6 +792,13 @@ m2cg_status m2cg_mlp_train(m2cg_mlp* m, int32_t epochs, int32_t batch, float lr,
   if (m->n_data == 0) { m2cg_set_error("no training data (m2cg_mlp_set_data)"); return M2CG_ERR_INVALID_ARG; }
   const int64_t n = m->n_data;
   if (batch > n) batch = (int32_t)n;
+  if (epochs > m->epoch_cap) {
+    if (m->epoch_loss) cudaFree(m->epoch_loss);
+    m->epoch_loss = nullptr;
+    m->epoch_cap = 0;
+    MCK(cudaMalloc(&m->epoch_loss, epochs * sizeof(float)));
+    m->epoch_cap = epochs;
+  }
   std::vector<int32_t> perm(n);
   for (int64_t i = 0; i < n; i++) perm[i] = (int32_t)i;
   std::mt19937_64 rng(seed);
@@ -780,31 +806,38 @@ m2cg_status m2cg_mlp_train(m2cg_mlp* m, int32_t epochs, int32_t batch, float lr,
   MCK(cudaEventCreate(&e0));
   MCK(cudaEventCreate(&e1));
   MCK(cudaEventRecord(e0, m->stream));
+  if (epochs > 0) MCK(cudaMemsetAsync(m->epoch_loss, 0, epochs * sizeof(float), m->stream));
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+  // The host shuffles an epoch's rows (0.35 ms for 131,072) while the device
+  // works through the epoch before, from the other half of perm; the losses are
+  // read once, after the last epoch (4 epochs of 131,072 rows 1.84 -> 1.38 ms).
   for (int ep = 0; ep < epochs; ep++) {
     // cosine decay from lr to lr / 20 over the epochs
     const float lr_ep = lr * (0.05f + 0.95f * 0.5f * (1.f + std::cos(3.14159265f * (float)ep / (float)epochs)));
+    if (ep > 0) MCK(cudaEventSynchronize(m->copied));   // the last permutation has left perm
     std::shuffle(perm.begin(), perm.end(), rng);
-    MCK(cudaMemcpyAsync(m->perm, perm.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, m->stream));
-    MCK(cudaMemsetAsync(m->loss, 0, sizeof(float), m->stream));
+    int32_t* dperm = m->perm + (ep & 1) * n;
+    if (ep > 1) MCK(cudaStreamWaitEvent(m->copies, m->used[ep & 1], 0));
+    MCK(cudaMemcpyAsync(dperm, perm.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, m->copies));
+    MCK(cudaEventRecord(m->copied, m->copies));
+    MCK(cudaStreamWaitEvent(m->stream, m->copied, 0));
     for (int64_t b0 = 0; b0 + batch <= n; b0 += batch) {  // whole batches only
       k_train<<<(unsigned)((batch + TILE - 1) / TILE), NTHR, SMEM_TRAIN, m->stream>>>(
-          batch, m->perm + b0, m->X, m->y, m->wbf, m->prm, m->grad, m->loss, m->err);
+          batch, dperm + b0, m->X, m->y, m->wbf, m->prm, m->grad, m->epoch_loss + ep, m->err);
       m->step++;
       float bc1 = 1.f - std::pow(b1, (float)m->step), bc2 = 1.f - std::pow(b2, (float)m->step);
       k_adam<<<(NPARAM + 127) / 128, 128, 0, m->stream>>>(m->prm, m->grad, m->adam_m, m->adam_v, m->wbf, lr_ep, b1, b2,
                                                           eps, bc1, bc2);
     }
     MCK(cudaGetLastError());
-    if (loss_per_epoch) {
-      float l = 0.f;
-      MCK(cudaMemcpyAsync(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
-      MCK(cudaStreamSynchronize(m->stream));
-      loss_per_epoch[ep] = l / (float)((n / batch) * batch);
-    }
+    MCK(cudaEventRecord(m->used[ep & 1], m->stream));
   }
   MCK(cudaEventRecord(e1, m->stream));
+  if (loss_per_epoch && epochs > 0)
+    MCK(cudaMemcpyAsync(loss_per_epoch, m->epoch_loss, epochs * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
   MCK(cudaStreamSynchronize(m->stream));
+  if (loss_per_epoch)
+    for (int ep = 0; ep < epochs; ep++) loss_per_epoch[ep] /= (float)((n / batch) * batch);
   if (ms) MCK(cudaEventElapsedTime(ms, e0, e1));
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
@@ -861,15 +894,19 @@ m2cg_status m2cg_mlp_predict(m2cg_mlp* m, int64_t n, const double* W, const doub
                              float* kernel_ms) {
   if (!m || n < 0 || !W || !eos || !p_pred) { m2cg_set_error("null argument"); return M2CG_ERR_INVALID_ARG; }
   if (n == 0) return M2CG_OK;
-  double *dW, *dE, *dp;
-  __nv_bfloat16* dX;
-  float *dt, *dref;
-  MCK(cudaMalloc(&dW, n * 6 * sizeof(double)));
-  MCK(cudaMalloc(&dE, n * 10 * sizeof(double)));
-  MCK(cudaMalloc(&dp, n * sizeof(double)));
-  MCK(cudaMalloc(&dX, n * NF * sizeof(__nv_bfloat16)));
-  MCK(cudaMalloc(&dt, n * sizeof(float)));
-  MCK(cudaMalloc(&dref, n * sizeof(float)));
+  // per row: W, eos and p* (17 doubles), the network input (32 bytes), output and p_ref
+  const size_t bytes = (size_t)n * (17 * sizeof(double) + NF * sizeof(__nv_bfloat16) + 2 * sizeof(float));
+  std::lock_guard<std::mutex> lock(m->ws_lock);
+  if (bytes > m->ws_bytes) {
+    if (m->ws) cudaFree(m->ws);
+    m->ws = nullptr;
+    m->ws_bytes = 0;
+    MCK(cudaMalloc(&m->ws, bytes));
+    m->ws_bytes = bytes;
+  }
+  __nv_bfloat16* dX = (__nv_bfloat16*)m->ws;   // first: its rows are read in 16-byte words
+  double *dW = (double*)(dX + n * NF), *dE = dW + 6 * n, *dp = dE + 10 * n;
+  float *dt = (float*)(dp + n), *dref = dt + n;
   MCK(cudaMemcpyAsync(dW, W, n * 6 * sizeof(double), cudaMemcpyHostToDevice, m->stream));
   MCK(cudaMemcpyAsync(dE, eos, n * 10 * sizeof(double), cudaMemcpyHostToDevice, m->stream));
   cudaEvent_t e0, e1;
@@ -889,7 +926,11 @@ m2cg_status m2cg_mlp_predict(m2cg_mlp* m, int64_t n, const double* W, const doub
   if (kernel_ms) MCK(cudaEventElapsedTime(kernel_ms, e0, e1));
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  for (void* p : {(void*)dW, (void*)dE, (void*)dp, (void*)dX, (void*)dt, (void*)dref}) cudaFree(p);
+  if (m->ws_bytes > WS_KEEP) {
+    cudaFree(m->ws);
+    m->ws = nullptr;
+    m->ws_bytes = 0;
+  }
   return mlp_check(m);
 }
 
