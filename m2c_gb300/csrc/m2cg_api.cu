@@ -51,13 +51,13 @@ void mlp_warm_faces(m2cg_mlp*, cudaStream_t, int, const Params&, const StateSet&
                     __nv_bfloat16*, float*, float*, float*, const DevScalars*);
 cudaError_t mlp_prepare();
 void launch_hold(cudaStream_t, long long);
-void launch_riemann_batch(cudaStream_t, const Params&, const Mats*, int64_t, const double*, const int32_t*,
-                          const double*, const int32_t*, const double*, double*, int32_t*, double*, double*, int32_t*,
-                          int32_t*, double*, int, int, int, const double*);
+int launch_riemann_batch(cudaStream_t, const Params&, const Mats*, int64_t, const double*, const int32_t*,
+                         const double*, const int32_t*, const double*, double*, int32_t*, double*, double*, int32_t*,
+                         int32_t*, double*, int, int, int, const double*, int, int32_t*, unsigned long long*);
 void launch_flux_batch(cudaStream_t, const Params&, int64_t, const int32_t*, const double*, const double*,
                        const int32_t*, double*);
-void launch_riemann_batch_eos(cudaStream_t, const Params&, int64_t, const double*, const double*, const double*,
-                              double*, int32_t*, int32_t*, double*, int, int, int);
+int launch_riemann_batch_eos(cudaStream_t, const Params&, int64_t, const double*, const double*, const double*,
+                             double*, int32_t*, int32_t*, double*, int, int, int, int, int32_t*, unsigned long long*);
 }  // namespace m2cg
 
 using namespace m2cg;
@@ -1145,13 +1145,14 @@ static m2cg_status batch_reserve(m2cg_ctx* x, int64_t n) {
   if (n <= x->batch_n) return M2CG_OK;
   for (void* p : x->batch) cudaFree(p);
   x->batch.clear();
-  // Vm Vp Vs Vsm Vsp (5 each), dir (3), warm (1) doubles; idm idp id iters err ints
+  // Vm Vp Vs Vsm Vsp (5 each), dir (3), warm (1) doubles; idm idp id iters err and
+  // the unfinished problems' list ints
   size_t doubles = (size_t)n * (5 * 5 + 3 + 1);
   void* d = nullptr;
   CK(cudaMalloc(&d, doubles * sizeof(double)));
   x->batch.push_back(d);
   void* q = nullptr;
-  CK(cudaMalloc(&q, (size_t)n * 5 * sizeof(int32_t)));
+  CK(cudaMalloc(&q, (size_t)n * 6 * sizeof(int32_t)));
   x->batch.push_back(q);
   x->batch_n = n;
   if (!x->batch_scratch) {
@@ -1188,9 +1189,9 @@ m2cg_status m2cg_riemann_batch(m2cg_ctx* x, int64_t n, const double* Vm, const i
   CK(cudaMemcpyAsync(ddir, dir, n * 3 * sizeof(double), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(didm, idm, n * sizeof(int32_t), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(didp, idp, n * sizeof(int32_t), cudaMemcpyHostToDevice, s));
-  launch_riemann_batch(s, x->P, x->d_mats, n, dVm, didm, dVp, didp, ddir, dVs, did, dVsm, dVsp, dit, derr,
-                       x->batch_scratch, x->path_cap, (int)(x->batch_threads / 128), 128, nullptr);
-  x->launches++;
+  x->launches += launch_riemann_batch(s, x->P, x->d_mats, n, dVm, didm, dVp, didp, ddir, dVs, did, dVsm, dVsp, dit, derr,
+                                      x->batch_scratch, x->path_cap, (int)(x->batch_threads / 128), 128, nullptr,
+                                      x->eval_limit, I + 5 * cap, x->strag_count);
   CK(cudaMemcpyAsync(Vs, dVs, n * 5 * sizeof(double), cudaMemcpyDeviceToHost, s));
   CK(cudaMemcpyAsync(Vsm, dVsm, n * 5 * sizeof(double), cudaMemcpyDeviceToHost, s));
   CK(cudaMemcpyAsync(Vsp, dVsp, n * 5 * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -1232,10 +1233,10 @@ m2cg_status m2cg_riemann_batch_eos(m2cg_ctx* x, int64_t n, const double* W, cons
   // start cost evaluations: 6.43 against 6.00 for one network, cold 6.87)
   Params Pb = x->P;
   if (!getenv("M2CG_WARM_GATE")) Pb.rp.warm_gate = 0.0;
-  launch_riemann_batch_eos(s, Pb, n, dW, dE, warm_p ? dwarm : nullptr, dout, dit, derr, x->batch_scratch,
-                           x->path_cap, (int)(x->batch_threads / 128), 128);
+  x->launches += launch_riemann_batch_eos(s, Pb, n, dW, dE, warm_p ? dwarm : nullptr, dout, dit, derr,
+                                          x->batch_scratch, x->path_cap, (int)(x->batch_threads / 128), 128,
+                                          x->eval_limit, I + 2 * n, x->strag_count);
   CK(cudaEventRecord(e1, s));
-  x->launches++;
   CK(cudaMemcpyAsync(out, dout, n * 4 * sizeof(double), cudaMemcpyDeviceToHost, s));
   if (iters) CK(cudaMemcpyAsync(iters, dit, n * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
   if (err) CK(cudaMemcpyAsync(err, derr, n * sizeof(int32_t), cudaMemcpyDeviceToHost, s));

@@ -196,7 +196,7 @@ __device__ __forceinline__ void init_coop(ExactRiemannCoop& rs, const Mats* md, 
 // Which solver a pass uses: one problem per warp (cooperative) while there are
 // no more problems than warps in the launch, else one per thread.  Measured on
 // GB300 with 1,216 warps: 733 faces of the 2D explosion 1.6 ms against 4.8 ms a
-// pass, 64 faces of the tube 0.42 against 0.50 ms; 5,760 faces of a stirred
+// pass, 64 faces of the tube 0.34 against 0.50 ms; 5,760 faces of a stirred
 // bubble (five rounds) 3.4 against 0.9 ms.
 __device__ __forceinline__ bool coop_pass(int64_t n) { return n <= (int64_t)gridDim.x * (blockDim.x >> 5); }
 
@@ -462,29 +462,61 @@ cudaError_t riemann_stragglers_ens_reserve(size_t bytes) {
   return cudaFuncSetAttribute(k_riemann_stragglers_ens, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-// Batched independent problems (device arrays, AoS rows of 5 / 3): one per
-// warp or one per thread (coop_pass; two kernels, since one that held both
-// solvers spilt 3.4 kB a thread and took 9.8 ms instead of 9.3 for 20,000 problems).
+// How a batch of n problems (host count) is dealt out.  Up to one problem per
+// warp of the launch: cooperative solves of all of them.  More: a first pass of
+// one problem per thread with the step's evaluation budget, which lists the
+// solves that exhaust it (stalled secants, 410 evaluations and more, among them
+// chains of seconds); these are solved from the start, one per warp while there
+// are warps, else one per thread -- two launches, of which the device count lets
+// one work.  (Two kernels, since one that held both solvers spilt 3.4 kB a
+// thread and took 9.8 ms instead of 9.3 ms for 20,000 problems.)  65,536 random
+// pairs with 570 unfinished ones: 17.8 s with the second pass, 22.1 s without.
+struct BatchPass {
+  const int32_t* list;                      // the problems to solve (NULL: 0 .. n - 1) ...
+  const unsigned long long* list_n;         // ... and their number
+  int eval_limit;                           // first pass: budget (0: none), and where
+  int32_t* strag;                           // the unfinished problems go
+  unsigned long long* strag_n;
+};
+// Calls f(q) for this thread's (or warp's) problems; f returns 2 for an
+// unfinished solve.
+template <bool Coop, class F>
+__device__ __forceinline__ void batch_problems(int64_t n, const BatchPass& bp, F f) {
+  const int64_t T = (int64_t)gridDim.x * blockDim.x, W = T >> 5;
+  if (bp.list) {
+    n = min(n, (int64_t)*bp.list_n);
+    if (Coop != (n <= W)) return;
+  }
+  const int64_t k0 = Coop ? (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x : (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (int64_t k = k0; k < n; k += T) {
+    const int64_t q = bp.list ? bp.list[k] : k;
+    if (f(q) == 2) bp.strag[atomicAdd(bp.strag_n, 1ull)] = (int32_t)q;   // each problem is listed once
+  }
+}
+
+// Batched independent problems (device arrays, AoS rows of 5 / 3).
 template <bool Coop>
 __global__ void k_riemann_batch(const Mats* __restrict__ md, RiemannPrm rp, int64_t n, const double* __restrict__ Vm,
                                 const int32_t* __restrict__ idm, const double* __restrict__ Vp,
                                 const int32_t* __restrict__ idp, const double* __restrict__ dir, double* Vs,
                                 int32_t* id, double* Vsm, double* Vsp, int32_t* iters, int32_t* err, double* scratch,
-                                int path_cap, const double* warm) {
+                                int path_cap, const double* warm, BatchPass bp) {
   int64_t T = (int64_t)gridDim.x * blockDim.x;
   int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   ExactRiemannDevT<Coop> rs;
-  const int64_t w = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;   // < T / 32
-  if constexpr (Coop) init_coop(rs, md, rp, scratch, path_cap, w);
+  if constexpr (Coop) init_coop(rs, md, rp, scratch, path_cap, (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x);
   else init_solver(rs, md, rp, scratch, path_cap, tid, T);
-  for (int64_t q = Coop ? w : tid; q < n; q += T) {
+  rs.eval_limit = bp.eval_limit;
+  batch_problems<Coop>(n, bp, [&](int64_t q) {
     int oid = 0;
     rs.warm_p = warm ? warm[q] : 0.0;
     int e = rs.solve(&dir[q * 3], &Vm[q * 5], idm[q], &Vp[q * 5], idp[q], &Vs[q * 5], oid, &Vsm[q * 5], &Vsp[q * 5]);
+    if (e == 2) return 2;
     id[q] = oid;
     if (iters) iters[q] = rs.evals;
     if (err) err[q] = e;
-  }
+    return 0;
+  });
 }
 
 // DevMat of a stiffened-gas / Noble-Abel stiffened-gas material from
@@ -505,7 +537,7 @@ __device__ __forceinline__ void make_devmat(const double* e, DevMat& d) {
 }
 
 template <class Solver>
-__device__ __forceinline__ void riemann_eos_problem(Solver& rs, Mats& mats, int64_t q, const double* __restrict__ W,
+__device__ __forceinline__ int riemann_eos_problem(Solver& rs, Mats& mats, int64_t q, const double* __restrict__ W,
                                                     const double* __restrict__ E, const double* __restrict__ warm,
                                                     const double* dir, double* out, int32_t* iters, int32_t* err) {
   make_devmat(&E[q * 10], mats.m[0]);
@@ -516,12 +548,14 @@ __device__ __forceinline__ void riemann_eos_problem(Solver& rs, Mats& mats, int6
   int oid = 0;
   rs.warm_p = warm ? warm[q] : 0.0;
   const int e = rs.solve(dir, Vm, 0, Vp, 1, Vs, oid, Vsm, Vsp);
+  if (e == 2) return 2;
   out[q * 4 + 0] = Vsm[4];
   out[q * 4 + 1] = Vsm[1];
   out[q * 4 + 2] = Vsm[0];
   out[q * 4 + 3] = Vsp[0];
   if (iters) iters[q] = rs.evals;
   if (err) err[q] = e;
+  return 0;
 }
 
 // Independent 1D problems, each with its own material pair (the warm-start
@@ -531,16 +565,16 @@ __device__ __forceinline__ void riemann_eos_problem(Solver& rs, Mats& mats, int6
 template <bool Coop>
 __global__ void k_riemann_batch_eos(RiemannPrm rp, int64_t n, const double* __restrict__ W,
                                     const double* __restrict__ E, const double* __restrict__ warm, double* out,
-                                    int32_t* iters, int32_t* err, double* scratch, int path_cap) {
+                                    int32_t* iters, int32_t* err, double* scratch, int path_cap, BatchPass bp) {
   int64_t T = (int64_t)gridDim.x * blockDim.x;
   int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   Mats mats;
   const double dir[3] = {1.0, 0.0, 0.0};
   ExactRiemannDevT<Coop> rs;
-  const int64_t w = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;   // < T / 32
-  if constexpr (Coop) init_coop(rs, &mats, rp, scratch, path_cap, w);
+  if constexpr (Coop) init_coop(rs, &mats, rp, scratch, path_cap, (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x);
   else init_solver(rs, &mats, rp, scratch, path_cap, tid, T);
-  for (int64_t q = Coop ? w : tid; q < n; q += T) riemann_eos_problem(rs, mats, q, W, E, warm, dir, out, iters, err);
+  rs.eval_limit = bp.eval_limit;
+  batch_problems<Coop>(n, bp, [&](int64_t q) { return riemann_eos_problem(rs, mats, q, W, E, warm, dir, out, iters, err); });
 }
 
 __global__ void k_flux_batch(Params P, int64_t n, const int32_t* __restrict__ dir, const double* __restrict__ Vm,
@@ -586,19 +620,37 @@ void launch_hold(cudaStream_t s, long long cycles) { k_hold<<<1, 32, 0, s>>>(cyc
 cudaError_t riemann_stragglers_reserve(size_t bytes) {
   return cudaFuncSetAttribute(k_riemann_stragglers, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
-void launch_riemann_batch(cudaStream_t s, const Params& P, const Mats* md, int64_t n, const double* Vm, const int32_t* idm,
-                          const double* Vp, const int32_t* idp, const double* dir, double* Vs, int32_t* id,
-                          double* Vsm, double* Vsp, int32_t* iters, int32_t* err, double* scratch, int path_cap,
-                          int blocks, int threads, const double* warm) {
-  const auto k = n <= (int64_t)blocks * (threads / 32) ? k_riemann_batch<true> : k_riemann_batch<false>;
-  k<<<blocks, threads, 0, s>>>(md, P.rp, n, Vm, idm, Vp, idp, dir, Vs, id, Vsm, Vsp, iters, err,
-                                             scratch, path_cap, warm);
+// f(coop, pass) launches one pass; returns the number of launches.
+template <class F>
+static int batch_passes(cudaStream_t s, int64_t n, int blocks, int threads, int eval_limit, int32_t* strag,
+                        unsigned long long* strag_n, F f) {
+  if (n <= (int64_t)blocks * (threads / 32)) { f(true, BatchPass{}); return 1; }
+  if (eval_limit <= 0) { f(false, BatchPass{}); return 1; }
+  cudaMemsetAsync(strag_n, 0, sizeof(unsigned long long), s);
+  f(false, BatchPass{nullptr, nullptr, eval_limit, strag, strag_n});
+  f(true, BatchPass{strag, strag_n, 0, nullptr, nullptr});
+  f(false, BatchPass{strag, strag_n, 0, nullptr, nullptr});
+  return 3;
 }
-void launch_riemann_batch_eos(cudaStream_t s, const Params& P, int64_t n, const double* W, const double* E,
-                              const double* warm, double* out, int32_t* iters, int32_t* err, double* scratch,
-                              int path_cap, int blocks, int threads) {
-  const auto k = n <= (int64_t)blocks * (threads / 32) ? k_riemann_batch_eos<true> : k_riemann_batch_eos<false>;
-  k<<<blocks, threads, 0, s>>>(P.rp, n, W, E, warm, out, iters, err, scratch, path_cap);
+int launch_riemann_batch(cudaStream_t s, const Params& P, const Mats* md, int64_t n, const double* Vm, const int32_t* idm,
+                         const double* Vp, const int32_t* idp, const double* dir, double* Vs, int32_t* id,
+                         double* Vsm, double* Vsp, int32_t* iters, int32_t* err, double* scratch, int path_cap,
+                         int blocks, int threads, const double* warm, int eval_limit, int32_t* strag,
+                         unsigned long long* strag_n) {
+  return batch_passes(s, n, blocks, threads, eval_limit, strag, strag_n, [&](bool coop, const BatchPass& bp) {
+    const auto k = coop ? k_riemann_batch<true> : k_riemann_batch<false>;
+    k<<<blocks, threads, 0, s>>>(md, P.rp, n, Vm, idm, Vp, idp, dir, Vs, id, Vsm, Vsp, iters, err, scratch, path_cap,
+                                 warm, bp);
+  });
+}
+int launch_riemann_batch_eos(cudaStream_t s, const Params& P, int64_t n, const double* W, const double* E,
+                             const double* warm, double* out, int32_t* iters, int32_t* err, double* scratch,
+                             int path_cap, int blocks, int threads, int eval_limit, int32_t* strag,
+                             unsigned long long* strag_n) {
+  return batch_passes(s, n, blocks, threads, eval_limit, strag, strag_n, [&](bool coop, const BatchPass& bp) {
+    const auto k = coop ? k_riemann_batch_eos<true> : k_riemann_batch_eos<false>;
+    k<<<blocks, threads, 0, s>>>(P.rp, n, W, E, warm, out, iters, err, scratch, path_cap, bp);
+  });
 }
 void launch_flux_batch(cudaStream_t s, const Params& P, int64_t n, const int32_t* dir, const double* Vm,
                        const double* Vp, const int32_t* id, double* F) {

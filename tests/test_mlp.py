@@ -283,3 +283,18 @@ def test_rows_do_not_depend_on_their_tile():
         assert np.array_equal(out[lo:lo + 128], net.forward(rows))
         assert np.array_equal(out[lo:lo + 1], net.forward(rows[:1]))
     net.close()
+
+
+@gpu
+def test_batch_passes_equal_one_pass():
+    """More problems than warps (1,217 against 1,216 on 152 SMs): a budgeted
+    first pass and a second one for the unfinished problems give, bit for bit,
+    what calls of fewer problems (one pass without a budget) give."""
+    W, E = ws.sample_problems(1217, 11)
+    solver = ws.BatchSolver(1e-10)
+    whole = solver.solve(W, E)
+    parts = [solver.solve(W[lo:lo + 400], E[lo:lo + 400]) for lo in range(0, 1217, 400)]
+    for k in ("pstar", "iters", "err"):
+        assert np.array_equal(whole[k], np.concatenate([q[k] for q in parts]), equal_nan=k == "pstar"), k
+    assert (whole["iters"] > 24).any()   # the second pass had work
+    solver.close()
