@@ -41,31 +41,18 @@ sys.path.insert(0, ROOT)
 METRIC = "FP64 cell-stage updates/s (1 GB300) + Newton iters/interface, MLP vs cold start @1e-10"
 UNIT = "cell-stage/s"
 MEASURED_PEAKS = os.path.join(ROOT, "MEASURED_PEAKS.json")
-# FP64-pipe instructions per cell of each stage kernel (warp instructions x 32 /
-# cells), binary64 FLOPs per cell (2 DFMA + DMUL + DADD, active lanes), and DRAM
-# bytes per cell, from the ncu capture of the 128^3 case in
-# profiles/fp64_stage_kernels_shock_bubble_128.txt; the counts per cell do not
-# depend on the grid size (the same code path runs on every cell or face).
+# FP64-pipe instructions per cell and stage of each stage kernel (warp
+# instructions x 32 / cells), binary64 FLOPs per cell (2 DFMA + DMUL + DADD,
+# thread level), and DRAM bytes per cell, from the ncu capture of the 128^3 case
+# in profiles/stage_kernels_shock_bubble_128.txt (mean of the two stages); the
+# counts per cell do not depend on the grid size (the same code path runs on
+# every cell or face).
 FP64_PROFILE = {
-    "reconstruct": {"fp64_pipe_inst_per_cell": 279.7, "fp64_flop_per_cell": 131.1, "dram_bytes_per_cell": 269.0},
-    "face_flux": {"fp64_pipe_inst_per_cell": 617.5, "fp64_flop_per_cell": 706.8, "dram_bytes_per_cell": 363.0},
-    "update": {"fp64_pipe_inst_per_cell": 104.5, "fp64_flop_per_cell": 122.6, "dram_bytes_per_cell": 293.9},
+    "reconstruct": {"fp64_pipe_inst_per_cell": 63.5, "fp64_flop_per_cell": 91.1, "dram_bytes_per_cell": 275.6},
+    "face_flux": {"fp64_pipe_inst_per_cell": 176.5, "fp64_flop_per_cell": 211.4, "dram_bytes_per_cell": 363.3},
+    "update": {"fp64_pipe_inst_per_cell": 81.5, "fp64_flop_per_cell": 103.6, "dram_bytes_per_cell": 295.5},
 }
-# The fused reconstruction + face-flux kernel (k_recon_flux_tile, the default
-# path) and the stage update: FP64-pipe slots, binary64 FLOPs (2 DFMA + DMUL +
-# DADD, thread level) and DRAM bytes per cell and launch, ncu on the 128^3 case
-# (profiles/k_recon_flux_tile_shock_bubble_128.txt; mean of the two stages).
-FP64_PROFILE_FUSED = {
-    "face_flux": {"fp64_pipe_inst_per_cell": 610.7, "fp64_flop_per_cell": 645.7, "dram_bytes_per_cell": 150.8},
-    "update": {"fp64_pipe_inst_per_cell": 104.0, "fp64_flop_per_cell": 117.5, "dram_bytes_per_cell": 295.3},
-}
-# DRAM bytes of one whole step graph of the 128^3 case (read + write, ncu
-# --graph-profiling graph) per cell-stage: split kernels
-# (profiles/reinit_graph_shock_bubble_128.txt) and fused
-# (profiles/step_graph_shock_bubble_128.txt).
-STEP_DRAM_BYTES_PER_CELL_STAGE = (2388.8e6 + 1971.9e6) / (128 ** 3 * 2)
-STEP_DRAM_BYTES_PER_CELL_STAGE_FUSED = (1305.2e6 + 956.4e6) / (128 ** 3 * 2)
-# Algorithmic bytes per cell-stage of the fused ideal (binary64 V and phi, int32
+# Algorithmic bytes per cell-stage of the ideal (binary64 V and phi, int32
 # ID, ideal halo reuse): a first stage reads W = (V, phi) 48 B + ID 4 B and
 # writes 48 B = 100 B; a later stage also reads W^n = 148 B.  Mean over the
 # integrator's stages: forward Euler 100, RK2 124, RK3 132.
@@ -516,26 +503,23 @@ def run_gb300(args):
              "riemann_stragglers"]
     phase = {n: float(v) / nph for n, v in zip(names, ph)}
     dom = max(("reconstruct", "face_flux", "update"), key=lambda n: phase[n])
-    fused = phase["reconstruct"] == 0.0   # the fused reconstruction + face-flux kernel ran
-    profile = FP64_PROFILE_FUSED if fused else FP64_PROFILE
     pk, pk_kind = peaks()
     per_launch_ms = phase[dom] / stages
-    prof = profile.get(dom)
+    prof = FP64_PROFILE.get(dom)
     # achieved = algorithmic bytes of the cell-stages one launch advances (the
-    # fused ideal's bytes per cell-stage x cells) / the launch's event-timed
+    # ideal's bytes per cell-stage x cells) / the launch's event-timed
     # duration; traffic = the kernel's own DRAM bytes per launch (ncu, 128^3
     # case, scaled by cells)
     alg = ALG_BYTES_PER_CELL_STAGE[stages]
     achieved_gbs = alg * cells / (per_launch_ms * 1e-3) / 1e9
-    # the kernels' own (unfused) bytes per cell: what each reads and writes
+    # the kernels' own bytes per cell: what each reads and writes
     #   reconstruct: V 40 + ID 4 in, 6 face states 240 out                     = 284
     #   face_flux:   2 face states per face (3 faces: 240) + IDs 8 in, 3 fluxes 120 out = 368
     #   update:      6 fluxes 240 + Un/Us 80 + ID 4 + phi 8 + V 40 in, V 40 + phi 8 + U 40 out = 460
-    #   fused reconstruction + face flux: V 40 + ID 4 in, 3 fluxes 120 out          = 164
-    own_bytes = {"reconstruct": 284, "face_flux": 164 if fused else 368, "update": 460}
+    own_bytes = {"reconstruct": 284, "face_flux": 368, "update": 460}
     step_ms = t_ms / args.steps
-    step_dram = (STEP_DRAM_BYTES_PER_CELL_STAGE_FUSED if fused else STEP_DRAM_BYTES_PER_CELL_STAGE)
-    roof = {"bound": "hbm", "kernel": "recon_flux_tile (fused)" if fused and dom == "face_flux" else dom,
+    step_dram = sum(v["dram_bytes_per_cell"] for v in FP64_PROFILE.values())
+    roof = {"bound": "hbm", "kernel": dom,
             "achieved": achieved_gbs, "peak": pk["hbm_gbs"], "unit": "GB/s",
             "frac": achieved_gbs / pk["hbm_gbs"],
             "traffic": prof["dram_bytes_per_cell"] * cells if prof else None, "peak_source": pk_kind,
@@ -546,8 +530,8 @@ def run_gb300(args):
                      "dram_over_alg": step_dram / alg if step_dram else None,
                      "achieved_gbs": alg * cells * stages / (step_ms * 1e-3) / 1e9,
                      "frac": alg * cells * stages / (step_ms * 1e-3) / 1e9 / pk["hbm_gbs"],
-                     "dram_source": "ncu whole-graph capture of the 128^3 step (profiles/" +
-                                    ("step_graph_shock_bubble_128.txt)" if fused else "reinit_graph_shock_bubble_128.txt)")}}
+                     "dram_source": "ncu, the stage kernels of the 128^3 step "
+                                    "(profiles/stage_kernels_shock_bubble_128.txt)"}}
     # the binding bound of the stage kernels: GB300's FP64 pipe.  Peak = binary64
     # FMAs/s of this GPU measured now (m2cg_fp64_peak); achieved = the kernel's
     # FP64-pipe instructions per launch (per-cell count from the ncu profile x
@@ -555,7 +539,7 @@ def run_gb300(args):
     # FP64-pipe instructions of one cell-stage summed over the stage kernels.
     dfma = C.c_double()
     fp64 = None
-    slots = sum(v["fp64_pipe_inst_per_cell"] for v in profile.values())
+    slots = sum(v["fp64_pipe_inst_per_cell"] for v in FP64_PROFILE.values())
     if lib.m2cg_fp64_peak(1 << 15, C.byref(dfma), None) == 0 and prof:
         inst = prof["fp64_pipe_inst_per_cell"] * cells / (per_launch_ms * 1e-3)
         flops = prof["fp64_flop_per_cell"] * cells / (per_launch_ms * 1e-3)
@@ -565,9 +549,9 @@ def run_gb300(args):
                 "fp64_pipe_inst_per_cell": prof["fp64_pipe_inst_per_cell"],
                 "fp64_flop_per_cell": prof["fp64_flop_per_cell"],
                 "peak_source": "measured now: m2cg_fp64_peak (independent binary64 FMA chains)",
-                "counts_source": "ncu, profiles/" + ("k_recon_flux_tile_shock_bubble_128.txt" if fused
-                                                     else "fp64_stage_kernels_shock_bubble_128.txt"),
-                "step_fp64_pipe_inst_per_cell_stage": {k: v["fp64_pipe_inst_per_cell"] for k, v in profile.items()},
+                "counts_source": "ncu, profiles/stage_kernels_shock_bubble_128.txt",
+                "step_fp64_pipe_inst_per_cell_stage": {k: v["fp64_pipe_inst_per_cell"]
+                                                       for k, v in FP64_PROFILE.items()},
                 "ceiling_cell_stage_per_s": dfma.value / slots,
                 "value_over_ceiling": value / (dfma.value / slots)}
     elif dfma.value > 0:

@@ -580,8 +580,7 @@ static __device__ __noinline__ double gen_minmod(double alpha, double dq0, doubl
 // van Albada on the integer pipe (if_van_albada: 182 cycles per warp with one
 // FP64 multiplication, against 666 for the FP64 form with its ten); products
 // next to the 1e-16 threshold and special operands take the FP64 form.  Every
-// operation is pinned (no contraction), so the split and fused stage kernels
-// produce the same bits.
+// operation is pinned (no contraction), so every caller gets the same bits.
 static __device__ __noinline__ double van_albada_fp64(double dq0, double dq1) {
   double pr = __dmul_rn(dq0, dq1);
   if (le_zero_bits(pr) || abs_lt_bits(pr, 1e-16)) return 0.0;
