@@ -134,7 +134,7 @@ struct m2cg_ctx {
   size_t sreserve = 0;         // their dynamic shared-memory request
   int32_t* strag = nullptr;
   unsigned long long* strag_count = nullptr;
-  int* stalled = nullptr;      // per stage: did the stage before it leave stalled solves (Gate)
+  int* stalled = nullptr;      // GATE_WORDS flags: did the stage before leave stalled solves (Gate)
   cudaEvent_t ev_a = nullptr;  // end of the first pass
   long long hold_cycles = 40000;  // ~20 us head start for the straggler blocks
   // learned warm start (m2cg_set_warm_start): per interface face features,
@@ -322,7 +322,7 @@ static m2cg_status ctx_alloc(m2cg_ctx* x) {
   else CK(x->alloc(&x->scratch, (size_t)6 * x->path_cap * x->rblocks * x->rthreads));
   CK(x->alloc(&x->strag, L.cap));
   CK(x->alloc(&x->strag_count, 1));
-  CK(x->alloc(&x->stalled, 3));
+  CK(x->alloc(&x->stalled, GATE_WORDS));
   x->sblocks = std::max(1, std::min(x->nsm, x->rblocks / 2));   // 256-thread blocks on the first pass's scratch
   // tuning overrides: M2CG_RIEMANN_EVAL_LIMIT (first-pass budget, 0 = none),
   // M2CG_RIEMANN_STRAGGLER_SMS (blocks of the second pass, one SM each),
@@ -441,7 +441,7 @@ static int64_t enqueue_stage(m2cg_ctx* x, int stage, bool last, const StateSet& 
   PHASE_ON(PH_RIEMANN_B, x->stream2,
            launch_riemann_stragglers(x->stream2, P, x->d_mats, in, x->id, x->d_fs, x->L, stage == 0, x->scratch,
                                      x->path_cap, x->sblocks, x->sreserve, x->strag, x->strag_count, warm, x->cnt,
-                                     x->sc, x->strag_lanes, &x->stalled[(stage + 1) % rk_stages(x)]));
+                                     x->sc, x->strag_lanes, &x->stalled[gate_word_out(stage, rk_stages(x))]));
   cudaEventRecord(x->ev_join, x->stream2);
   n += 2;
   n += enqueue_recon_flux(x, s, in, !after_recon, Gate{&x->stalled[stage], 0});
@@ -449,6 +449,8 @@ static int64_t enqueue_stage(m2cg_ctx* x, int stage, bool last, const StateSet& 
   if (x->hold_cycles > 0) { launch_hold(s, x->hold_cycles); n++; }
   n += enqueue_recon_flux(x, s, in, !after_recon, Gate{&x->stalled[stage], 1});
   cudaStreamWaitEvent(s, x->ev_join, 0);
+  if (rk_stages(x) == 1)
+    cudaMemcpyAsync(&x->stalled[0], &x->stalled[gate_word_out(0, 1)], sizeof(int), cudaMemcpyDeviceToDevice, s);
   StageArgs A = stage_args(x, stage, last, in, out);
   if (P.ls_fv) {   // the finite-volume level-set residual of the stage input
     PHASE(PH_UPDATE, launch_ls_residual(s, P, in, x->rphi)); n++;
@@ -1513,7 +1515,7 @@ static m2cg_status ens_enqueue_step(m2cg_ensemble* e, int64_t* nl) {
                                e->strag_count);
       cudaEventRecord(e->ev_a, e->stream2);
       launch_riemann_ens_stragglers(e->stream2, ra_d, e->scratch, e->path_cap, e->strag, e->strag_count, e->sblocks,
-                                    e->sreserve, e->strag_lanes, &e->stalled[(stage + 1) % nst]);
+                                    e->sreserve, e->strag_lanes, &e->stalled[gate_word_out(stage, nst)]);
       cudaEventRecord(e->ev_join, e->stream2);
     }
     recon_flux(Gate{&e->stalled[stage], 0});
@@ -1641,7 +1643,8 @@ m2cg_status m2cg_ensemble_create(const m2cg_config* cfgs, int32_t n, m2cg_ensemb
       cudaEventCreate(&e->e0) != cudaSuccess || cudaEventCreate(&e->e1) != cudaSuccess ||
       cudaMalloc(&e->scratch, (size_t)6 * e->path_cap * e->rblocks * 128 * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&e->strag_count, sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMalloc(&e->stalled, 3 * sizeof(int)) != cudaSuccess || cudaMemset(e->stalled, 0, 3 * sizeof(int)) != cudaSuccess ||
+      cudaMalloc(&e->stalled, GATE_WORDS * sizeof(int)) != cudaSuccess ||
+      cudaMemset(e->stalled, 0, GATE_WORDS * sizeof(int)) != cudaSuccess ||
       cudaMalloc(&e->off, (size_t)(n + 1) * sizeof(int64_t)) != cudaSuccess) {
     set_err("ensemble set-up failed: %s", cudaGetErrorString(cudaGetLastError()));
     m2cg_ensemble_destroy(e);

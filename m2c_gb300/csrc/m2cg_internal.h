@@ -130,6 +130,19 @@ struct Gate {
   int want;
   M2CG_DEV bool closed() const { return flag && *flag != want; }
 };
+// The flags: stage k's launches read word k.  The stragglers of stage k write
+// their result while those launches still run, so it goes to a word that none of
+// them reads: the next stage's, and for a scheme of one stage word 1, which the
+// main stream copies to word 0 once the stragglers are done.
+constexpr int GATE_WORDS = 3;
+constexpr int gate_word_out(int stage, int stages) { return stages > 1 ? (stage + 1) % stages : 1; }
+constexpr bool gate_words_apart() {
+  for (int stages = 1; stages <= 3; stages++)
+    for (int k = 0; k < stages; k++)
+      if (gate_word_out(k, stages) == k || gate_word_out(k, stages) >= GATE_WORDS) return false;
+  return true;
+}
+static_assert(gate_words_apart(), "a stage's stragglers write a flag that the stage's own launches read");
 
 // A primitive state set: rho, u, v, w, p, phi (SoA, ghosted).
 struct StateSet {
