@@ -50,7 +50,7 @@ cudaError_t riemann_stragglers_reserve(size_t bytes);
 void mlp_warm_faces(m2cg_mlp*, cudaStream_t, int, const Params&, const StateSet&, const int32_t*, const IfaceList&,
                     __nv_bfloat16*, float*, float*, float*, const DevScalars*);
 cudaError_t mlp_prepare();
-void launch_hold(cudaStream_t, long long);
+void launch_hold(cudaStream_t, long long, const Gate&);
 int launch_riemann_batch(cudaStream_t, const Params&, const Mats*, int64_t, const double*, const int32_t*,
                          const double*, const int32_t*, const double*, double*, int32_t*, double*, double*, int32_t*,
                          int32_t*, double*, int, int, int, const double*, int, int32_t*, unsigned long long*);
@@ -446,8 +446,9 @@ static int64_t enqueue_stage(m2cg_ctx* x, int stage, bool last, const StateSet& 
   n += 2;
   n += enqueue_recon_flux(x, s, in, !after_recon, Gate{&x->stalled[stage], 0});
   cudaStreamWaitEvent(s, x->ev_a, 0);
-  if (x->hold_cycles > 0) { launch_hold(s, x->hold_cycles); n++; }
-  n += enqueue_recon_flux(x, s, in, !after_recon, Gate{&x->stalled[stage], 1});
+  const Gate after_pass{&x->stalled[stage], 1};
+  if (x->hold_cycles > 0) { launch_hold(s, x->hold_cycles, after_pass); n++; }
+  n += enqueue_recon_flux(x, s, in, !after_recon, after_pass);
   cudaStreamWaitEvent(s, x->ev_join, 0);
   if (rk_stages(x) == 1)
     cudaMemcpyAsync(&x->stalled[0], &x->stalled[gate_word_out(0, 1)], sizeof(int), cudaMemcpyDeviceToDevice, s);
@@ -1521,7 +1522,7 @@ static m2cg_status ens_enqueue_step(m2cg_ensemble* e, int64_t* nl) {
     recon_flux(Gate{&e->stalled[stage], 0});
     if (!e->building) {
       cudaStreamWaitEvent(s, e->ev_a, 0);
-      launch_hold(s, e->hold_cycles);
+      launch_hold(s, e->hold_cycles, Gate{&e->stalled[stage], 1});
     }
     recon_flux(Gate{&e->stalled[stage], 1});
     n += 4;

@@ -608,14 +608,17 @@ void launch_riemann_stragglers(cudaStream_t s, const Params& P, const Mats* md, 
 // Riemann pass and the reconstruction: without it the reconstruction's blocks,
 // which become ready at the same moment as the straggler blocks, take every
 // SM, and the straggler blocks -- which need an empty SM -- wait for the face
-// fluxes to drain.
-__global__ void k_hold(long long cycles) {
+// fluxes to drain.  It returns at once where its gate says that the
+// reconstruction behind it does not run (four tubes of 100 cells as an
+// ensemble: 156 us a step with the wait, 119 without).
+__global__ void k_hold(long long cycles, Gate gt) {
+  if (gt.closed()) return;
   long long t0 = clock64();
   for (int i = 0; i < (1 << 22); i++) {
     if (clock64() - t0 >= cycles) break;
   }
 }
-void launch_hold(cudaStream_t s, long long cycles) { k_hold<<<1, 32, 0, s>>>(cycles); }
+void launch_hold(cudaStream_t s, long long cycles, const Gate& gt) { k_hold<<<1, 32, 0, s>>>(cycles, gt); }
 
 cudaError_t riemann_stragglers_reserve(size_t bytes) {
   return cudaFuncSetAttribute(k_riemann_stragglers, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);

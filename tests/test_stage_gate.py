@@ -140,3 +140,24 @@ def test_ensemble_steps_do_not_depend_on_the_step_before(monkeypatch, ts):
             _same(a, b, name)
         assert counts == want[name][1], name
     e.close()
+
+
+@pytest.mark.parametrize("batched", [False, True])
+def test_steps_without_unfinished_solves_wait_for_nobody(monkeypatch, batched):
+    """The second pass's head start holds a stage back only where the stage
+    before left unfinished solves: ten calm steps of two stages under one of
+    1e8 cycles (about 50 ms; the first step after an upload may hold) end
+    within a quarter of the 1 s that twenty such waits take."""
+    import time
+    monkeypatch.setenv("M2CG_RIEMANN_HOLD_CYCLES", "100000000")
+    cfg, _, calm = _states(abi.TS_RK2)
+    e = Ensemble([cfg, cfg]) if batched else None
+    members = [e.member(i) for i in range(2)] if batched else [Solver(cfg)]
+    for m in members:
+        m.set_state(calm)
+    run = e.run if batched else members[0].run
+    run(1)   # captures the step
+    t0 = time.perf_counter()
+    run(10)
+    assert time.perf_counter() - t0 < 0.25
+    (e or members[0]).close()
