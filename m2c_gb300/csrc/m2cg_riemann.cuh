@@ -5,11 +5,18 @@
 // secant/bisection Hugoniot root (the reference's WITHOUT_BOOST branch,
 // ExactRiemannSolverBase.cpp:1545-1587) and the xi = 0 sampling.
 //
-// One thread solves one problem.  Every loop is bounded by the reference's own
+// One thread solves one problem, or a warp does (Coop below).  Every loop is bounded by the reference's own
 // caps (MaxIts, MaxItsBracketing, MaxItsShock, 3 x IntegrationSteps), so a
 // solve always ends.  The integration-path cache lives in global scratch:
 // `cap` entries of {p, rho, u} per wave, strided by `stride` doubles so that
 // the lanes of a warp touch adjacent words.
+//
+// A warp that solves one problem has one path cache and one row of results.
+// Its lanes hold equal values, but they are ordered only by warp barriers, so
+// memory that they share is written by lane 0 alone, a cache entry between two
+// __syncwarp() (earlier reads before it, later ones after), and no lane reads
+// results back.  Where the solver itself reads what it has written (finalize's
+// `Vs[i] +=`), the caller gives each lane arrays of its own.
 #pragma once
 #include "m2cg_device.cuh"
 
@@ -28,6 +35,7 @@ struct RiemannPrm {
 // Status bits returned alongside the reference's error code.
 enum { RS_PATH_CAPPED = 1 };
 
+template <bool Coop>
 struct PathCache {
   double* base;    // entry e, component c at base[(e * 3 + c) * stride]
   int64_t stride;
@@ -36,9 +44,13 @@ struct PathCache {
   int capped;
   M2CG_DEV double get(int e, int c) const { return base[(int64_t)(e * 3 + c) * stride]; }
   M2CG_DEV void put(int e, double p, double rho, double u) {
-    base[(int64_t)(e * 3 + 0) * stride] = p;
-    base[(int64_t)(e * 3 + 1) * stride] = rho;
-    base[(int64_t)(e * 3 + 2) * stride] = u;
+    if constexpr (Coop) __syncwarp();
+    if (!Coop || (threadIdx.x & 31u) == 0u) {
+      base[(int64_t)(e * 3 + 0) * stride] = p;
+      base[(int64_t)(e * 3 + 1) * stride] = rho;
+      base[(int64_t)(e * 3 + 2) * stride] = u;
+    }
+    if constexpr (Coop) __syncwarp();
   }
   M2CG_DEV void reset(double p, double rho, double u) { n = 1; capped = 0; put(0, p, rho, u); }
   M2CG_DEV void push(double p, double rho, double u) {
@@ -94,7 +106,8 @@ template <bool Coop>
 struct ExactRiemannDevT {
   const Mats* mats;
   RiemannPrm P;
-  PathCache path1, path3;
+  using Path = PathCache<Coop>;
+  Path path1, path3;
   int evals;
   // Learned warm start: with warm_p > 0 on a face whose acoustic pressure
   // jump exceeds P.warm_gate times the mean pressure, the starting pair is
@@ -121,6 +134,7 @@ struct ExactRiemannDevT {
 
   M2CG_DEV const DevMat& mat(int id) const { return mats->m[id]; }
   M2CG_DEV static int lane() { return (int)(threadIdx.x & 31u); }
+  M2CG_DEV static bool writes() { return !Coop || lane() == 0; }   // this thread stores the problem's results
   M2CG_DEV static double bc(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
   M2CG_DEV static Quot qof(double b) { return quot_of(b); }
   M2CG_DEV static double qd(double a, const Quot& d) { return qdiv(a, d); }
@@ -464,7 +478,7 @@ struct ExactRiemannDevT {
   }
 
   // Fixed-step rarefaction of the non-adaptive solver, ExactRiemannSolverBase.cpp:2534-2651
-  __device__ __noinline__ bool rarefaction_fixed(int wave, PathCache& path, const DevMat& M, double rho, double u,
+  __device__ __noinline__ bool rarefaction_fixed(int wave, Path& path, const DevMat& M, double rho, double u,
                                                  double p, double ps, double& rhos, double& us, bool* trans_rare,
                                                  double* Vrare) {
     double rhos_0 = rho, us_0 = u, ps_0 = p, xi_0;
@@ -538,7 +552,7 @@ struct ExactRiemannDevT {
   }
 
   // ExactRiemannSolverBase.cpp:1212-1624
-  __device__ __noinline__ bool rho_u_star(int wave, PathCache& path, double rho, double u, double p, double ps, int id,
+  __device__ __noinline__ bool rho_u_star(int wave, Path& path, double rho, double u, double p, double ps, int id,
                            double rhos0, double rhos1, double& rhos, double& us, bool* trans_rare, double* Vrare) {
     const DevMat& M = mat(id);
     rhos = rho;

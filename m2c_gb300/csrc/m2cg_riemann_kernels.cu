@@ -42,13 +42,13 @@ __device__ __forceinline__ void iface_inputs(const Params& P, const StateSet& S,
 // stage only) and form the two one-sided fluxes (SpaceOperator.cpp:1641-1690).
 __device__ __forceinline__ int iface_finish(const Params& P, const IfaceList& L, int64_t s, int d, int idm, int idp,
                                             const double* Vm, const double* Vp, double* Vs, int midid, double* Vsm,
-                                            double* Vsp, int err, int store) {
+                                            double* Vsp, int err, int store, bool writes) {
   int bad = 0;
   eos_clip(P.mats.m[idm], Vsm);
   bad += eos_bad5(P.mats.m[idm], Vsm);
   eos_clip(P.mats.m[idp], Vsp);
   bad += eos_bad5(P.mats.m[idp], Vsp);
-  if (store) {
+  if (store && writes) {
     L.err[s] = err ? 1 : 0;
     for (int p = 0; p < 5; p++) { L.vsm[p][s] = Vsm[p]; L.vsp[p][s] = Vsp[p]; }
   }
@@ -60,7 +60,8 @@ __device__ __forceinline__ int iface_finish(const Params& P, const IfaceList& L,
     bad += !num_flux_if(P, d, Vm, Vsm, idm, lf1);
     bad += !num_flux_if(P, d, Vsp, Vp, idp, lf2);
   }
-  for (int p = 0; p < 5; p++) { L.lf1[p][s] = lf1[p]; L.lf2[p][s] = lf2[p]; }
+  if (writes)
+    for (int p = 0; p < 5; p++) { L.lf1[p][s] = lf1[p]; L.lf2[p][s] = lf2[p]; }
   return bad;
 }
 
@@ -155,8 +156,9 @@ __device__ __forceinline__ int iface_solve(const Params& P, StateSet S, const in
   if (P.mp_flux == M2CG_MPFLUX_LLF) {   // SpaceOperator.cpp:1617-1626: no Riemann solve
     double lf[5];
     acc[3] += !flux_llf2(P.mats.m[idm], P.mats.m[idp], d, Vm, Vp, lf);
-    for (int p = 0; p < 5; p++) { L.lf1[p][s] = lf[p]; L.lf2[p][s] = lf[p]; }
-    if (store) L.err[s] = 1;  // no star states for the phase-change update
+    if (Solver::writes())
+      for (int p = 0; p < 5; p++) { L.lf1[p][s] = lf[p]; L.lf2[p][s] = lf[p]; }
+    if (store && Solver::writes()) L.err[s] = 1;  // no star states for the phase-change update
     return 0;
   }
   double dir[3] = {0.0, 0.0, 0.0};
@@ -171,10 +173,10 @@ __device__ __forceinline__ int iface_solve(const Params& P, StateSet S, const in
   acc[1]++;
   acc[4] += rs.path1.capped | rs.path3.capped;
   acc[5] += rs.fallback;
-  L.iters[s] = rs.evals;
+  if (Solver::writes()) L.iters[s] = rs.evals;
   if (err) acc[2]++;
   if (err < 0) acc[3]++;
-  acc[3] += iface_finish(P, L, s, d, idm, idp, Vm, Vp, Vs, midid, Vsm, Vsp, err, store);
+  acc[3] += iface_finish(P, L, s, d, idm, idp, Vm, Vp, Vs, midid, Vsm, Vsp, err, store, Solver::writes());
   return err;
 }
 
@@ -510,8 +512,16 @@ __global__ void k_riemann_batch(const Mats* __restrict__ md, RiemannPrm rp, int6
   batch_problems<Coop>(n, bp, [&](int64_t q) {
     int oid = 0;
     rs.warm_p = warm ? warm[q] : 0.0;
-    int e = rs.solve(&dir[q * 3], &Vm[q * 5], idm[q], &Vp[q * 5], idp[q], &Vs[q * 5], oid, &Vsm[q * 5], &Vsp[q * 5]);
-    if (e == 2) return 2;
+    int e;
+    if constexpr (Coop) {
+      double s[5], sm[5], sp[5];
+      e = rs.solve(&dir[q * 3], &Vm[q * 5], idm[q], &Vp[q * 5], idp[q], s, oid, sm, sp);
+      if (!rs.writes()) return 0;
+      for (int p = 0; p < 5; p++) { Vs[q * 5 + p] = s[p]; Vsm[q * 5 + p] = sm[p]; Vsp[q * 5 + p] = sp[p]; }
+    } else {
+      e = rs.solve(&dir[q * 3], &Vm[q * 5], idm[q], &Vp[q * 5], idp[q], &Vs[q * 5], oid, &Vsm[q * 5], &Vsp[q * 5]);
+      if (e == 2) return 2;
+    }
     id[q] = oid;
     if (iters) iters[q] = rs.evals;
     if (err) err[q] = e;
@@ -549,6 +559,7 @@ __device__ __forceinline__ int riemann_eos_problem(Solver& rs, Mats& mats, int64
   rs.warm_p = warm ? warm[q] : 0.0;
   const int e = rs.solve(dir, Vm, 0, Vp, 1, Vs, oid, Vsm, Vsp);
   if (e == 2) return 2;
+  if (!rs.writes()) return 0;
   out[q * 4 + 0] = Vsm[4];
   out[q * 4 + 1] = Vsm[1];
   out[q * 4 + 2] = Vsm[0];
