@@ -61,11 +61,7 @@ M2CG_DEV bool i_le0(double x) { return i_eq0(x) || (hi_word(x) < 0 && !is_nan_bi
 M2CG_DEV bool i_gt0(double x) { return hi_word(x) >= 0 && !i_eq0(x) && !is_nan_bits(x); }            // x > 0
 M2CG_DEV bool i_ge0(double x) { return i_eq0(x) || (hi_word(x) >= 0 && !is_nan_bits(x)); }           // x >= 0
 M2CG_DEV double flip_sign(double x) { return __hiloint2double(hi_word(x) ^ (int)0x80000000, __double2loint(x)); }
-// order-preserving integer of a double that is not NaN (-0 just below +0)
-M2CG_DEV long long i_key(double x) {
-  const int m = __double2hiint(x) >> 31;
-  return ((long long)(__double2hiint(x) ^ (m & 0x7fffffff)) << 32) | (unsigned)(__double2loint(x) ^ m);
-}
+M2CG_DEV long long i_key(double x) { return if_key(x); }
 M2CG_DEV bool i_special(double a, double b) {   // an infinity or NaN among the two
   return (__double2hiint(a) & 0x7ff00000) == 0x7ff00000 || (__double2hiint(b) & 0x7ff00000) == 0x7ff00000;
 }

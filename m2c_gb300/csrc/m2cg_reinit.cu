@@ -45,32 +45,19 @@ M2CG_DEV bool ri_live(const ReinitState* st) { return st->run && st->detected; }
 // when sb is set, on the integer pipe.
 M2CG_DEV double flip(double x, long long sb) { return __longlong_as_double(__double_as_longlong(x) ^ sb); }
 
-// Godunov's one-sided difference along one axis: max(p - m, p - n, 0), for
-// phi < 0 (sb set) max(m - p, n - p, 0).  Rounding is monotone, so the larger
-// difference is that of the smaller (larger) neighbour, chosen on the integer
-// pipe: one subtraction instead of two, the same bits.  A NaN neighbour gives
-// NaN.
-M2CG_DEV double one_sided(double p, double m, double n, long long sb) {
-  // the neighbours with their signs flipped for phi < 0; the smaller of the two
-  const double x = flip(m, sb), y = flip(n, sb);
-  const bool xl = i_key(x) <= i_key(y) ? !is_nan_bits(y) : is_nan_bits(x);
-  const double d = flip(p, sb) - (xl ? x : y);
-  const long long db = __double_as_longlong(d);
-  return __longlong_as_double(db > 0 ? db : 0);   // negative differences (-0 included) fall below +0
-}
-
 // |grad phi| - 1 by Godunov's upwind rule (LevelSetReinitializer.cpp:1009-1026).
 // For phi >= 0 the x term is max(max(a,0)^2, min(b,0)^2) with a, b the backward
 // and forward differences; it equals (max(p - p_{i-1}, p - p_{i+1}, 0) / h)^2.
-// For phi < 0 the differences change sign (phi = -0 counts as >= 0, as there).
+// For phi < 0 the differences change sign (phi = -0 counts as >= 0, as there):
+// if_one_sided (m2cg_intfp.cuh).
 // With one spacing h the three squares share one product by 1/h.
 M2CG_DEV double ri_res(const double* __restrict__ q, int64_t c, int64_t sy, int64_t sz, const double* rh, bool cube) {
   const double p = q[c];
   const long long pb = __double_as_longlong(p);
-  const long long sb = (pb < 0 && pb != (long long)0x8000000000000000ull) ? (long long)0x8000000000000000ull : 0ll;
-  double gx = one_sided(p, q[c - 1], q[c + 1], sb);
-  double gy = one_sided(p, q[c - sy], q[c + sy], sb);
-  double gz = one_sided(p, q[c - sz], q[c + sz], sb);
+  const uint32_t sb = (pb < 0 && pb != (long long)0x8000000000000000ull) ? 0x80000000u : 0u;
+  double gx = if_one_sided(p, q[c - 1], q[c + 1], sb);
+  double gy = if_one_sided(p, q[c - sy], q[c + sy], sb);
+  double gz = if_one_sided(p, q[c - sz], q[c + sz], sb);
   if (!cube) { gx *= rh[0]; gy *= rh[1]; gz *= rh[2]; }
   const double g2 = fma(gz, gz, fma(gy, gy, gx * gx));
   const double g = if_rsqrt_range(if_hi(g2)) ? g2 * if_rsqrt_core(if_hi(g2), if_lo(g2)) : sqrt(g2);
