@@ -182,62 +182,45 @@ __global__ void __launch_bounds__(RI_THREADS) k_ri_stage(ReinitArgs a) {
   const bool cube = a.rh[0] == a.rh[1] && a.rh[0] == a.rh[2];
   const int64_t n = (int64_t)g.nx * g.ny * g.nz;
   unsigned long long mx = 0;   // the thread's largest value
-  int mxw = 0;                 // the warp's largest high word so far
-  for (int64_t t0 = (int64_t)blockIdx.x * RI_THREADS + (threadIdx.x & ~31); t0 < n; t0 += (int64_t)gridDim.x * RI_THREADS) {
-    const int64_t t = t0 + (threadIdx.x & 31);
-    const bool in = t < n;
+  for (int64_t t = (int64_t)blockIdx.x * RI_THREADS + threadIdx.x; t < n; t += (int64_t)gridDim.x * RI_THREADS) {
     int i, j, k;
     if (n <= 0x7fffffffll) {   // 32-bit divisions where they reach
-      const unsigned u = (unsigned)(in ? t : n - 1), r = u / (unsigned)g.nx;
+      const unsigned u = (unsigned)t, r = u / (unsigned)g.nx;
       i = (int)(u - r * (unsigned)g.nx); k = (int)(r / (unsigned)g.ny); j = (int)(r - (unsigned)k * (unsigned)g.ny);
     } else {
-      const int64_t r = (in ? t : n - 1) / g.nx;
-      i = (int)((in ? t : n - 1) - r * g.nx); k = (int)(r / g.ny); j = (int)(r - (int64_t)k * g.ny);
+      const int64_t r = t / g.nx;
+      i = (int)(t - r * g.nx); k = (int)(r / g.ny); j = (int)(r - (int64_t)k * g.ny);
     }
     const int64_t c = g.at(i, j, k);
-    double e = 0.0, anw = 1.0;
-    if (in) {
-      double R = 0.0;
-      if (!a.tag[c]) {
-        const double res = ri_res(src, c, g.sy, g.sz, a.rh, cube);
-        const double f = mdt * a.sign[c];
-        // f max(-1, min(1, res)): beyond 1 only the sign of res remains
-        const long long rb = __double_as_longlong(res) & (long long)0x8000000000000000ull;
-        const unsigned long long ab = as_bits(res) & 0x7fffffffffffffffull;
-        if (ab <= 0x3ff0000000000000ull) R = f * res;
-        else if (ab < 0x7ff0000000000000ull) R = flip(f, rb);
-        else R = (f * res) / fabs(res);   // infinite or NaN
-        if (S == 1) mx = ab > mx ? ab : mx;
-      }
-      if (S == 1) {
-        const double p = src[c];
-        if (restore) a.phi[c] = p;
-        out[c] = p + R;
-      } else if (S == 2) {
-        // products by 1/4 are exact: the fused forms round as the separate ones
-        out[c] = fma(0.25, R, fma(0.25, src[c], 0.75 * a.phi[c]));
-      } else {
-        const double old = out[c];
-        const double nw = ((1.0 / 3.0) * old + (2.0 / 3.0) * src[c]) + (2.0 / 3.0) * R;
-        out[c] = nw;
-        e = fabs(nw - old);
-        anw = fabs(nw);
-      }
+    double R = 0.0;
+    if (!a.tag[c]) {
+      const double res = ri_res(src, c, g.sy, g.sz, a.rh, cube);
+      const double f = mdt * a.sign[c];
+      // f max(-1, min(1, res)): beyond 1 only the sign of res remains
+      const long long rb = __double_as_longlong(res) & (long long)0x8000000000000000ull;
+      const unsigned long long ab = as_bits(res) & 0x7fffffffffffffffull;
+      if (ab <= 0x3ff0000000000000ull) R = f * res;
+      else if (ab < 0x7ff0000000000000ull) R = flip(f, rb);
+      else R = (f * res) / fabs(res);   // infinite or NaN
+      if (S == 1) mx = ab > mx ? ab : mx;
     }
-    if (S == 3) {
-      // The largest e / |nw|: a quotient's high word is at most the difference
-      // of the operands' plus 1.0's (the binary logarithm is above its chord),
-      // so nodes that cannot raise the warp's maximum skip the division.
-      const int cand = __double2hiint(e) - __double2hiint(anw) + 0x3ff00001;
-      const bool odd = !(anw > 1e-300) || (__double2hiint(e) & 0x7ff00000) == 0x7ff00000;
-      if (__any_sync(0xffffffffu, e != 0.0 && (cand >= mxw || odd))) {
-        double q = e;
-        if (anw > 1e-300) q = e * rcp_fast(anw);
-        else if (anw != 0.0) q = e / anw;
-        const unsigned long long b = as_bits(q);
-        mx = b > mx ? b : mx;
-        mxw = __reduce_max_sync(0xffffffffu, (int)(mx >> 32));
-      }
+    if (S == 1) {
+      const double p = src[c];
+      if (restore) a.phi[c] = p;
+      out[c] = p + R;
+    } else if (S == 2) {
+      // products by 1/4 are exact: the fused forms round as the separate ones
+      out[c] = fma(0.25, R, fma(0.25, src[c], 0.75 * a.phi[c]));
+    } else {
+      const double old = out[c];
+      const double nw = ((1.0 / 3.0) * old + (2.0 / 3.0) * src[c]) + (2.0 / 3.0) * R;
+      out[c] = nw;
+      double e = fabs(nw - old);
+      const double anw = fabs(nw);
+      if (anw > 1e-300) e *= rcp_fast(anw);
+      else if (nw != 0.0) e /= anw;
+      const unsigned long long b = as_bits(e);
+      mx = b > mx ? b : mx;
     }
   }
   if (S == 1) block_max_atomic(mx, &st->res_bits);
