@@ -268,26 +268,27 @@ M2CG_INT int64_t if_key(double x) {
   const uint32_t m = (uint32_t)((int32_t)if_hi(x) >> 31);
   return (int64_t)(((uint64_t)(if_hi(x) ^ (m & 0x7fffffffu)) << 32) | (if_lo(x) ^ m));
 }
-M2CG_INT bool if_special(double x) { return (if_hi(x) & 0x7ff00000u) == 0x7ff00000u; }   // infinite or NaN
+// bit 31 set for an infinity or a NaN (several operands: or them, one test)
+M2CG_INT uint32_t if_special_bit(double x) { return (if_hi(x) & 0x7fffffffu) + 0x00100000u; }
 // x, negated where sb (0 or the sign bit) is set
 M2CG_INT double if_flip(double x, uint32_t sb) { return if_dbl(if_hi(x) ^ sb, if_lo(x)); }
 
 // Godunov's one-sided difference along one axis: max(p - m, p - n, 0), for
 // phi < 0 (sb set) max(m - p, n - p, 0), the maximum taken over the bit patterns
 // as signed integers (a NaN with a clear sign bit wins, one with a set sign bit
-// counts as negative).  Rounding is monotone, so the larger difference is that of
-// the smaller (larger) neighbour, chosen on the integer pipe: one subtraction
-// instead of two, the same bits.  Infinities and NaNs take both differences.
-M2CG_INT_SLOW double if_one_sided_special(double p, double m, double n, uint32_t sb) {
-  const double a = if_flip(p - m, sb), b = if_flip(p - n, sb);
-  const int64_t x = (int64_t)(((uint64_t)if_hi(a) << 32) | if_lo(a)), y = (int64_t)(((uint64_t)if_hi(b) << 32) | if_lo(b));
-  return x > y ? (x > 0 ? a : 0.0) : (y > 0 ? b : 0.0);
-}
+// counts as negative).  Rounding is monotone, so for finite operands the larger
+// difference is that of the smaller (larger) neighbour, chosen on the integer
+// pipe: one subtraction instead of two, the same bits (if_one_sided; the caller
+// has seen to the operands with if_special_bit).  if_one_sided_any forms both.
 M2CG_INT double if_one_sided(double p, double m, double n, uint32_t sb) {
-  if (if_special(p) || if_special(m) || if_special(n)) return if_one_sided_special(p, m, n, sb);
   const double x = if_flip(m, sb), y = if_flip(n, sb);
   const double d = if_flip(p, sb) - (if_key(x) <= if_key(y) ? x : y);
   return (int32_t)if_hi(d) < 0 ? 0.0 : d;
+}
+M2CG_INT double if_one_sided_any(double p, double m, double n, uint32_t sb) {
+  const double a = if_flip(p - m, sb), b = if_flip(p - n, sb);
+  const int64_t x = (int64_t)(((uint64_t)if_hi(a) << 32) | if_lo(a)), y = (int64_t)(((uint64_t)if_hi(b) << 32) | if_lo(b));
+  return x > y ? (x > 0 ? a : 0.0) : (y > 0 ? b : 0.0);
 }
 
 }  // namespace m2cg

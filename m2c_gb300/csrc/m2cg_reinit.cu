@@ -49,19 +49,28 @@ M2CG_DEV double flip(double x, long long sb) { return __longlong_as_double(__dou
 // For phi >= 0 the x term is max(max(a,0)^2, min(b,0)^2) with a, b the backward
 // and forward differences; it equals (max(p - p_{i-1}, p - p_{i+1}, 0) / h)^2.
 // For phi < 0 the differences change sign (phi = -0 counts as >= 0, as there):
-// if_one_sided (m2cg_intfp.cuh).
-// With one spacing h the three squares share one product by 1/h.
-M2CG_DEV double ri_res(const double* __restrict__ q, int64_t c, int64_t sy, int64_t sz, const double* rh, bool cube) {
-  const double p = q[c];
-  const long long pb = __double_as_longlong(p);
-  const uint32_t sb = (pb < 0 && pb != (long long)0x8000000000000000ull) ? 0x80000000u : 0u;
-  double gx = if_one_sided(p, q[c - 1], q[c + 1], sb);
-  double gy = if_one_sided(p, q[c - sy], q[c + sy], sb);
-  double gz = if_one_sided(p, q[c - sz], q[c + sz], sb);
+// if_one_sided (m2cg_intfp.cuh).  With one spacing h the three squares share one
+// product by 1/h.
+M2CG_DEV double ri_norm(double gx, double gy, double gz, const double* rh, bool cube) {
   if (!cube) { gx *= rh[0]; gy *= rh[1]; gz *= rh[2]; }
   const double g2 = fma(gz, gz, fma(gy, gy, gx * gx));
   const double g = if_rsqrt_range(if_hi(g2)) ? g2 * if_rsqrt_core(if_hi(g2), if_lo(g2)) : sqrt(g2);
   return cube ? fma(g, rh[0], -1.0) : g - 1.0;
+}
+// with an infinity or a NaN in the stencil
+static __device__ __noinline__ double ri_res_special(const double* q, int64_t c, int64_t sy, int64_t sz, const double* rh,
+                                                     bool cube, uint32_t sb) {
+  return ri_norm(if_one_sided_any(q[c], q[c - 1], q[c + 1], sb), if_one_sided_any(q[c], q[c - sy], q[c + sy], sb),
+                 if_one_sided_any(q[c], q[c - sz], q[c + sz], sb), rh, cube);
+}
+M2CG_DEV double ri_res(const double* __restrict__ q, int64_t c, int64_t sy, int64_t sz, const double* rh, bool cube) {
+  const double p = q[c];
+  const double xm = q[c - 1], xp = q[c + 1], ym = q[c - sy], yp = q[c + sy], zm = q[c - sz], zp = q[c + sz];
+  const uint32_t sb = lt_zero_bits(p) ? 0x80000000u : 0u;
+  const uint32_t sp = if_special_bit(p) | if_special_bit(xm) | if_special_bit(xp) | if_special_bit(ym) |
+                      if_special_bit(yp) | if_special_bit(zm) | if_special_bit(zp);
+  if ((int32_t)sp < 0) return ri_res_special(q, c, sy, sz, rh, cube, sb);
+  return ri_norm(if_one_sided(p, xm, xp, sb), if_one_sided(p, ym, yp, sb), if_one_sided(p, zm, zp, sb), rh, cube);
 }
 
 // Block maximum of non-negative bit patterns, one atomic per block.

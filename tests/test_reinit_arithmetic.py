@@ -37,9 +37,12 @@ int main() {
   for (long i = 0; i < 20000000; i++) {
     const double p = draw(0.1), m = draw(p), n = draw(i & 1 ? p : m);
     const bool neg = nx() & 1;
-    const double x = if_one_sided(p, m, n, neg ? 0x80000000u : 0u), y = both(p, m, n, neg);
-    bad += u64(x) != u64(y);
-    special += if_special(p) || if_special(m) || if_special(n);
+    const bool sp = (int32_t)(if_special_bit(p) | if_special_bit(m) | if_special_bit(n)) < 0;
+    const uint32_t sb = neg ? 0x80000000u : 0u;
+    const double x = if_one_sided_any(p, m, n, sb), y = both(p, m, n, neg);
+    bad += u64(x) != u64(y) || sp != !(std::isfinite(p) && std::isfinite(m) && std::isfinite(n));
+    if (sp) special++;
+    else bad += u64(if_one_sided(p, m, n, sb)) != u64(y);
   }
   printf("%ld %ld\n", bad, special);
 }
