@@ -505,6 +505,8 @@ cudaError_t reinit_build_graph(cudaStream_t s, const ReinitArgs& a, int nsm, int
   cudaGraphConditionalHandle h;
   const int64_t rows = (int64_t)a.g.ny * a.g.nz;
   const int64_t nreal = rows * a.g.nx;
+  // the preparation walks rows, a sub-stage nodes
+  const int pblocks = (int)std::min<int64_t>(rows, (int64_t)nsm * 16);
   const int sblocks = (int)std::max<int64_t>(1, std::min<int64_t>((nreal + RI_THREADS - 1) / RI_THREADS, (int64_t)nsm * 16));
   const int64_t nghost = 2 * ((int64_t)a.g.ny * a.g.nz + (int64_t)a.g.nx * a.g.nz + (int64_t)a.g.nx * a.g.ny);
   const int gblocks = (int)std::max<int64_t>(1, std::min<int64_t>((nghost + 255) / 256, (int64_t)nsm * 4));
@@ -518,7 +520,7 @@ cudaError_t reinit_build_graph(cudaStream_t s, const ReinitArgs& a, int nsm, int
   RI_CK(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
   RI_CK(cudaStreamBeginCaptureToGraph(s, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
   k_ri_begin<<<1, 1, 0, s>>>(a, h, gated);
-  k_ri_prep<<<sblocks, RI_THREADS, 0, s>>>(a);
+  k_ri_prep<<<pblocks, RI_THREADS, 0, s>>>(a);
   e = cudaStreamGetCaptureInfo(s, &cs, nullptr, nullptr, &deps, nullptr, &nd);
   if (e == cudaSuccess) {
     np.type = cudaGraphNodeTypeConditional;
