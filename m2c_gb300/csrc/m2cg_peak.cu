@@ -98,10 +98,17 @@ __global__ void k_selftest_quotient(int64_t n, uint64_t seed, unsigned long long
         if ((r3 >> 40) & 1) { a = x; b = y; } else { a = y; b = x; }
         break;
       }
-      case 5: {   // exponents at and around 128 and 1920
-        const int ea = ((r3 & 1) ? 128 : 1920) + (int)((r3 >> 1) % 9) - 4;
-        const int eb = ((r3 >> 8) & 1) ? 1023 + (int)((r3 >> 9) % 1000) - 500 : ((r3 >> 20) & 1 ? 128 : 1920) + (int)((r3 >> 21) % 9) - 4;
-        a = with_exp(r1, ea); b = with_exp(r2, eb);
+      case 5: {   // the integer path's limits: operand fields at 0..3 and 2044..2047, quotient fields about 2 and 2045
+        const int lim = (int)((r3 >> 2) & 7), f = lim < 4 ? lim : 2040 + lim;   // 0..3, 2044..2047
+        const int mid = 700 + (int)((r3 >> 8) % 650);
+        if ((r3 & 3) == 0) { a = with_exp(r1, f); b = with_exp(r2, mid); }
+        else if ((r3 & 3) == 1) { a = with_exp(r1, mid); b = with_exp(r2, f); }
+        else {
+          const int eq = (r3 & 1) ? 2043 + (int)((r3 >> 5) % 5) : (int)((r3 >> 5) % 5);   // a's field less b's, plus 1023
+          const int eb = (r3 & 1) ? 1 + (int)((r3 >> 8) % 1000) : 1024 + (int)((r3 >> 8) % 1000);
+          a = with_exp(r1, eq + eb - 1023);
+          b = with_exp(r2, eb);
+        }
         break;
       }
       case 6: {   // exact quotients: a = b * m for a small integer m
@@ -120,14 +127,18 @@ __global__ void k_selftest_quotient(int64_t n, uint64_t seed, unsigned long long
     const bool both_nan = isnan(q) && isnan(ref);
     if (!both_nan && __double_as_longlong(q) != __double_as_longlong(ref)) bad++;
     if (m2cg::qfast(1.0, d) && __double_as_longlong(m2cg::qdiv(1.0, d)) != __double_as_longlong(1.0 / b)) bad++;
-    const double w = fabs(a), root = m2cg::dsqrt(w);
-    if (!isnan(w) && __double_as_longlong(root) != __double_as_longlong(sqrt(w))) bad++;
+    const double w = fabs(a), root = sqrt(w);
+    if (!isnan(w) && __double_as_longlong(m2cg::dsqrt(w)) != __double_as_longlong(root)) bad++;
     const double dq = m2cg::ddiv(a, b);
     if (!both_nan && __double_as_longlong(dq) != __double_as_longlong(ref)) bad++;
     double q2, w2;   // the paired form, also with the other quotient out of range
     m2cg::ddiv2(a, b, 1.0, w, q2, w2);
     if (!both_nan && __double_as_longlong(q2) != __double_as_longlong(ref)) bad++;
     if (!isnan(w) && __double_as_longlong(w2) != __double_as_longlong(1.0 / w)) bad++;
+    // the low-latency forms of the warp's solver
+    const double lq = m2cg::ddiv_lat(a, b), lr = m2cg::if_sqrt_lat(w);
+    if (!both_nan && __double_as_longlong(lq) != __double_as_longlong(ref)) bad++;
+    if (!isnan(w) && __double_as_longlong(lr) != __double_as_longlong(root)) bad++;
     fast += m2cg::qfast(a, d) ? 1 : 0;
   }
   if (bad) atomicAdd(&out[0], bad);
