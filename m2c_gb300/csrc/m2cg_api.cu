@@ -388,11 +388,12 @@ static StageArgs stage_args(m2cg_ctx* x, int stage, bool last, const StateSet& i
   const int ts = x->cfg.ts_type;
   if (stage == 0) { A.store_un = (ts != M2CG_TS_FORWARD_EULER); }
   if (ts == M2CG_TS_FORWARD_EULER) A.ls_use_updated_v = 1;
-  if (ts == M2CG_TS_RK2 && stage == 1) { A.a_own = 0.5; A.b_un = 0.5; A.c_dt = 0.5; A.la = 0.5; A.lb = 0.5; A.lc = 0.5; }
-  if (ts == M2CG_TS_RK3 && stage == 1) { A.a_own = 0.25; A.b_un = 0.75; A.c_dt = 0.25; A.la = 0.25; A.lb = 0.75; A.lc = 0.25; }
+  if (ts == M2CG_TS_RK2 && stage == 1) { A.a_own = 0.5; A.b_un = 0.5; A.la = 0.5; A.lb = 0.5; }
+  if (ts == M2CG_TS_RK3 && stage == 1) { A.a_own = 0.25; A.b_un = 0.75; A.la = 0.25; A.lb = 0.75; }
   if (ts == M2CG_TS_RK3 && stage == 2) {
-    A.a_own = 2.0 / 3.0; A.b_un = 1.0 / 3.0; A.c_dt = 2.0 / 3.0; A.la = 2.0 / 3.0; A.lb = 1.0 / 3.0; A.lc = 2.0 / 3.0;
+    A.a_own = 2.0 / 3.0; A.b_un = 1.0 / 3.0; A.la = 2.0 / 3.0; A.lb = 1.0 / 3.0;
   }
+  if (stage > 0) A.lc = rk_share(ts, stage);
   return A;
 }
 

@@ -140,7 +140,6 @@ struct Quot {
   double b;
   uint64_t D, R;
 };
-M2CG_DEV int exp_field(double x) { return (int)((bits(x) >> 52) & 0x7ff); }
 M2CG_DEV Quot quot_of(double b) {
   Quot q;
   q.b = b;

@@ -245,6 +245,12 @@ struct Box3 {
   double lo[3], hi[3];
 };
 
+// Share of dt that a stage's residual enters the state with: the conserved
+// variables through DevScalars::cf, the level set through StageArgs::lc.
+__host__ __device__ constexpr double rk_share(int ts_type, int stage) {
+  return stage == 0 ? 1.0 : ts_type == M2CG_TS_RK2 ? 0.5 : stage == 1 ? 0.25 : 2.0 / 3.0;
+}
+
 struct StageArgs {
   // residual input (neighbors) and own-cell inputs of the stage combination
   StateSet in;          // V and phi of the stage input (residual evaluated here)
@@ -257,7 +263,7 @@ struct StageArgs {
   int stage;            // 0, 1, 2
   int last;             // 1 on the final stage
   int store_un;         // write Un (first stage)
-  double a_own, b_un, c_dt;   // U = a*Us + b*Un + c*dt*R  (first stage: a=0, b=1, c=1)
+  double a_own, b_un;         // U = a*Us + b*Un + rk_share*dt*R  (first stage: a=0, b=1)
   double la, lb, lc;          // phi = la*phi_own_other + lb*phi_n + lc*dt*R (see kernel)
   int ls_use_updated_v;       // forward Euler: level set advected with the updated velocity
   double* R[5];               // residual output (residual-only mode)

@@ -834,7 +834,7 @@ __device__ __forceinline__ void k_dt_finalize_body(const Params& P, DevScalars* 
   sc->dt = dt;
   sc->cfl = cfl;
   for (int st = 0; st < 3; st++) {
-    const double w = st == 0 ? 1.0 : P.ts_type == M2CG_TS_RK2 ? 0.5 : st == 1 ? 0.25 : 2.0 / 3.0;   // stage_args' c_dt
+    const double w = rk_share(P.ts_type, st);
     for (int d = 0; d < 3; d++) sc->cf[st][d] = (P.area[d] * P.inv_negvol) * (w * dt);
   }
   sc->time = t + dt;
