@@ -114,6 +114,28 @@ def test_evaluation_budget_changes_no_step(monkeypatch, ts, mp_recon):
         np.testing.assert_array_equal(got[2], ref[2], err_msg=limit)
 
 
+@pytest.mark.parametrize("sms,lanes", [(1, 1), (2, 1), (40, 1), (1, 8), (152, 4)])
+def test_layout_of_the_second_pass_changes_no_step(monkeypatch, sms, lanes):
+    """About 300 handed-over solves a stage: several a warp in one and in more
+    rounds (8 and 16 warps), one a warp on all eight warps of a block (320
+    warps), packed by the lane setting; the default has one a warp on four."""
+    monkeypatch.setenv(LIMIT, "3")
+    cfg, stirred, _ = _states(abi.TS_RK2)
+    ref = None
+    for env in ({}, {"M2CG_RIEMANN_STRAGGLER_SMS": str(sms), "M2CG_RIEMANN_STRAGGLER_LANES": str(lanes)}):
+        for k, v in env.items():
+            monkeypatch.setenv(k, v)
+        s = Solver(cfg, stirred)
+        s.run(3)
+        got = s.get_state(), s.counters()
+        s.close()
+        if ref is None:
+            ref = got
+    _same(got[0], ref[0], (sms, lanes))
+    for k in COUNTS:
+        assert got[1][k] == ref[1][k], k
+
+
 @pytest.mark.parametrize("ts", [abi.TS_RK2, abi.TS_RK3])
 def test_ensemble_steps_do_not_depend_on_the_step_before(monkeypatch, ts):
     monkeypatch.setenv(LIMIT, "3")
