@@ -174,10 +174,11 @@ __global__ void __launch_bounds__(RI_THREADS) k_ri_prep(ReinitArgs a) {
 //
 // Bound by the FP64 pipe: about 13 FP64 instructions per node and sub-stage
 // (three differences, three squares, the root's product, the product by 1/h
-// with the -1, two for R, the combination; 30 before the choices, the root and
-// the sign of R moved to the integer pipe): 0.41 ms per sub-stage at
-// 256 x 224 x 192 against 0.58.  A warp covers 32 consecutive interior nodes of
-// the x-fastest order (rows of any length leave no idle lanes).
+// with the -1, two for R, the combination; 30 with the choices, the root and
+// the sign of R on that pipe): 1.31 ms an iteration of three sub-stages at
+// 256 x 224 x 192 against 1.91, 2.01 against 2.90 at 256^3.  A warp covers 32
+// consecutive interior nodes of the x-fastest order (rows of any length leave no
+// idle lanes).
 template <int S>
 __global__ void __launch_bounds__(RI_THREADS) k_ri_stage(ReinitArgs a) {
   ReinitState* st = a.st;

@@ -294,8 +294,8 @@ struct ExactRiemannDevT {
   // Here and in the other steps a stage's density is checked before its sound
   // speed is formed: a step from c^2 = 0 (p = -p_inf) has a stage of density
   // -infinity, whose special quotients leave the integer pipe, and a solve that
-  // ends there takes up to a million such steps (500 label
-  // problems, one of them such: 6.1 s with the check behind, 2.6 s).
+  // ends there takes up to a million such steps (500 label problems, one of them
+  // such: 2.6 s, 6.1 s with the check behind the sound speed).
   __device__ __noinline__ bool rk4_coop(int wave, const DevMat& M, double rho_0, double u_0, double p_0, double dp,
                                         double& rho, double& u, double& p, double& xi) const {
     const int l = lane();
@@ -342,8 +342,8 @@ struct ExactRiemannDevT {
 
   // Cash-Karp step, ExactRiemannSolverBase.cpp:1771-1896.  The same
   // operations in the same order; a divisor that serves several quotients
-  // (c_k^2, c_k, rho_k) takes its correctly rounded reciprocal once and each
-  // quotient comes out of qdiv bit-identical to the division.
+  // (c_k^2, c_k, rho_k) has its fixed-point reciprocal formed once (Quot) and
+  // each quotient comes out of qdiv bit-identical to the division.
   __device__ __noinline__ bool rk45(int wave, const DevMat& M, double rho_0, double u_0, double p_0, double dp,
                      double& rho, double& u, double& p, double& xi, double& uErr, double& rhoErr) const {
     if constexpr (Coop) return rk45_coop(wave, M, rho_0, u_0, p_0, dp, rho, u, p, xi, uErr, rhoErr);
@@ -429,7 +429,7 @@ struct ExactRiemannDevT {
   }
 
   // Classical RK4 step of the non-adaptive solver, ExactRiemannSolverBase.cpp:2896-2990
-  // (shared reciprocals as in rk45)
+  // (divisors with several quotients as in rk45)
   __device__ __noinline__ bool rk4(int wave, const DevMat& M, double rho_0, double u_0, double p_0, double dp,
                                    double& rho, double& u, double& p, double& xi) const {
     if constexpr (Coop) return rk4_coop(wave, M, rho_0, u_0, p_0, dp, rho, u, p, xi);

@@ -284,11 +284,11 @@ __device__ __forceinline__ StragglerWarps straggler_warps(int64_t n, int lanes, 
 // reconstruction and fluxes run on the other SMs.  The shared memory it asks
 // for holds the path caches of half its warps (of a warp's first lane when
 // there are several faces per warp); the rest go through L1 to the scratch.
-// Eight warps an SM instead of four, and none of the path caches shared by the
-// upper four, cost a chain little (it waits for latencies) and halve the rounds
+// Eight warps an SM instead of four, the upper four with their path caches in
+// the scratch, cost a chain little (it waits for latencies) and halve the rounds
 // where more than 608 faces stall: five steps of the bubble cluster (1,100 to
-// 1,600 stalled faces) 241, 222, 272, 350 ms for four sets of states against
-// 286, 251, 283, 380.
+// 1,600 stalled faces) take 216, 196, 248, 321 ms for four sets of states with
+// eight, 254, 221, 261, 353 with four.
 __global__ void __launch_bounds__(256) k_riemann_stragglers(Params P, const Mats* __restrict__ md, StateSet S,
                                                             const int32_t* __restrict__ id, double* const* fs,
                                                             IfaceList L, int store, double* scratch, int path_cap,
@@ -472,7 +472,8 @@ cudaError_t riemann_stragglers_ens_reserve(size_t bytes) {
 // are warps, else one per thread -- two launches, of which the device count lets
 // one work.  (Two kernels, since one that held both solvers spilt 3.4 kB a
 // thread and took 9.8 ms instead of 9.3 ms for 20,000 problems.)  65,536 random
-// pairs with 570 unfinished ones: 17.8 s with the second pass, 22.1 s without.
+// pairs with 570 unfinished ones take 5.6 s (17.8 s with the second pass against
+// 22.1 s without it before the steps checked their density first).
 struct BatchPass {
   const int32_t* list;                      // the problems to solve (NULL: 0 .. n - 1) ...
   const unsigned long long* list_n;         // ... and their number
